@@ -259,6 +259,12 @@ int lq_ssd_bmm_chunk(const lq_ssd_problem* p, int b_is_fp, lq_stream stream);
  * Replaces _quant_chunk_scan_fwd (mamba2/chunk_scan_v2.py:14-366). */
 int lq_ssd_chunk_scan(const lq_ssd_problem* p, lq_stream stream);
 
+/* Whole call of _quant_mamba_chunk_scan_combined_fwd (mamba2/ssd_combined.py:19-131): cumsum, chunk state, state passing,
+ * C.B^T and chunk scan. The descriptor names the inputs, the scales and out; dt, dA, states, passed, final_state, cb and
+ * q_BT are carved from the caller's 256-byte aligned workspace and what the descriptor holds for them is ignored. */
+size_t lq_ssd_combined_workspace_bytes(const lq_ssd_problem* p);
+int lq_ssd_combined_fwd(const lq_ssd_problem* p, int keyside, void* workspace, size_t workspace_bytes, lq_stream stream);
+
 /* Mamba-2 prologue on the B and C lanes of xBC [B,T,d_ssm+2*G*N] f16: [x D_QK, fp16 round] -> signs ->
  * H_2 (x) H_{N/2} on bf16-rounded values -> fp16 round -> rint(. * inv_scale) clamp [-128,127].
  * Replaces fused_split_rotate_quant_xBC (mamba2/fused_split_rotate_xBC.py:31-329). */

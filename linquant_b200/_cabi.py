@@ -61,6 +61,22 @@ def lib():
     return _lib
 
 
+_host = None
+
+
+def host():
+    """The ``_host`` module: the library's whole-call entries on torch tensors, without a ctypes descriptor in between."""
+    global _host
+    if _host is None:
+        lib()  # one message for a missing build
+        try:
+            from . import _host as mod
+        except ImportError as e:
+            raise LinQuantError(f"linquant_b200/_host.so cannot be loaded ({e}): build it with `python -m linquant_b200.build`") from e
+        _host = mod
+    return _host
+
+
 _STATUS_WORDS = {}
 
 

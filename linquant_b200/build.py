@@ -1,18 +1,22 @@
-"""In-tree build of the CUDA library: ``python -m linquant_b200.build`` -> linquant_b200/liblinquant_b200.so.
+"""In-tree build: ``python -m linquant_b200.build`` -> linquant_b200/liblinquant_b200.so and linquant_b200/_host.so.
 
-Plain nvcc for sm_100a; the library has a C ABI and links against the CUDA runtime only (no torch headers)."""
+The CUDA library is plain nvcc for sm_100a with a C ABI; it links against the CUDA runtime only (no torch headers).
+``_host`` is the CPython module that hands torch tensors to the library's whole-call entries (g++, torch headers)."""
 
 from __future__ import annotations
 
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "csrc", "build")
 LIB = os.path.join(HERE, "liblinquant_b200.so")
+HOST_SRC = os.path.join(CSRC, "host", "lq_host.cpp")
+HOST_LIB = os.path.join(HERE, "_host.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 # no fast-math: precise division / sqrt / expf are required by the code rule
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-Xptxas", "-v"]
@@ -41,15 +45,38 @@ def _compile(src):
     return src, r.stderr
 
 
+def _compile_host(_=None):
+    """The object file of ``_host``, and the torch library directories to link it against."""
+    from torch.utils import cpp_extension as ext
+
+    obj = os.path.join(OBJ, "lq_host.o")
+    if _stale(os.path.join("host", "lq_host.cpp"), obj):
+        inc = ext.include_paths() + [sysconfig.get_paths()["include"], "/usr/local/cuda/include"]
+        cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-w", *[a for i in inc for a in ("-isystem", i)],
+               "-c", HOST_SRC, "-o", obj]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            raise RuntimeError(f"g++ failed on lq_host.cpp:\n{r.stdout}\n{r.stderr}")
+    return obj, ext.library_paths()
+
+
 def build(verbose=False):
     os.makedirs(OBJ, exist_ok=True)
     with ThreadPoolExecutor(max_workers=os.cpu_count() or 4) as ex:
+        host = ex.submit(_compile_host)
         logs = list(ex.map(_compile, sources()))
+        host_obj, torch_libs = host.result()
     objs = [os.path.join(OBJ, s[:-3] + ".o") for s in sources()]
     if (not os.path.exists(LIB)) or any(os.path.getmtime(o) > os.path.getmtime(LIB) for o in objs):
         r = subprocess.run([NVCC, "-shared", "-o", LIB, *objs, "-lcudart"], capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    if (not os.path.exists(HOST_LIB)) or any(os.path.getmtime(o) > os.path.getmtime(HOST_LIB) for o in (host_obj, LIB)):
+        r = subprocess.run(["g++", "-shared", "-o", HOST_LIB, host_obj, f"-L{HERE}", "-llinquant_b200", *[f"-L{d}" for d in torch_libs], "-ltorch_python",
+                            "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN"],
+                           capture_output=True, text=True)
+        if r.returncode != 0:
+            raise RuntimeError(f"link of _host failed:\n{r.stdout}\n{r.stderr}")
     if verbose:
         for s, log in logs:
             if log:

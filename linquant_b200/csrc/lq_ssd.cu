@@ -1013,6 +1013,46 @@ extern "C" int lq_ssd_chunk_scan(const lq_ssd_problem* p, lq_stream stream) {
   return p->N == 128 ? launch_scan<__nv_bfloat16, 128>(p, st) : launch_scan<__nv_bfloat16, 64>(p, st);
 }
 
+// ---- the whole forward on one carved block of scratch
+static size_t carve_combined(lq_ssd_problem& p, void* ws) {
+  size_t off = 0;
+  auto take = [&](size_t n) {
+    uint8_t* r = ws ? reinterpret_cast<uint8_t*>(ws) + off : nullptr;
+    off += (n + 255) & ~size_t(255);
+    return r;
+  };
+  const size_t ht = (size_t)p.B * p.H * p.L, nc = p.L / p.chunk, st = (size_t)p.B * nc * p.H * p.P * p.N;
+  p.dt = reinterpret_cast<float*>(take(ht * sizeof(float)));
+  p.dA = reinterpret_cast<float*>(take(ht * sizeof(float)));
+  p.states = reinterpret_cast<int8_t*>(take(st));
+  p.passed = reinterpret_cast<int8_t*>(take(st));
+  p.final_state = reinterpret_cast<int8_t*>(take((size_t)p.B * p.H * p.P * p.N));
+  p.cb = reinterpret_cast<int8_t*>(take((size_t)p.B * p.L * p.G * p.chunk));
+  // the transposed q_B: only the shapes without the transposition-free chunk state read it
+  p.q_BT = chunk_state_value_tc2_applies(&p) ? nullptr : reinterpret_cast<int8_t*>(take((size_t)p.B * p.L * p.G * p.N));
+  return off;
+}
+extern "C" size_t lq_ssd_combined_workspace_bytes(const lq_ssd_problem* p) {
+  if (!p || p->chunk <= 0 || p->B <= 0 || p->L <= 0 || p->H <= 0 || p->G <= 0 || p->P <= 0 || p->N <= 0) return 0;
+  lq_ssd_problem q = *p;
+  return carve_combined(q, nullptr);
+}
+extern "C" int lq_ssd_combined_fwd(const lq_ssd_problem* p, int keyside, void* workspace, size_t workspace_bytes, lq_stream stream) {
+  if (int e = ssd_check(p, "ssd_combined")) return e;
+  if (int e = ssd_check_pn(p, "ssd_combined")) return e;
+  if (!workspace) return fail(LQ_ERR_NULL, "ssd_combined: workspace is null");
+  if (reinterpret_cast<uintptr_t>(workspace) & 255u) return fail(LQ_ERR_ALIGN, "ssd_combined: workspace must be 256-byte aligned");
+  lq_ssd_problem q = *p;
+  const size_t need = carve_combined(q, workspace);
+  if (workspace_bytes < need) return fail(LQ_ERR_WORKSPACE, "ssd_combined: workspace holds %zu bytes, %zu needed", workspace_bytes, need);
+  q.carry_in = nullptr; q.carry_out = nullptr; q.wait_flags = nullptr; q.post_flags = nullptr;
+  if (int e = lq_ssd_chunk_cumsum(&q, stream)) return e;
+  if (int e = ssd_chunk_state(&q, keyside != 0, stream)) return e;
+  if (int e = lq_ssd_state_passing(&q, stream)) return e;
+  if (int e = lq_ssd_bmm_chunk(&q, keyside, stream)) return e;
+  return lq_ssd_chunk_scan(&q, stream);
+}
+
 template <typename T, bool QUANT>
 static int launch_rotate(const T* x, long long sb, long long stt, long long ob, long long oc, int B, int T_len, int G, int N,
                          int gy, const float* signs, const float* ib, const float* ic, const float* db, const float* dc,

@@ -27,6 +27,11 @@ def kronecker_hadamard_fwd(x, signs, num_heads, n_chunks=2):
         raise _cabi.LinQuantError("kronecker_hadamard_fwd runs on CUDA tensors only (no CPU path)")
     if n_chunks != 2:
         raise NotImplementedError("only the H_2 (x) H_{D/2} factorisation is implemented")
+    y = _cabi.host().hadamard(x, signs)
+    if y is not None:
+        if type(y) is int:
+            _cabi.check(y, "lq_kronecker_hadamard")
+        return y
     B, T, H, D = x.shape
     assert D >= 64, f"Kronecker Hadamard needs D >= 64, got {D}"
     if x.stride(-1) != 1 or x.stride(2) != D or x.stride(0) != T * x.stride(1):

@@ -19,6 +19,12 @@ def fused_split_rotate_quant_xBC(xBC, r_signs, nheads, ngroups, d_state, headdim
     dqk_b / dqk_c (G,N) or None. Returns (x view (B,T,H,P), q_B int8 (B,T,G,N), q_C int8 (B,T,G,N))."""
     if not xBC.is_cuda:
         raise _cabi.LinQuantError("fused_split_rotate_quant_xBC runs on CUDA tensors only (no CPU path)")
+    if dqk_b is None and dqk_c is None:
+        r = _cabi.host().split_rotate(xBC, r_signs, nheads, ngroups, d_state, headdim, B_inv_scale, C_inv_scale)
+        if r is not None:
+            if type(r) is int:
+                _cabi.check(r, "lq_ssd_split_rotate_quant")
+            return r
     batch, seq_len, xBC_dim = xBC.shape
     d_ssm, g_n = nheads * headdim, ngroups * d_state
     assert xBC_dim == d_ssm + 2 * g_n, f"xBC_dim={xBC_dim} != {d_ssm + 2 * g_n}"

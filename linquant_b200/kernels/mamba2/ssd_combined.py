@@ -2,6 +2,7 @@
 (``linquant/kernels/mamba2/ssd_combined.py:19-131``). The five sub-ops are module attributes under the reference's
 names, so callers that wrap or replace them by name keep working."""
 
+from ... import _cabi
 from .bmm_chunk import _quant_bmm_chunk_fwd
 from .chunk_cumsum import _quant_chunk_cumsum_fwd
 from .chunk_scan_v2 import _quant_chunk_scan_fwd as _chunk_scan_v2
@@ -10,6 +11,8 @@ from .chunk_state_keyside import _chunk_state_keyside_fwd
 from .state_passing import _fixedpoint_state_passing_fwd
 
 _GATE_SHIFT = 7  # Q0.7 fixed-point gate
+_SUB_OPS = (_quant_bmm_chunk_fwd, _quant_chunk_cumsum_fwd, _chunk_scan_v2, _quant_chunk_state_fwd_xfp_static_int8,
+            _chunk_state_keyside_fwd, _fixedpoint_state_passing_fwd)
 
 
 def _quant_mamba_chunk_scan_combined_fwd(x_fp, q_dt, dt_scale, q_A_log, A_log_scale, q_B, B_scale, q_C, C_scale,
@@ -21,6 +24,16 @@ def _quant_mamba_chunk_scan_combined_fwd(x_fp, q_dt, dt_scale, q_A_log, A_log_sc
     side: INT8 x with ``x_scale_hp`` against the gate-weighted ``b_fp`` quantised with ``b_gate_scale``), INT32
     fixed-point recurrence, INT8 CB on ``static_cb_scale``, INT8 chunk scan. Returns (out fp16 [B,L,H,P], None).
     ``_link`` (not in the reference signature) is the sequence-parallel hand-off of ``linquant_b200.seqpar``."""
+    # one native call for the whole forward, unless a sub-op has been replaced or the sequence-parallel hand-off is on
+    if _link is None and _SUB_OPS == (_quant_bmm_chunk_fwd, _quant_chunk_cumsum_fwd, _chunk_scan_v2, _quant_chunk_state_fwd_xfp_static_int8,
+                                      _chunk_state_keyside_fwd, _fixedpoint_state_passing_fwd):
+        out = _cabi.host().ssd_fwd(x_fp, q_dt, dt_scale, q_A_log, A_log_scale, q_B, B_scale, q_C, C_scale, chunk_size, q_D, D_scale,
+                                   dt_bias, dt_softplus, dt_limit[0], dt_limit[1], static_state_scale, static_cb_scale, alpha_hp,
+                                   bscale_g, keyside, x_scale_hp, b_fp, b_gate_scale)
+        if out is not None:
+            if type(out) is int:
+                _cabi.check(out, "lq_ssd_combined_fwd")
+            return out, None
     batch, seqlen, nheads, headdim = x_fp.shape
     _, _, ngroups, dstate = q_B.shape
     dA_cumsum, dt = _quant_chunk_cumsum_fwd(q_dt, dt_scale, q_A_log, A_log_scale, chunk_size, dt_bias=dt_bias,

@@ -69,6 +69,38 @@ def make_problem(q, k, v, g, beta, scales, *, decay, eta, sigma, tau, scale, chu
     return P
 
 
+CELLS = {"lq_simple_gla_fwd": 0, "lq_gla_fwd": 1, "lq_delta_fwd": 2, "lq_kda_fwd": 3}
+
+
+def call(entry, q, k, v, g, beta, scales, eta, sigma, tau, scale, chunk_size, output_final_state, unrot, bits, out_dtype, rot,
+         dqk, initial_state, debug):
+    """One whole-call entry on torch tensors. The native host path takes every call whose tensors are in the kernels' form
+    (or need no more than an fp32 / dense copy); anything else, and a call that wants its workspace back, goes through the
+    descriptor below."""
+    if rot is not None and not (isinstance(rot, torch.Tensor) and rot.dim() == 1):
+        rot = signs_of(rot, q.shape[-1], q.device)
+    if debug is None:
+        r = _cabi.host().zoo_fwd(CELLS[entry], q, k, v, g, beta, scales, eta, sigma, tau, scale, chunk_size, output_final_state,
+                                 unrot, bits, out_dtype, rot, dqk, initial_state)
+        if type(r) is tuple:
+            return r
+        if r is not None:
+            _cabi.check(r, entry)
+    q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
+    B, T, H, K = q.shape
+    V = v.shape[-1]
+    assert T % chunk_size == 0 and K <= 128, f"T={T} must be a multiple of the chunk size {chunk_size}, K={K} at most 128"
+    o = torch.empty(v.shape, dtype=out_dtype or v.dtype, device=v.device)
+    ht = torch.empty(B, H, K, V, dtype=torch.float32, device=q.device) if output_final_state else None
+    keep = []
+    decay = _cabi.DECAY_DIAGONAL if CELLS[entry] & 1 else _cabi.DECAY_NONE if g is None else _cabi.DECAY_SCALAR
+    P = make_problem(q, k, v, g, beta, scales, decay=decay, eta=eta, sigma=sigma, tau=tau,
+                     scale=K**-0.5 if scale is None else scale, chunk_size=chunk_size, bits=bits, out=o, final_state=ht,
+                     rot_signs=signs_of(rot, K, q.device), dqk=dqk, keep=keep, unrot=unrot, initial_state=initial_state)
+    run(entry, P, CELLS[entry] >= 2, q, debug)
+    return o, ht
+
+
 def run(entry, P, delta, like, debug=None):
     L = _cabi.lib()
     ws = _cabi.Workspace(P, delta, like.device)

@@ -5,8 +5,6 @@ Same call as ``linquant/kernels/zoo/gated_delta_rule.py:159-203``; the device wo
 
 from __future__ import annotations
 
-import torch
-
 from . import _common
 from ... import _cabi
 
@@ -23,16 +21,5 @@ def chunk_delta_int8(q, k, v, g, beta, scales, *, sigma=1.0, tau=1.0, eta=1.0, s
     Returns (o, final fp32 state [B,H,K,V] or None)."""
     if not q.is_cuda:
         raise _cabi.LinQuantError("chunk_delta_int8 runs on CUDA tensors only (no CPU path)")
-    q, k, v, beta = q.contiguous(), k.contiguous(), v.contiguous(), beta.contiguous()
-    B, T, H, K = q.shape
-    V = v.shape[-1]
-    assert T % chunk_size == 0 and K <= 128
-    scale = K**-0.5 if scale is None else scale
-    o = torch.empty(v.shape, dtype=out_dtype or v.dtype, device=v.device)
-    ht = torch.empty(B, H, K, V, dtype=torch.float32, device=q.device) if output_final_state else None
-    keep = []
-    P = _common.make_problem(q, k, v, g, beta, scales, decay=_cabi.DECAY_NONE if g is None else _cabi.DECAY_SCALAR,
-                             eta=eta, sigma=sigma, tau=tau, scale=scale, chunk_size=chunk_size, bits=bits, out=o,
-                             final_state=ht, rot_signs=_common.signs_of(rot, K, q.device), dqk=dqk, keep=keep, unrot=unrot, initial_state=initial_state)
-    _common.run("lq_delta_fwd", P, True, q, _debug)
-    return o, ht
+    return _common.call("lq_delta_fwd", q, k, v, g, beta, scales, eta, sigma, tau, scale, chunk_size, output_final_state, unrot,
+                        bits, out_dtype, rot, dqk, initial_state, _debug)

@@ -5,8 +5,6 @@ Same call as ``linquant/kernels/zoo/gla.py:235-279``; the device work is the C-A
 
 from __future__ import annotations
 
-import torch
-
 from . import _common
 from ... import _cabi
 
@@ -22,16 +20,6 @@ def chunk_gla_int8(q, k, v, g, scales, *, eta=0.0, scale=None, chunk_size=64, ou
     Returns (o [B,T,H,V] in v.dtype or out_dtype, final fp32 state [B,H,K,V] or None)."""
     if not q.is_cuda:
         raise _cabi.LinQuantError("chunk_gla_int8 runs on CUDA tensors only (no CPU path)")
-    q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-    B, T, H, K = q.shape
-    V = v.shape[-1]
-    assert T % chunk_size == 0 and K <= 128 and chunk_size % BC == 0
-    scale = K**-0.5 if scale is None else scale
-    o = torch.empty(v.shape, dtype=out_dtype or v.dtype, device=v.device)
-    ht = torch.empty(B, H, K, V, dtype=torch.float32, device=q.device) if output_final_state else None
-    keep = []
-    P = _common.make_problem(q, k, v, g, None, scales, decay=_cabi.DECAY_DIAGONAL, eta=eta, sigma=1.0, tau=1.0,
-                             scale=scale, chunk_size=chunk_size, bits=bits, out=o, final_state=ht,
-                             rot_signs=_common.signs_of(rot, K, q.device), dqk=None, keep=keep, unrot=unrot, initial_state=initial_state)
-    _common.run("lq_gla_fwd", P, False, q, _debug)
-    return o, ht
+    assert chunk_size % BC == 0
+    return _common.call("lq_gla_fwd", q, k, v, g, None, scales, eta, 1.0, 1.0, scale, chunk_size, output_final_state, unrot, bits,
+                        out_dtype, rot, None, initial_state, _debug)

@@ -5,8 +5,6 @@ Same call as ``linquant/kernels/zoo/kda.py:154-203``; the device work is the C-A
 
 from __future__ import annotations
 
-import torch
-
 from . import _common
 from ... import _cabi
 from .gla import BC
@@ -22,16 +20,6 @@ def chunk_kda_int8(q, k, v, g, beta, scales, *, sigma=1.0, tau=1.0, eta=0.0, sca
     Returns (o [B,T,H,V] in v.dtype or out_dtype, final fp32 state or None)."""
     if not q.is_cuda:
         raise _cabi.LinQuantError("chunk_kda_int8 runs on CUDA tensors only (no CPU path)")
-    q, k, v, beta = q.contiguous(), k.contiguous(), v.contiguous(), beta.contiguous()
-    B, T, H, K = q.shape
-    V = v.shape[-1]
-    assert T % chunk_size == 0 and K <= 128 and chunk_size % BC == 0
-    scale = K**-0.5 if scale is None else scale
-    o = torch.empty(v.shape, dtype=out_dtype or v.dtype, device=v.device)
-    ht = torch.empty(B, H, K, V, dtype=torch.float32, device=q.device) if output_final_state else None
-    keep = []
-    P = _common.make_problem(q, k, v, g, beta, scales, decay=_cabi.DECAY_DIAGONAL, eta=eta, sigma=sigma, tau=tau,
-                             scale=scale, chunk_size=chunk_size, bits=bits, out=o, final_state=ht,
-                             rot_signs=_common.signs_of(rot, K, q.device), dqk=None, keep=keep, unrot=unrot, initial_state=initial_state)
-    _common.run("lq_kda_fwd", P, True, q, _debug)
-    return o, ht
+    assert chunk_size % BC == 0
+    return _common.call("lq_kda_fwd", q, k, v, g, beta, scales, eta, sigma, tau, scale, chunk_size, output_final_state, unrot, bits,
+                        out_dtype, rot, None, initial_state, _debug)

@@ -5,8 +5,6 @@ Same call as ``linquant/kernels/zoo/simple_gla.py:175-212``; the device work is 
 
 from __future__ import annotations
 
-import torch
-
 from . import _common
 from ... import _cabi
 
@@ -24,17 +22,5 @@ def chunk_simple_gla_int8(q, k, v, g, scales, *, eta=1.0, scale=None, chunk_size
     Returns (o [B,T,H,V] in v.dtype or out_dtype, final fp32 state [B,H,K,V] or None)."""
     if not q.is_cuda:
         raise _cabi.LinQuantError("chunk_simple_gla_int8 runs on CUDA tensors only (no CPU path)")
-    q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-    B, T, H, K = q.shape
-    V = v.shape[-1]
-    assert T % chunk_size == 0, f"T={T} must be a multiple of the chunk size {chunk_size}"
-    scale = K**-0.5 if scale is None else scale
-    o = torch.empty(v.shape, dtype=out_dtype or v.dtype, device=v.device)
-    ht = torch.empty(B, H, K, V, dtype=torch.float32, device=q.device) if output_final_state else None
-    keep = []
-    P = _common.make_problem(q, k, v, g, None, scales, decay=_cabi.DECAY_NONE if g is None else _cabi.DECAY_SCALAR,
-                             eta=eta, sigma=1.0, tau=1.0, scale=scale, chunk_size=chunk_size, bits=bits, out=o,
-                             final_state=ht, rot_signs=_common.signs_of(rot, K, q.device), dqk=dqk, keep=keep,
-                             initial_state=initial_state, unrot=unrot)
-    _common.run("lq_simple_gla_fwd", P, False, q, _debug)
-    return o, ht
+    return _common.call("lq_simple_gla_fwd", q, k, v, g, None, scales, eta, 1.0, 1.0, scale, chunk_size, output_final_state, unrot,
+                        bits, out_dtype, rot, dqk, initial_state, _debug)
