@@ -25,6 +25,7 @@ __device__ __forceinline__ int round_rint(float y, float lo, float hi) {
 // index contiguous. The running sum is kept in double and rounded to fp32 per prefix: a warp scan per 32 tokens plus a
 // carry.
 __global__ void __launch_bounds__(1024) ssd_cumsum_kernel(lq_ssd_problem p) {
+  pdl_enter();
   extern __shared__ float s_dtv[];  // [C][H + 1]
   const int c = blockIdx.x, b = blockIdx.y;
   const int C = p.chunk, NC = p.L / C, H = p.H, LD = H + 1;
@@ -75,6 +76,7 @@ __global__ void __launch_bounds__(1024) ssd_cumsum_kernel(lq_ssd_problem p) {
 // q_B [B,L,G,N] -> q_BT [B,NC,G,N,C] (token index contiguous) so both operands of the value-side chunk-state
 // product have the reduction index contiguous. One CTA per (64-token block, group, batch).
 __global__ void __launch_bounds__(256) ssd_transpose_b_kernel(const int8_t* qB, int8_t* qBT, int L, int G, int N, int C) {
+  pdl_enter();
   __shared__ uint32_t s[128][17];
   const int blk = blockIdx.x, g = blockIdx.y, b = blockIdx.z;
   const int t0 = blk * 64;
@@ -137,6 +139,7 @@ __device__ __forceinline__ void st_release_sys(unsigned* p, unsigned v) {
 __global__ void __launch_bounds__(256) ssd_state_passing_kernel(const int8_t* states, const float* dA, int8_t* out,
                                                                 int8_t* final_state, int H, int NC, int C, int D,
                                                                 PassingLink link) {
+  pdl_enter();
   extern __shared__ int s_gq[];  // [NC] Q0.7 gate of every chunk: the serial loop must not wait on its loads
   __shared__ int s_ok;
   const int h = blockIdx.y, b = blockIdx.z;
@@ -229,6 +232,7 @@ __global__ void __launch_bounds__(256) ssd_state_passing_kernel(const int8_t* st
 //   key side    mamba2/chunk_state_keyside.py:267-321  xq = rint(x / x_scale_p), Bq = rint(B*gate_k*127/bg_n), rint requant
 template <typename T, int N, bool KEYSIDE>
 __global__ void __launch_bounds__(128) ssd_chunk_state_kernel(lq_ssd_problem p) {
+  pdl_enter();
   constexpr int P = 64, LDW = 20;
   __shared__ __align__(16) uint32_t s_x[2][P][LDW];
   __shared__ __align__(16) uint32_t s_b[KEYSIDE ? 2 : 1][KEYSIDE ? N : 1][LDW];
@@ -392,6 +396,7 @@ __global__ void __launch_bounds__(128) ssd_chunk_state_kernel(lq_ssd_problem p) 
 // operands). B_IS_FP quantises B in the fragment load: rint(b / s_B), clamp +-127.
 template <typename T, int N, bool B_IS_FP>
 __global__ void __launch_bounds__(128) ssd_bmm_kernel(lq_ssd_problem p) {
+  pdl_enter();
   const int C = p.chunk, NC = p.L / C;
   const int tiles = C / 64;
   const int m0 = (blockIdx.x / tiles) * 64, n0 = (blockIdx.x % tiles) * 64;
@@ -503,6 +508,7 @@ __device__ __forceinline__ void scan_kstep(float (&conv)[8][4], const uint32_t (
 
 template <typename T, int N>
 __global__ void __launch_bounds__(256, 2) ssd_chunk_scan_kernel(lq_ssd_problem p) {
+  pdl_enter();
   constexpr int P = 64;
   extern __shared__ __align__(128) uint8_t smem[];
   const int C = p.chunk, NC = p.L / C;
@@ -751,6 +757,7 @@ __global__ void __launch_bounds__(256) ssd_rotate_rows_kernel(const T* x, long l
                                                               const float* signs, const float* inv_b, const float* inv_c,
                                                               const float* dqk_b, const float* dqk_c, int8_t* q_b,
                                                               int8_t* q_c, T* y, int rows_per_cta) {
+  pdl_enter();
   // QUANT: blockIdx.y in [0, 2G) selects (B|C, group); otherwise blockIdx.y is the head and y is the dense output.
   // A CTA walks rows_per_cta consecutive tokens: a row is short (N values), so the per-row constants (signs, D_QK,
   // reciprocal scale) are loaded once per thread and four rows per thread are in flight at a time.
@@ -836,7 +843,7 @@ template <typename T, int N, bool KEYSIDE>
 static void launch_chunk_state_T(const lq_ssd_problem* p, dim3 grid, cudaStream_t st) {
   const int smem = p->chunk * 128;  // static + dynamic shared memory exceeds 48 KB on the key side: opt in
   cudaFuncSetAttribute(ssd_chunk_state_kernel<T, N, KEYSIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-  ssd_chunk_state_kernel<T, N, KEYSIDE><<<grid, 128, smem, st>>>(*p);
+  launch(ssd_chunk_state_kernel<T, N, KEYSIDE>, grid, 128, smem, st, *p);
 }
 template <bool KEYSIDE>
 static void launch_chunk_state(const lq_ssd_problem* p, dim3 grid, cudaStream_t st) {
@@ -851,11 +858,11 @@ static void launch_chunk_state(const lq_ssd_problem* p, dim3 grid, cudaStream_t 
 template <bool B_IS_FP>
 static void launch_bmm(const lq_ssd_problem* p, dim3 grid, cudaStream_t st) {
   if (p->x_dtype == LQ_BF16) {
-    if (p->N == 128) ssd_bmm_kernel<__nv_bfloat16, 128, B_IS_FP><<<grid, 128, 0, st>>>(*p);
-    else ssd_bmm_kernel<__nv_bfloat16, 64, B_IS_FP><<<grid, 128, 0, st>>>(*p);
+    if (p->N == 128) launch(ssd_bmm_kernel<__nv_bfloat16, 128, B_IS_FP>, grid, 128, 0, st, *p);
+    else launch(ssd_bmm_kernel<__nv_bfloat16, 64, B_IS_FP>, grid, 128, 0, st, *p);
   } else {
-    if (p->N == 128) ssd_bmm_kernel<__half, 128, B_IS_FP><<<grid, 128, 0, st>>>(*p);
-    else ssd_bmm_kernel<__half, 64, B_IS_FP><<<grid, 128, 0, st>>>(*p);
+    if (p->N == 128) launch(ssd_bmm_kernel<__half, 128, B_IS_FP>, grid, 128, 0, st, *p);
+    else launch(ssd_bmm_kernel<__half, 64, B_IS_FP>, grid, 128, 0, st, *p);
   }
 }
 
@@ -869,7 +876,7 @@ extern "C" int lq_ssd_chunk_cumsum(const lq_ssd_problem* p, lq_stream stream) {
   const size_t smem = (size_t)p->chunk * (p->H + 1) * sizeof(float);
   if (smem > 200 * 1024) return fail(LQ_ERR_UNSUPPORTED, "chunk_cumsum: chunk * nheads = %d * %d exceeds the shared-memory tile", p->chunk, p->H);
   cudaFuncSetAttribute(ssd_cumsum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  ssd_cumsum_kernel<<<dim3(p->L / p->chunk, p->B), 1024, smem, (cudaStream_t)stream>>>(*p);
+  launch(ssd_cumsum_kernel, dim3(p->L / p->chunk, p->B), 1024, smem, (cudaStream_t)stream, *p);
   return check_launch("ssd_cumsum_kernel");
 }
 
@@ -885,7 +892,7 @@ extern "C" int lq_ssd_state_passing(const lq_ssd_problem* p, lq_stream stream) {
   dim3 grid((D / 8 + 255) / 256, p->H, p->B);
   if ((size_t)(p->L / p->chunk) * sizeof(int) > 48 * 1024) return fail(LQ_ERR_UNSUPPORTED, "state_passing: more than 12288 chunks");
   PassingLink link{p->carry_in, p->carry_out, p->wait_flags, p->post_flags, p->epoch, p->wait_ns, p->status};
-  ssd_state_passing_kernel<<<grid, 256, (size_t)(p->L / p->chunk) * sizeof(int), (cudaStream_t)stream>>>(p->states, p->dA, p->passed, p->final_state, p->H,
+  launch(ssd_state_passing_kernel, grid, 256, (size_t)(p->L / p->chunk) * sizeof(int), (cudaStream_t)stream, p->states, p->dA, p->passed, p->final_state, p->H,
                                                                     p->L / p->chunk, p->chunk, D, link);
   return check_launch("ssd_state_passing_kernel");
 }
@@ -918,7 +925,7 @@ static int ssd_chunk_state(const lq_ssd_problem* p, bool keyside, lq_stream stre
     // d_state 128 with chunks of 128 / 256 tokens: both tcgen05 operands in their natural layouts, no scratch at all
     if (!with_qbt && chunk_state_value_tc2_applies(p)) return run_chunk_state_value_tc2(p, p->status, st);
     if (!p->q_BT) return fail(LQ_ERR_NULL, "%s: q_BT (scratch for the transposed q_B) required for this shape", what);
-    ssd_transpose_b_kernel<<<dim3(p->L / 64, p->G, p->B), 256, 0, st>>>(p->q_B, p->q_BT, p->L, p->G, p->N, p->chunk);
+    launch(ssd_transpose_b_kernel, dim3(p->L / 64, p->G, p->B), 256, 0, st, p->q_B, p->q_BT, p->L, p->G, p->N, p->chunk);
     if (int e = check_launch("ssd_transpose_b_kernel")) return e;
     // chunks of 128 or 256 tokens run on tcgen05 + TMA; 64- and 192-token chunks on the warp-level MMA kernel
     if (p->chunk % 128 == 0) return run_chunk_state_value_tc(p, p->status, st);
@@ -994,7 +1001,7 @@ static int launch_scan(const lq_ssd_problem* p, cudaStream_t st) {
   const size_t smem = (size_t)p->chunk * 128 + 6 * sizeof(float) * p->chunk + (size_t)64 * N + 128 * sizeof(float);
   dim3 grid(p->L / p->chunk, p->H, p->B);
   cudaFuncSetAttribute(ssd_chunk_scan_kernel<T, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
-  ssd_chunk_scan_kernel<T, N><<<grid, 256, smem, st>>>(*p);
+  launch(ssd_chunk_scan_kernel<T, N>, grid, 256, smem, st, *p);
   return check_launch("ssd_chunk_scan_kernel");
 }
 extern "C" int lq_ssd_chunk_scan(const lq_ssd_problem* p, lq_stream stream) {
@@ -1061,8 +1068,8 @@ static int launch_rotate(const T* x, long long sb, long long stt, long long ob, 
   int rows_per_cta = 256;
   while (rows_per_cta > 64 && (long long)((T_len + rows_per_cta - 1) / rows_per_cta) * gy * B < 592) rows_per_cta >>= 1;
   dim3 grid((T_len + rows_per_cta - 1) / rows_per_cta, gy, B);
-  if (N == 128) ssd_rotate_rows_kernel<T, 128, QUANT><<<grid, 256, 0, st>>>(x, sb, stt, ob, oc, T_len, G, signs, ib, ic, db, dc, qb, qc, y, rows_per_cta);
-  else if (N == 64) ssd_rotate_rows_kernel<T, 64, QUANT><<<grid, 256, 0, st>>>(x, sb, stt, ob, oc, T_len, G, signs, ib, ic, db, dc, qb, qc, y, rows_per_cta);
+  if (N == 128) launch(ssd_rotate_rows_kernel<T, 128, QUANT>, grid, 256, 0, st, x, sb, stt, ob, oc, T_len, G, signs, ib, ic, db, dc, qb, qc, y, rows_per_cta);
+  else if (N == 64) launch(ssd_rotate_rows_kernel<T, 64, QUANT>, grid, 256, 0, st, x, sb, stt, ob, oc, T_len, G, signs, ib, ic, db, dc, qb, qc, y, rows_per_cta);
   else return fail(LQ_ERR_UNSUPPORTED, "Hadamard rows: width %d (64 or 128 supported)", N);
   return check_launch("ssd_rotate_rows_kernel");
 }

@@ -31,6 +31,7 @@ __device__ __forceinline__ void sts64(uint32_t addr, uint32_t a, uint32_t b) {
 template <typename T, int C, bool B_IS_FP>
 __global__ void __launch_bounds__(256, 1) ssd_bmm_tc_kernel(const __grid_constant__ CUtensorMap tm_c,
                                                            const __grid_constant__ CUtensorMap tm_b, lq_ssd_problem p, int* status) {
+  pdl_enter();
   using namespace bmmtc;
   constexpr int N = 128, MB = C / 128, COLS = C * MB;  // accumulator columns: one [128 x C] block per 128 rows of C_q
   const int NC = p.L / C;
@@ -154,7 +155,7 @@ static int launch_bmm_tc(const lq_ssd_problem* p, const CUtensorMap& tc, const C
   cudaError_t e = cudaFuncSetAttribute(ssd_bmm_tc_kernel<T, C, B_IS_FP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return fail(LQ_ERR_LAUNCH, "bmm_chunk: shared memory opt-in failed: %s", cudaGetErrorString(e));
   dim3 grid((p->L / C) * p->G, p->B);
-  ssd_bmm_tc_kernel<T, C, B_IS_FP><<<grid, 256, smem, st>>>(tc, tb, *p, status);
+  launch(ssd_bmm_tc_kernel<T, C, B_IS_FP>, grid, 256, smem, st, tc, tb, *p, status);
   return check_launch("ssd_bmm_tc_kernel");
 }
 

@@ -157,6 +157,7 @@ __global__ void __launch_bounds__(576, 1) ssd_chunk_scan_tc_kernel(const __grid_
                                                                   const __grid_constant__ CUtensorMap tm_x,
                                                                   const __grid_constant__ CUtensorMap tm_out, lq_ssd_problem p,
                                                                   int* status, int n_items) {
+  pdl_enter();
   using namespace scantc;
   constexpr int P = 64, N = 128, C = 128 * MB, NT = MB == 2 ? 6 : 2;
   constexpr bool XBF16 = !std::is_same<T, __half>::value;
@@ -548,7 +549,7 @@ template <typename T, int MB>
 static cudaError_t launch_scan_tc(int grid, size_t smem, cudaStream_t st, const CUtensorMap& tq, const CUtensorMap& ts, const CUtensorMap& tx,
                              const CUtensorMap& to, const lq_ssd_problem* p, int* status, int items) {
   cudaError_t e = cudaFuncSetAttribute(ssd_chunk_scan_tc_kernel<T, MB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess) ssd_chunk_scan_tc_kernel<T, MB><<<grid, scantc::kWorkers + 64, smem, st>>>(tq, ts, tx, to, *p, status, items);
+  if (e == cudaSuccess) launch(ssd_chunk_scan_tc_kernel<T, MB>, grid, scantc::kWorkers + 64, smem, st, tq, ts, tx, to, *p, status, items);
   return e;
 }
 

@@ -52,6 +52,7 @@ __device__ __forceinline__ int code_rint127(float y) { return __float2int_rn(fmi
 template <typename T, int C>
 __global__ void __launch_bounds__(256, 2) ssd_chunk_state_key_tc_kernel(const __grid_constant__ CUtensorMap tm_out, lq_ssd_problem p,
                                                                        int* status) {
+  pdl_enter();
   using namespace statekey;
   constexpr int P = 64, N = 128;
   const int NC = p.L / C;
@@ -225,7 +226,7 @@ static int launch_state_key_tc(const lq_ssd_problem* p, const CUtensorMap& to, i
   cudaError_t e = cudaFuncSetAttribute(ssd_chunk_state_key_tc_kernel<T, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return fail(LQ_ERR_LAUNCH, "chunk_state_key: shared memory opt-in failed: %s", cudaGetErrorString(e));
   dim3 grid(p->L / C, p->H / 2, p->B);
-  ssd_chunk_state_key_tc_kernel<T, C><<<grid, 256, smem, st>>>(to, *p, status);
+  launch(ssd_chunk_state_key_tc_kernel<T, C>, grid, 256, smem, st, to, *p, status);
   return check_launch("ssd_chunk_state_key_tc_kernel");
 }
 

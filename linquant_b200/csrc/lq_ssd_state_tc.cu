@@ -30,6 +30,7 @@ __device__ __forceinline__ int ssd_half_away(float y, float lim) {
 template <typename T, int N>
 __global__ void __launch_bounds__(128) ssd_chunk_state_tc_kernel(const __grid_constant__ CUtensorMap tm_b, lq_ssd_problem p,
                                                                  int* status) {
+  pdl_enter();
   constexpr int P = 64;
   const int C = p.chunk, KB = C >> 7, NC = p.L / C;
   extern __shared__ uint8_t smem_dyn[];
@@ -208,7 +209,7 @@ static int launch_state_tc(const lq_ssd_problem* p, int* status, cudaStream_t st
   cudaError_t e = cudaFuncSetAttribute(ssd_chunk_state_tc_kernel<T, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return fail(LQ_ERR_LAUNCH, "chunk_state: shared memory opt-in failed: %s", cudaGetErrorString(e));
   dim3 grid(NC, p->H, p->B);
-  ssd_chunk_state_tc_kernel<T, N><<<grid, 128, smem, st>>>(tm, *p, status);
+  launch(ssd_chunk_state_tc_kernel<T, N>, grid, 128, smem, st, tm, *p, status);
   return check_launch("ssd_chunk_state_tc_kernel");
 }
 

@@ -55,6 +55,7 @@ template <typename T, int C>
 __global__ void __launch_bounds__(256, 3) ssd_chunk_state_tc2_kernel(const __grid_constant__ CUtensorMap tm_b,
                                                                     const __grid_constant__ CUtensorMap tm_out, lq_ssd_problem p,
                                                                     int* status) {
+  pdl_enter();
   using namespace statetc2;
   constexpr int P = 64, N = 128;
   const int NC = p.L / C;
@@ -208,7 +209,7 @@ static int launch_state_tc2(const lq_ssd_problem* p, const CUtensorMap& tb, cons
   cudaError_t e = cudaFuncSetAttribute(ssd_chunk_state_tc2_kernel<T, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return fail(LQ_ERR_LAUNCH, "chunk_state: shared memory opt-in failed: %s", cudaGetErrorString(e));
   dim3 grid(p->L / C, p->H / 2, p->B);
-  ssd_chunk_state_tc2_kernel<T, C><<<grid, 256, smem, st>>>(tb, to, *p, status);
+  launch(ssd_chunk_state_tc2_kernel<T, C>, grid, 256, smem, st, tb, to, *p, status);
   return check_launch("ssd_chunk_state_tc2_kernel");
 }
 

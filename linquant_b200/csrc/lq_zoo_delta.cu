@@ -34,6 +34,7 @@ struct DeltaPrepArgs {
 
 template <typename T, int K, int V>
 __global__ void __launch_bounds__(256) zoo_prologue_delta_kernel(DeltaPrepArgs d) {
+  pdl_enter();
   constexpr int C = kChunk, LDK = K + 8, LDV = V + 8;
   extern __shared__ __align__(16) uint8_t smem_raw[];
   float* s_gc = reinterpret_cast<float*>(smem_raw);
@@ -190,6 +191,7 @@ __device__ __forceinline__ int swz_row(int row, int chunk) {
 
 template <typename T, int K, int V, bool DIAG>
 __global__ void __launch_bounds__(128) zoo_state_delta_kernel(DeltaStateArgs a) {
+  pdl_enter();
   constexpr int C = 64, BV = 32;
   constexpr int NTK = K / 32;  // key n-tiles per warp in the carry layout
   constexpr int KK = K / 64;
@@ -420,6 +422,7 @@ __global__ void __launch_bounds__(128) zoo_state_delta_kernel(DeltaStateArgs a) 
 // exactness of the reference's rounding points.
 template <typename T, int K, int V, bool DIAG>
 __global__ void __launch_bounds__(256) zoo_state_delta_unrot_kernel(DeltaStateArgs a, const __half* unrot_t) {
+  pdl_enter();
   constexpr int C = 64, LDH = V + 8, KK = K / 64, KW = K / 16;
   constexpr int NT2 = V / 16;                 // value n-tiles per warp in the read phase (two value halves)
   constexpr int MTV = V / 16, NHALF = 8 / MTV, NTW = (K / 8) / NHALF;  // write product: value m-tile, key n-tiles per warp
@@ -670,7 +673,7 @@ static int launch_delta_prep(const DeltaPrepArgs& d, int BH, cudaStream_t st) {
   constexpr size_t smem = sizeof(float) * (6 * 64 + 64 * (K + 8) + 64 * (V + 8) + 2 * 64 * 68) + sizeof(uint32_t) * K * 17;
   cudaError_t e = cudaFuncSetAttribute(zoo_prologue_delta_kernel<T, K, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return fail(LQ_ERR_LAUNCH, "delta prologue: cannot opt in to %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
-  zoo_prologue_delta_kernel<T, K, V><<<dim3(d.pro.NT, BH), 256, smem, st>>>(d);
+  launch(zoo_prologue_delta_kernel<T, K, V>, dim3(d.pro.NT, BH), 256, smem, st, d);
   return check_launch("zoo_prologue_delta_kernel");
 }
 
@@ -701,10 +704,10 @@ static int launch_delta_state_unrot(const lq_zoo_problem* p, const DeltaStateArg
   cudaError_t e;
   if (p->decay == LQ_DECAY_DIAGONAL) {
     e = cudaFuncSetAttribute(zoo_state_delta_unrot_kernel<T, K, V, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) zoo_state_delta_unrot_kernel<T, K, V, true><<<p->B * p->H, 256, smem, st>>>(a, rt);
+    if (e == cudaSuccess) launch(zoo_state_delta_unrot_kernel<T, K, V, true>, p->B * p->H, 256, smem, st, a, rt);
   } else {
     e = cudaFuncSetAttribute(zoo_state_delta_unrot_kernel<T, K, V, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) zoo_state_delta_unrot_kernel<T, K, V, false><<<p->B * p->H, 256, smem, st>>>(a, rt);
+    if (e == cudaSuccess) launch(zoo_state_delta_unrot_kernel<T, K, V, false>, p->B * p->H, 256, smem, st, a, rt);
   }
   if (e != cudaSuccess) return fail(LQ_ERR_LAUNCH, "delta state (canonical storage): shared memory opt-in failed: %s", cudaGetErrorString(e));
   return check_launch("zoo_state_delta_unrot_kernel");
@@ -722,8 +725,8 @@ static int dispatch_delta_state(const lq_zoo_problem* p, const DeltaStateArgs& a
   dim3 grid(p->V / 32, p->B * p->H), block(128);
   const bool diag = p->decay == LQ_DECAY_DIAGONAL;
 #define LQ_LAUNCH_DSTATE(KK_, VV_)                                                         \
-  if (diag) zoo_state_delta_kernel<T, KK_, VV_, true><<<grid, block, 0, st>>>(a);          \
-  else zoo_state_delta_kernel<T, KK_, VV_, false><<<grid, block, 0, st>>>(a)
+  if (diag) launch(zoo_state_delta_kernel<T, KK_, VV_, true>, grid, block, 0, st, a);          \
+  else launch(zoo_state_delta_kernel<T, KK_, VV_, false>, grid, block, 0, st, a)
   if (p->K == 64 && p->V == 64) { LQ_LAUNCH_DSTATE(64, 64); }
   else if (p->K == 64 && p->V == 128) { LQ_LAUNCH_DSTATE(64, 128); }
   else if (p->K == 128 && p->V == 64) { LQ_LAUNCH_DSTATE(128, 64); }

@@ -50,6 +50,7 @@ __device__ __forceinline__ void load_gc_tile(const float* gc_tile, float* s_gc) 
 // ------------------------------------------------------------------------------------------------ rows
 template <typename T, int K, int V, bool DELTA>
 __global__ void __launch_bounds__(256) zoo_diag_rows_kernel(DiagArgs a) {
+  pdl_enter();
   constexpr int C = 64, LD = K + 4;
   extern __shared__ __align__(16) uint8_t smem_raw[];
   float* s_gc = reinterpret_cast<float*>(smem_raw);
@@ -222,6 +223,7 @@ __global__ void __launch_bounds__(256) zoo_diag_rows_kernel(DiagArgs a) {
 // ------------------------------------------------------------------------------------------------ A matrix
 template <typename T, int K>
 __global__ void __launch_bounds__(256) zoo_diag_amat_kernel(DiagArgs a) {
+  pdl_enter();
   constexpr int C = 64, LD = K + 4, SUB = 16;
   extern __shared__ __align__(16) uint8_t smem_raw[];
   float* s_gc = reinterpret_cast<float*>(smem_raw);
@@ -530,6 +532,7 @@ __device__ __forceinline__ void kda_scaled_rows(const DiagArgs& a, int b, int c,
 
 template <typename T, int K, int V>
 __global__ void __launch_bounds__(256) zoo_kda_wy_kernel(DiagArgs a) {
+  pdl_enter();
   constexpr int C = 64, LD = K + 4, LDV = V + 8, SUB = 16;
   constexpr int REG0 = C * (LD > LDV ? LD : LDV);
   extern __shared__ __align__(16) uint8_t smem_raw[];
@@ -815,7 +818,7 @@ template <typename KernelT>
 static int launch_big_smem(KernelT kern, const char* name, dim3 grid, size_t smem, const DiagArgs& a, cudaStream_t st) {
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return fail(LQ_ERR_LAUNCH, "%s: cannot opt in to %zu bytes of shared memory: %s", name, smem, cudaGetErrorString(e));
-  kern<<<grid, 256, smem, st>>>(a);
+  launch(kern, grid, 256, smem, st, a);
   return check_launch(name);
 }
 

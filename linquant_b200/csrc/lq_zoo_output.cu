@@ -53,6 +53,7 @@ __device__ __forceinline__ void store8<__nv_bfloat16>(__nv_bfloat16* dst, const 
 
 template <int K, int V, typename OT, bool DIAG, bool UNROT>
 __global__ void __launch_bounds__(128) zoo_output_scalar_kernel(OutputArgs a) {
+  pdl_enter();
   constexpr int C = 64, LDR = V + 8;
   constexpr int KK = K / 64;  // 64-byte reduction blocks per row
   extern __shared__ __align__(128) uint8_t smem[];
@@ -255,7 +256,7 @@ static int launch_output(const lq_zoo_problem* p, const OutputArgs& a, cudaStrea
   do {                                                                                                                 \
     auto kern = zoo_output_scalar_kernel<K, V, OT_, DIAG_, UNROT_>;                                                    \
     if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);         \
-    kern<<<grid, block, smem, st>>>(a);                                                                                \
+    launch(kern, grid, block, smem, st, a);                                                                                \
   } while (0)
 #define LQ_LAUNCH_OUT(OT_)                                 \
   if (diag && unrot) LQ_LAUNCH_ONE(OT_, true, true);       \

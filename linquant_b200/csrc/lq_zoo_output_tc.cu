@@ -49,6 +49,7 @@ template <int V, typename OT>
 __global__ void __launch_bounds__(128) zoo_output_tc_kernel(const __grid_constant__ CUtensorMap tm_q,
                                                             const __grid_constant__ CUtensorMap tm_k,
                                                             const __grid_constant__ CUtensorMap tm_h, OutputTcArgs a) {
+  pdl_enter();
   constexpr int C = 64, K = 128;
   constexpr uint32_t TMEM_COLS = 128;  // S2 in [0,64), first 64 state columns in [64,128); the second 64 reuse [0,64)
   extern __shared__ uint8_t smem_dyn[];
@@ -266,9 +267,9 @@ static int launch_output_tc(const lq_zoo_problem* p, const lq_zoo_workspace* ws,
   if (int e = make_map(&th, ws->hT, tiles * V, V)) return e;
   const size_t smem = (size_t)2 * 64 * 128 + (size_t)V * 128 + (size_t)V * 64 + sizeof(float) * (64 + 2 * V) + 64 + 1024;  // + barriers, TMEM base, 1 KiB alignment slack
   dim3 grid(a.NT, p->B * p->H), block(128);
-  if (p->out_dtype == LQ_F16) zoo_output_tc_kernel<V, __half><<<grid, block, smem, st>>>(tq, tk, th, a);
-  else if (p->out_dtype == LQ_BF16) zoo_output_tc_kernel<V, __nv_bfloat16><<<grid, block, smem, st>>>(tq, tk, th, a);
-  else if (p->out_dtype == LQ_F32) zoo_output_tc_kernel<V, float><<<grid, block, smem, st>>>(tq, tk, th, a);
+  if (p->out_dtype == LQ_F16) launch(zoo_output_tc_kernel<V, __half>, grid, block, smem, st, tq, tk, th, a);
+  else if (p->out_dtype == LQ_BF16) launch(zoo_output_tc_kernel<V, __nv_bfloat16>, grid, block, smem, st, tq, tk, th, a);
+  else if (p->out_dtype == LQ_F32) launch(zoo_output_tc_kernel<V, float>, grid, block, smem, st, tq, tk, th, a);
   else return fail(LQ_ERR_UNSUPPORTED, "output: out dtype must be f16, bf16 or f32");
   return check_launch("zoo_output_tc_kernel");
 }

@@ -18,6 +18,7 @@ namespace lq {
 
 template <typename T, int K, int V>
 __global__ void __launch_bounds__(256) zoo_prologue_linear_kernel(PrologueArgs a) {
+  pdl_enter();
   constexpr int C = kChunk;
   __shared__ float s_gc[C], s_fk[C], s_fv[C];
   __shared__ uint32_t s_kw[K][17];
@@ -99,10 +100,10 @@ __global__ void __launch_bounds__(256) zoo_prologue_linear_kernel(PrologueArgs a
 template <typename T>
 static int launch_prologue(const lq_zoo_problem* p, const PrologueArgs& a, cudaStream_t st) {
   dim3 grid(a.NT, p->B * p->H), block(256);
-  if (p->K == 64 && p->V == 64) zoo_prologue_linear_kernel<T, 64, 64><<<grid, block, 0, st>>>(a);
-  else if (p->K == 64 && p->V == 128) zoo_prologue_linear_kernel<T, 64, 128><<<grid, block, 0, st>>>(a);
-  else if (p->K == 128 && p->V == 64) zoo_prologue_linear_kernel<T, 128, 64><<<grid, block, 0, st>>>(a);
-  else if (p->K == 128 && p->V == 128) zoo_prologue_linear_kernel<T, 128, 128><<<grid, block, 0, st>>>(a);
+  if (p->K == 64 && p->V == 64) launch(zoo_prologue_linear_kernel<T, 64, 64>, grid, block, 0, st, a);
+  else if (p->K == 64 && p->V == 128) launch(zoo_prologue_linear_kernel<T, 64, 128>, grid, block, 0, st, a);
+  else if (p->K == 128 && p->V == 64) launch(zoo_prologue_linear_kernel<T, 128, 64>, grid, block, 0, st, a);
+  else if (p->K == 128 && p->V == 128) launch(zoo_prologue_linear_kernel<T, 128, 128>, grid, block, 0, st, a);
   else return fail(LQ_ERR_UNSUPPORTED, "prologue: K and V must be 64 or 128 (got K=%d V=%d)", p->K, p->V);
   return check_launch("zoo_prologue_linear_kernel");
 }

@@ -57,6 +57,7 @@ __device__ __forceinline__ void mma_had(float (&c)[4], uint32_t a0, uint32_t a1,
 
 template <typename T, int K, int V, bool Q127>
 __global__ void __launch_bounds__(256, 2) zoo_prologue_linear_mma_kernel(PrologueArgs a, int n_tiles) {
+  pdl_enter();
   constexpr int C = kChunk;
   constexpr int KS = K / 16;
   constexpr int RAW_Q = C * K * 2, RAW_V = C * V * 2;
@@ -346,11 +347,11 @@ static int launch_mma(const lq_zoo_problem* p, const PrologueArgs& a, cudaStream
   if (p->qmax == 127.f) {
     e = cudaFuncSetAttribute(zoo_prologue_linear_mma_kernel<T, K, V, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(zoo_prologue_linear_mma_kernel<T, K, V, true>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    if (e == cudaSuccess) zoo_prologue_linear_mma_kernel<T, K, V, true><<<grid, block, smem, st>>>(a, tiles);
+    if (e == cudaSuccess) launch(zoo_prologue_linear_mma_kernel<T, K, V, true>, grid, block, smem, st, a, tiles);
   } else {
     e = cudaFuncSetAttribute(zoo_prologue_linear_mma_kernel<T, K, V, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(zoo_prologue_linear_mma_kernel<T, K, V, false>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    if (e == cudaSuccess) zoo_prologue_linear_mma_kernel<T, K, V, false><<<grid, block, smem, st>>>(a, tiles);
+    if (e == cudaSuccess) launch(zoo_prologue_linear_mma_kernel<T, K, V, false>, grid, block, smem, st, a, tiles);
   }
   if (e != cudaSuccess) return fail(LQ_ERR_LAUNCH, "prologue: cannot opt in to %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
   return check_launch("zoo_prologue_linear_mma_kernel");

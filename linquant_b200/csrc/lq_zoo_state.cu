@@ -27,6 +27,7 @@ struct StateArgs {
 
 template <int K, int V, bool DIAG>
 __global__ void __launch_bounds__(128) zoo_state_linear_kernel(StateArgs a) {
+  pdl_enter();
   constexpr int C = 64;
   constexpr int TK = K / 64;
   const int vt = blockIdx.x / TK, kt = blockIdx.x % TK;
@@ -157,8 +158,8 @@ int run_state_linear(const lq_zoo_problem* p, const lq_zoo_workspace* ws, cudaSt
   const bool diag = p->decay == LQ_DECAY_DIAGONAL;
   dim3 grid((p->V / 32) * (p->K / 64), p->B * p->H), block(128);
 #define LQ_LAUNCH_STATE(KK_, VV_)                                                          \
-  if (diag) zoo_state_linear_kernel<KK_, VV_, true><<<grid, block, 0, st>>>(a);            \
-  else zoo_state_linear_kernel<KK_, VV_, false><<<grid, block, 0, st>>>(a)
+  if (diag) launch(zoo_state_linear_kernel<KK_, VV_, true>, grid, block, 0, st, a);            \
+  else launch(zoo_state_linear_kernel<KK_, VV_, false>, grid, block, 0, st, a)
   if (p->K == 64 && p->V == 64) { LQ_LAUNCH_STATE(64, 64); }
   else if (p->K == 64 && p->V == 128) { LQ_LAUNCH_STATE(64, 128); }
   else if (p->K == 128 && p->V == 64) { LQ_LAUNCH_STATE(128, 64); }

@@ -24,6 +24,7 @@ struct StateUnrotArgs {
 
 template <int K, int V, bool DIAG>
 __global__ void __launch_bounds__(128) zoo_state_linear_unrot_kernel(StateUnrotArgs a) {
+  pdl_enter();
   constexpr int C = 64, KB = 16, LDR = V + 8;
   constexpr int MTW = V / 64;   // 16-row value tiles of the write product per warp
   constexpr int NTW = V / 32;   // 8-column canonical value tiles of the carry per warp
@@ -169,10 +170,10 @@ static int launch_state_unrot(const lq_zoo_problem* p, const StateUnrotArgs& a, 
   cudaError_t e;
   if (p->decay == LQ_DECAY_DIAGONAL) {
     e = cudaFuncSetAttribute(zoo_state_linear_unrot_kernel<K, V, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) zoo_state_linear_unrot_kernel<K, V, true><<<grid, 128, smem, st>>>(a);
+    if (e == cudaSuccess) launch(zoo_state_linear_unrot_kernel<K, V, true>, grid, 128, smem, st, a);
   } else {
     e = cudaFuncSetAttribute(zoo_state_linear_unrot_kernel<K, V, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) zoo_state_linear_unrot_kernel<K, V, false><<<grid, 128, smem, st>>>(a);
+    if (e == cudaSuccess) launch(zoo_state_linear_unrot_kernel<K, V, false>, grid, 128, smem, st, a);
   }
   if (e != cudaSuccess) return fail(LQ_ERR_LAUNCH, "state (canonical storage): shared memory opt-in failed: %s", cudaGetErrorString(e));
   return check_launch("zoo_state_linear_unrot_kernel");
