@@ -103,8 +103,8 @@ size_t lq_zoo_workspace_bytes(const lq_zoo_problem* p, int delta_family);
  *   qq  [BH,NT,C,K]  q codes (read == local, invariances.py:54)      kl  [BH,NT,C,K]  k_local codes
  *   kwT [BH,NT,K,C]  k_write codes, token index contiguous            vlT [BH,NT,V,C]  v_local / e_local codes
  *   vwT [BH,NT,V,C]  v_write codes                                     hT  [BH,NT,V,K]  stored state entering the chunk
- *   gc  [BH,NT,C]    chunk-local cumulative log-decay (fp32)           wq  [BH,NT,C,K]  w_read codes (delta)
- *   u   [BH,NT,C,V]  WY right-hand side U in the activation dtype (delta)
+ *   gc  [BH,NT,C]    chunk-local cumulative log-decay (fp32)           wq  [BH,NT,C*K]  w_read codes (delta; MMA order)
+ *   u   [BH,NT,V,C]  WY right-hand side U in the activation dtype, token index contiguous (delta)
  *   fw  [BH,NT,C]    value-side share of the outer beta factor (delta)
  * Diagonal decay adds gc [BH,NT,C,K], amat, genv, gcl (see the fields below).
  */
@@ -114,8 +114,9 @@ typedef struct {
   void* u;
   float* fw;
   void* amat;  /* [BH,NT,C,C] fp16 intra-chunk matrix (diagonal decay) */
-  float* genv; /* [BH,NT,C]   log of the scalar write envelope (diagonal decay) */
-  float* gcl;  /* [BH,NT,K]   cumulative log-decay at the chunk end (diagonal decay) */
+  float* genv; /* [BH,NT,C]   value-side write gate: the write decay (its envelope, diagonal decay) to the power eta (delta
+                  family, diagonal decay) */
+  float* gcl;  /* [BH,NT,K]   decay factor of the chunk, exp of its cumulative log-decay (diagonal decay) */
   int* status; /* one word, zeroed by the whole-call entries; a kernel whose bounded device-side wait expired sets it */
 } lq_zoo_workspace;
 int lq_zoo_carve_workspace(const lq_zoo_problem* p, int delta_family, void* workspace, size_t workspace_bytes,

@@ -144,7 +144,7 @@ _WS_LAYOUT = {  # name -> (torch dtype, lambda(BH,NT,C,K,V) -> shape)
     "hT": (torch.int8, lambda BH, NT, Cc, K, V: (BH, NT, V, K)),
     "wq": (torch.int8, lambda BH, NT, Cc, K, V: (BH, NT, Cc, K)),
     "gc": (torch.float32, lambda BH, NT, Cc, K, V: (BH, NT, Cc)),
-    "u": (None, lambda BH, NT, Cc, K, V: (BH, NT, Cc, V)),  # activation dtype
+    "u": (None, lambda BH, NT, Cc, K, V: (BH, NT, V, Cc)),  # activation dtype
     "fw": (torch.float32, lambda BH, NT, Cc, K, V: (BH, NT, Cc)),
     "amat": (torch.float16, lambda BH, NT, Cc, K, V: (BH, NT, Cc, Cc)),
     "gcl": (torch.float32, lambda BH, NT, Cc, K, V: (BH, NT, K)),
@@ -197,6 +197,10 @@ class Workspace:
             tok = torch.arange(shape[2], device=t.device)
             pos = (tok & ~15) | (((tok >> 1) & 1) << 3) | (((tok >> 2) & 3) << 1) | (tok & 1)
             t = t[:, :, pos]
+        elif name == "wq":  # MMA-column order (wq_offset in csrc/lq_common.cuh)
+            tok, k = torch.arange(shape[2], device=t.device)[:, None], torch.arange(shape[3], device=t.device)
+            pos = (((tok >> 1) & 7) << 3) | ((tok >> 4) << 1) | (tok & 1)
+            t = t.flatten(2)[:, :, (k >> 5) * 2048 + pos * 32 + (k & 31)]
         elif name == "hT":
             v = torch.arange(shape[2], device=t.device)
             pos = (v & ~31) | (((v >> 1) & 3) << 3) | (((v >> 3) & 3) << 1) | (v & 1)

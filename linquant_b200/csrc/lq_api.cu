@@ -74,7 +74,7 @@ static size_t carve(const lq_zoo_problem* p, int delta, void* ws, lq_zoo_workspa
   w.u = delta ? cv.take<uint16_t>(BH * NT * C * V) : nullptr;
   w.fw = delta ? cv.take<float>(BH * NT * C) : nullptr;
   w.amat = p->decay == LQ_DECAY_DIAGONAL ? cv.take<uint16_t>(BH * NT * C * C) : nullptr;
-  w.genv = p->decay == LQ_DECAY_DIAGONAL ? cv.take<float>(BH * NT * C) : nullptr;
+  w.genv = delta || p->decay == LQ_DECAY_DIAGONAL ? cv.take<float>(BH * NT * C) : nullptr;
   w.gcl = p->decay == LQ_DECAY_DIAGONAL ? cv.take<float>(BH * NT * K) : nullptr;
   w.status = cv.take<int>(64);
   if (out) *out = w;

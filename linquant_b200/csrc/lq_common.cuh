@@ -38,7 +38,14 @@ static inline cudaError_t launch(void (*kern)(KArgs...), dim3 grid, dim3 block, 
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
+}// More than 48 KB of dynamic shared memory: the opt-in is set on every launch (it is per kernel and device and costs a
+// fraction of a microsecond).
+template <typename... KArgs, typename... Args>
+static inline cudaError_t launch_opt_in(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  return e != cudaSuccess ? e : launch(kern, grid, block, smem, st, args...);
 }
+
 // ---- the code rule (zoo/simple_gla.py:16-20; invariances.py:91-100)
 // y = x * inv (fp32, its own rounding), half away from zero, clamp to +-qmax. Clamping first and truncating
 // y + copysign(0.5, y) afterwards gives the same integer for every finite y.
@@ -90,6 +97,12 @@ __device__ __host__ __forceinline__ int kl_row_of_token(int t) {  // low 4 bits 
 __device__ __host__ __forceinline__ int state_row_of_channel(int v) {  // low 5 bits [j1 j0 n1 n0 e] -> [n1 n0 j1 j0 e]
   return (v & ~31) | (((v >> 1) & 3) << 3) | (((v >> 3) & 3) << 1) | (v & 1);
 }
+// The w_read tile [C,K] is the B operand of the delta state pass: per 32-channel block, the 32-byte rows of the 64 tokens in
+// MMA-column order (n-tile (t >> 1) & 7, column 2 (t >> 4) + (t & 1): a lane's accumulators are then sixteen consecutive
+// tokens), so that a fragment load is 256 contiguous bytes.
+__device__ __host__ __forceinline__ int wq_offset(int t, int k) {
+  return (k >> 5) * 2048 + ((((t >> 1) & 7) << 3) | ((t >> 4) << 1) | (t & 1)) * 32 + (k & 31);
+}
 
 // ---- activation dtype traits
 template <typename T>
@@ -106,6 +119,11 @@ struct Act<__half> {
     }
   }
   static __device__ __forceinline__ float round(float x) { return __half2float(__float2half_rn(x)); }
+  static __device__ __forceinline__ __half from(float x) { return __float2half_rn(x); }
+  static __device__ __forceinline__ float to(__half x) { return __half2float(x); }
+  static __device__ __forceinline__ float get(uint32_t w, int hi) {  // one of the two values of a packed word
+    return __half2float(__ushort_as_half((unsigned short)(hi ? w >> 16 : w & 0xffffu)));
+  }
   static __device__ __forceinline__ uint32_t pack2(float a, float b) {
     __half2 h = __floats2half2_rn(a, b);
     return *reinterpret_cast<uint32_t*>(&h);
@@ -122,6 +140,9 @@ struct Act<__nv_bfloat16> {
     }
   }
   static __device__ __forceinline__ float round(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
+  static __device__ __forceinline__ __nv_bfloat16 from(float x) { return __float2bfloat16_rn(x); }
+  static __device__ __forceinline__ float to(__nv_bfloat16 x) { return __bfloat162float(x); }
+  static __device__ __forceinline__ float get(uint32_t w, int hi) { return __uint_as_float(hi ? w & 0xffff0000u : w << 16); }
   static __device__ __forceinline__ uint32_t pack2(float a, float b) {
     __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
     return *reinterpret_cast<uint32_t*>(&h);

@@ -10,14 +10,15 @@
 //   Operands k, v are fp16/bf16 values, exactly representable in TF32, and the fp32 left factor is split into three
 //   TF32 pieces, so every product is exact and only the fp32 accumulation rounds.
 //
-// State pass (one CTA per (batch*head, 32 value channels), serial over chunks, fp32 carry [v,k] in registers):
-//   hq = q8(carry)  -> stored state (global + shared);  ws = wq . hq (INT8 MMA);  E = (U - deq(ws)) * fw
+// State pass (groups of warps own 16 value channels of a (batch, head), serial over chunks, fp32 carry [v,k] in registers):
+//   hq = q8(carry)  -> stored state and MMA operand;  ws = wq . hq (INT8 MMA);  E = (U - deq(ws)) * fw
 //   e_local codes from the activation-rounded E, e_write codes from E * Omega^eta;  carry <- gamma carry + deq(ew^T kw)
 //
 // Reference arithmetic: zoo/gated_delta_rule.py:20-47 (_prep), :51-115 (_delta_state_body);
 // reference.py:202-229 (_chunk_delta).
 #include <type_traits>
 
+#include "lq_tc.cuh"
 #include "lq_wy.cuh"
 #include "lq_zoo_rows.cuh"
 
@@ -28,7 +29,7 @@ struct DeltaPrepArgs {
   const float *beta, *sw;
   int8_t* wq;
   void* u;
-  float* fw;
+  float *fw, *genv;
   float sigma, tau;
 };
 
@@ -70,6 +71,7 @@ __global__ void __launch_bounds__(256) zoo_prologue_delta_kernel(DeltaPrepArgs d
     const float dd = s_gc[C - 1] - s_gc[tid];
     s_fk[tid] = a.g ? expf((1.0f - a.eta) * dd) : 1.0f;
     a.gc[tile * C + tid] = s_gc[tid];
+    d.genv[tile * C + tid] = a.g ? expf(a.eta * dd) : 1.0f;
     const float bt = d.beta[((size_t)b * a.T + (size_t)c * C + tid) * a.H + h];
     const float bs = pow_exact01(bt, d.sigma);
     s_bs[tid] = bs;
@@ -146,8 +148,8 @@ __global__ void __launch_bounds__(256) zoo_prologue_delta_kernel(DeltaPrepArgs d
         const int col = n0 + 8 * nt + 2 * j;
         const int a0 = q8(Act<T>::round(acc[nt][0]), inv_sw, a.qmax), a1 = q8(Act<T>::round(acc[nt][1]), inv_sw, a.qmax);
         const int b0 = q8(Act<T>::round(acc[nt][2]), inv_sw, a.qmax), b1 = q8(Act<T>::round(acc[nt][3]), inv_sw, a.qmax);
-        *reinterpret_cast<uint16_t*>(d.wq + (tile * C + ia) * K + col) = (uint16_t)((a0 & 0xff) | ((a1 & 0xff) << 8));
-        *reinterpret_cast<uint16_t*>(d.wq + (tile * C + ib) * K + col) = (uint16_t)((b0 & 0xff) | ((b1 & 0xff) << 8));
+        *reinterpret_cast<uint16_t*>(d.wq + tile * (C * K) + wq_offset(ia, col)) = (uint16_t)((a0 & 0xff) | ((a1 & 0xff) << 8));
+        *reinterpret_cast<uint16_t*>(d.wq + tile * (C * K) + wq_offset(ib, col)) = (uint16_t)((b0 & 0xff) | ((b1 & 0xff) << 8));
       }
     }
     // ---- U = T diag(beta^sigma) v  -> activation dtype
@@ -161,8 +163,11 @@ __global__ void __launch_bounds__(256) zoo_prologue_delta_kernel(DeltaPrepArgs d
 #pragma unroll
       for (int nt = 0; nt < NTU; ++nt) {
         const int col = n0 + 8 * nt + 2 * j;
-        *reinterpret_cast<uint32_t*>(up + (tile * C + ia) * V + col) = Act<T>::pack2(acc[nt][0], acc[nt][1]);
-        *reinterpret_cast<uint32_t*>(up + (tile * C + ib) * V + col) = Act<T>::pack2(acc[nt][2], acc[nt][3]);
+        T* uc = up + (tile * V + col) * C;  // [V][C]: the token index contiguous
+        uc[ia] = Act<T>::from(acc[nt][0]);
+        uc[C + ia] = Act<T>::from(acc[nt][1]);
+        uc[ib] = Act<T>::from(acc[nt][2]);
+        uc[C + ib] = Act<T>::from(acc[nt][3]);
       }
     }
   }
@@ -172,244 +177,343 @@ __global__ void __launch_bounds__(256) zoo_prologue_delta_kernel(DeltaPrepArgs d
 
 // ------------------------------------------------------------------------------------------------ state pass
 struct DeltaStateArgs {
-  const int8_t *wq, *kwT;
-  const void* u;
+  const int8_t *wq, *kwT;  // wq tile in MMA order: wq_offset()
+  const void* u;           // [BH,NT,V,C]
   const float *fw, *gc, *skw, *sw, *sel, *sew, *ss;
-  const float *gcl, *genv;  // diagonal decay: [BH,NT,K] end-of-chunk log-decay, [BH,NT,C] log envelope
+  const float *gcl, *genv;  // [BH,NT,K] decay factor of the chunk (diagonal decay), [BH,NT,C] value-side write gate
   int8_t *hT, *elT;
   float* final_state;
   const float* initial_state;  // [B,H,K,V] fp32 carry entering the first chunk, or null
-  int H, NT, use_g;
+  int* status;
+  int H, NT, V, use_g;
   float eta, qmax;
 };
 
+// two fp32 values in one register pair: one instruction for both (each rounded on its own, as the scalar forms)
+struct F2 {
+  unsigned long long v;
+  __device__ __forceinline__ F2() {}
+  __device__ __forceinline__ F2(float x, float y) { asm("mov.b64 %0, {%1, %2};\n" : "=l"(v) : "f"(x), "f"(y)); }
+  __device__ __forceinline__ void get(float& x, float& y) const { asm("mov.b64 {%0, %1}, %2;\n" : "=f"(x), "=f"(y) : "l"(v)); }
+};
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) { F2 r; asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+__device__ __forceinline__ F2 add2(F2 a, F2 b) { F2 r; asm("add.rn.f32x2 %0, %1, %2;\n" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) { F2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v)); return r; }
+
+// four codes of two pairs, packed: the rule of q8 (fp32 product, clamp, half away from zero)
+template <bool Q127>
+__device__ __forceinline__ uint32_t codes4(F2 x01, F2 x23, F2 inv, float qmax) {
+  float y[4], h[4];
+  mul2(x01, inv).get(y[0], y[1]);
+  mul2(x23, inv).get(y[2], y[3]);
+  int c[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    y[i] = fmaxf(y[i], Q127 ? -127.f : -qmax);  // at 127 the upper clamp is the saturating pack
+    if (!Q127) y[i] = fminf(y[i], qmax);
+    h[i] = copysignf(0.5f, y[i]);
+  }
+  add2(F2(y[0], y[1]), F2(h[0], h[1])).get(y[0], y[1]);
+  add2(F2(y[2], y[3]), F2(h[2], h[3])).get(y[2], y[3]);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) c[i] = __float2int_rz(y[i]);
+  return pack_sat_s8x2(c[1], c[0], pack_sat_s8x2(c[3], c[2], 0u));
+}
+// INT8 products accumulate on top of the bit pattern of 1.5 * 2^23 (|sum| <= 128 * 127 * 127 < 2^22): the accumulator read as
+// a float is 1.5 * 2^23 + sum, and one subtraction gives the sum exactly, two at a time
+__device__ __forceinline__ void mma_s8_biased(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
+               : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0x4B400000));
+}
+__device__ __forceinline__ F2 unbias2(int a, int b) { return add2(F2(__int_as_float(a), __int_as_float(b)), F2(-12582912.f, -12582912.f)); }
+
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst), "l"(src), "r"(bytes),
+               "r"(bar)
+               : "memory");
+}
+
+// One stage of the operand ring: W tile, kwT tile, the CTA's rows of U, the per-token factors, the decay of the chunk.
+template <int K, int GV>
+struct DeltaStage {
+  static constexpr int kW = 0, kK = 64 * K, kU = 2 * 64 * K, kF = kU + GV * 16 * 128, kG = kF + 256, kD = kG + 256, kBytes = kD + 4 * K;
+};
+template <int K, int KS, int GV, int NS>
+constexpr size_t delta_state_smem() {
+  return (size_t)NS * DeltaStage<K, GV>::kBytes + GV * 2048 + (KS > 1 ? GV * KS * 8 * 512 : 0) + 16 * NS + 4 * K;
+}
+
+// A group of KS warps owns 16 value rows of the state; a warp keeps K / KS key channels of the fp32 carry in registers (rows
+// g, g + 8; eight channels 32 b + 8j .. per lane and 32-channel block b). Everything is laid out so that the codes a lane
+// makes are the MMA fragment it needs next:
+//   * the read is computed transposed, ws^T = hq . W^T: A = the lane's own codes of the carry, B = rows of the W tile, whose
+//     tokens are dealt to the MMA columns so that a lane ends up with consecutive tokens of its two value rows;
+//   * a warp contracts its own channels; the KS partial sums cross through shared memory, each warp finishing the E codes of
+//     TE = 16 / KS tokens per (row, lane), and the e_write codes cross back the same way: two barriers of KS warps a step;
+//   * the write product's A operand is one 16-byte read of those codes per row, its B operand rows of the kwT tile, whose
+//     channels are dealt to the columns so that the lane gets its own carry channels back.
+// One more warp brings the tiles by bulk copies in a ring of NS stages (every tile is contiguous in the workspace), shared by
+// the GV groups of the CTA. The step is serial over the chunks: bound by its latency with few (b, h), by instruction issue
+// with many (about 400 instructions per warp and step; shared memory 40 %, ALU pipe 26 % busy). Measured at K = V = 128
+// against one CTA per 32 value rows with E codes stored bytewise and two block barriers per step: 25.6 -> 15.5 us at 16
+// (b, h) x 16 chunks, 280 -> 237 us at 64 x 128; diagonal decay 54 -> 38 us at 32 x 31, 994 -> 720 us at 256 x 128.
+// Every wait is bounded; on expiry the CTA raises the status word, stores nothing more and waits no more.
+template <typename T, int K, int KS, int GV, int NS, int MINB, bool DIAG, bool Q127>
+__global__ void __launch_bounds__(32 * (KS * GV + 1), MINB) zoo_state_delta_kernel(DeltaStateArgs a) {
+  pdl_enter();
+  constexpr int C = 64, NB = K / 32 / KS, NTE = 8 / KS, TE = 2 * NTE;
+  typedef DeltaStage<K, GV> S;
+  extern __shared__ __align__(128) uint8_t smem_raw[];
+  uint8_t* s_stage = smem_raw;                                  // [NS][S::kBytes]
+  uint8_t* s_codes = s_stage + NS * S::kBytes;                  // [GV][e_write | e_local][16][C]
+  int4* s_part = reinterpret_cast<int4*>(s_codes + GV * 2048);  // [GV][from][n-tile][lane]
+  const uint32_t bars = smem_u32(s_codes + GV * 2048 + (KS > 1 ? GV * KS * 8 * 512 : 0));  // full[NS], empty[NS]
+  float* s_skw = reinterpret_cast<float*>(s_codes + GV * 2048 + (KS > 1 ? GV * KS * 8 * 512 : 0) + 16 * NS);  // [K]
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int bh = blockIdx.y, h = bh % a.H;
+  const int V = a.V, v0 = 16 * GV * blockIdx.x;
+  const size_t tile0 = (size_t)bh * a.NT;
+  const bool gate = a.eta != 0.f && (DIAG || a.use_g);  // genv holds a factor other than 1
+  for (int i = threadIdx.x; i < K; i += 32 * (KS * GV + 1)) s_skw[i] = a.skw[h * K + i];
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < NS; ++i) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(bars + 8 * i));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bars + 8 * (NS + i)), "r"(KS * GV));
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  __syncthreads();
+
+  if (warp == KS * GV) {
+    if (lane == 0) {
+      bool ok = true;
+      int issued = 0;
+      for (int c = 0; c < a.NT && ok; ++c) {
+        const int slot = c % NS;
+        if (c >= NS) ok = mbar_wait_bounded(bars + 8 * (NS + slot), (c / NS - 1) & 1);
+        if (!ok) break;
+        const uint32_t st = smem_u32(s_stage) + slot * S::kBytes, bar = bars + 8 * slot;
+        const size_t tile = tile0 + c;
+        const uint32_t bytes = 2 * C * K + GV * 16 * 128 + 256 + (gate ? 256 : 0) + (DIAG ? 4 * K : (a.use_g ? 16 : 0));
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
+        bulk_load(st + S::kW, a.wq + tile * (C * K), C * K, bar);
+        bulk_load(st + S::kU, reinterpret_cast<const T*>(a.u) + (tile * V + v0) * C, GV * 16 * 128, bar);
+        bulk_load(st + S::kF, a.fw + tile * C, 256, bar);
+        if (gate) bulk_load(st + S::kG, a.genv + tile * C, 256, bar);
+        bulk_load(st + S::kK, a.kwT + tile * (K * C), K * C, bar);
+        if (DIAG) bulk_load(st + S::kD, a.gcl + tile * K, 4 * K, bar);
+        else if (a.use_g) bulk_load(st + S::kD, a.gc + tile * C + C - 4, 16, bar);
+        ++issued;
+      }
+      // copies still in flight must land before the CTA may exit
+      for (int c = max(0, issued - NS); c < issued; ++c) ok = mbar_wait_bounded(bars + 8 * (c % NS), (c / NS) & 1) && ok;
+      if (!ok) atomicExch(a.status, 1);
+    }
+    return;
+  }
+
+  const int ks = warp % KS, gv = warp / KS;
+  const int g = lane >> 2, j = lane & 3;
+  const int va = v0 + 16 * gv + g, vb = va + 8;
+  const int kc0 = 32 * NB * ks + 8 * j;  // first of the lane's eight key channels in its first block
+  const int t0 = 16 * j + TE * ks;       // first of the lane's TE tokens
+  auto group_sync = [&]() {
+    if (KS == 1) __syncwarp();
+    else asm volatile("bar.sync %0, %1;\n" ::"r"(1 + gv), "n"(32 * KS) : "memory");
+  };
+  F2 nsws[2], ihq[2], isel[2], isew[2], sew[2];  // per value row: -s_w s_state, 1 / s_state, 1 / s_el, 1 / s_ew, s_ew
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const int v = r ? vb : va;
+    const float ss = a.ss[h * V + v], n = -a.sw[h] * ss, iel = 1.0f / a.sel[h * V + v];
+    const float ew = a.sew[h * V + v], iew = 1.0f / ew, ih = 1.0f / ss;
+    sew[r] = F2(ew, ew);
+    nsws[r] = F2(n, n); ihq[r] = F2(ih, ih); isel[r] = F2(iel, iel); isew[r] = F2(iew, iew);
+  }
+  F2 skw[NB == 1 ? 4 : 1], carry[NB][2][4];  // several blocks per warp: the key scales stay in shared memory
+#pragma unroll
+  for (int b = 0; b < NB; ++b) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int k = kc0 + 32 * b + 2 * i;
+      if (NB == 1) skw[NB == 1 ? i : 0] = F2(s_skw[k], s_skw[k + 1]);
+      const size_t r0 = ((size_t)bh * K + k) * V, r1 = r0 + V;
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const int v = r ? vb : va;
+        carry[b][r][i] = a.initial_state ? F2(a.initial_state[r0 + v], a.initial_state[r1 + v]) : F2(0.f, 0.f);
+      }
+    }
+  }
+
+  bool ok = true;
+  int slot = 0;
+  uint32_t phase = 0;
+  for (int c = 0; c < a.NT; ++c) {
+    if (ok) ok = mbar_wait_bounded(bars + 8 * slot, phase);
+    const uint8_t* st = s_stage + slot * S::kBytes;
+    // with one channel block per warp every operand of the step is read up front: no read waits behind a barrier
+    constexpr bool EARLY = NB == 1;
+    const uint8_t* wrow = st + S::kW + ks * NB * 2048 + g * 32 + 8 * j;
+    const uint8_t* krow = st + S::kK + (32 * NB * ks + 8 * (g >> 1) + (g & 1)) * C + 16 * j;
+    uint2 wf[EARLY ? 8 : 1], uf[2][TE / 4];
+    uint4 kf[EARLY ? 4 : 1];
+    float4 ff[TE / 4], gf[TE / 4];
+    if constexpr (EARLY) {
+#pragma unroll
+      for (int nt = 0; nt < 8; ++nt) wf[nt] = *reinterpret_cast<const uint2*>(wrow + nt * 256);
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt) kf[nt] = *reinterpret_cast<const uint4*>(krow + 2 * nt * C);
+    }
+    auto read_factors = [&]() {
+#pragma unroll
+      for (int i4 = 0; i4 < TE / 4; ++i4) {
+        ff[i4] = *reinterpret_cast<const float4*>(st + S::kF + 4 * (t0 + 4 * i4));
+        if (gate) gf[i4] = *reinterpret_cast<const float4*>(st + S::kG + 4 * (t0 + 4 * i4));
+#pragma unroll
+        for (int r = 0; r < 2; ++r) uf[r][i4] = *reinterpret_cast<const uint2*>(st + S::kU + (16 * gv + g + 8 * r) * 128 + 2 * (t0 + 4 * i4));
+      }
+    };
+    if (EARLY) read_factors();
+
+    // ---- 1. INT8 copy of the carry entering the chunk: stored state and A fragments in one
+    uint32_t hq[NB][2][2];
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        hq[b][r][0] = codes4<true>(carry[b][r][0], carry[b][r][1], ihq[r], 127.f);
+        hq[b][r][1] = codes4<true>(carry[b][r][2], carry[b][r][3], ihq[r], 127.f);
+        if (ok)
+          *reinterpret_cast<uint2*>(a.hT + ((tile0 + c) * V + state_row_of_channel(r ? vb : va)) * K + kc0 + 32 * b) =
+              make_uint2(hq[b][r][0], hq[b][r][1]);
+      }
+    }
+
+    // ---- 2. reads over this warp's channels, partial sums exchanged within the group
+    int ws[NTE][4];
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt) {
+      int acc[4];
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
+        const uint2 w = EARLY ? wf[EARLY ? nt : 0] : *reinterpret_cast<const uint2*>(wrow + b * 2048 + nt * 256);
+        if (b == 0 && KS == 1) mma_s8_biased(acc, hq[b][0][0], hq[b][1][0], hq[b][0][1], hq[b][1][1], w.x, w.y);
+        else if (b == 0) mma_s8_first(acc, hq[b][0][0], hq[b][1][0], hq[b][0][1], hq[b][1][1], w.x, w.y);
+        else mma_s8(acc, hq[b][0][0], hq[b][1][0], hq[b][0][1], hq[b][1][1], w.x, w.y);
+      }
+      if (KS > 1) {
+        s_part[((gv * KS + ks) * 8 + nt) * 32 + lane] = make_int4(acc[0], acc[1], acc[2], acc[3]);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) ws[nt % NTE][e] = acc[e];
+      }
+    }
+    if (KS > 1) {
+      group_sync();
+#pragma unroll
+      for (int i = 0; i < NTE; ++i) {
+        const int4* p = s_part + (gv * KS * 8 + NTE * ks + i) * 32 + lane;
+        int4 s = p[0];
+#pragma unroll
+        for (int q = 1; q < KS; ++q) {
+          const int4 x = p[q * 256];
+          s.x += x.x; s.y += x.y; s.z += x.z; s.w += x.w;
+        }
+        ws[i][0] = s.x + 0x4B400000; ws[i][1] = s.y + 0x4B400000; ws[i][2] = s.z + 0x4B400000; ws[i][3] = s.w + 0x4B400000;
+      }
+    }
+
+    // ---- 3. E = (U - ws) fw and its codes for TE tokens of two value rows
+    uint8_t* s_ew = s_codes + gv * 2048;
+    if (!EARLY) read_factors();
+#pragma unroll
+    for (int i4 = 0; i4 < TE / 4; ++i4) {
+      const F2 f01(ff[i4].x, ff[i4].y), f23(ff[i4].z, ff[i4].w);
+      const F2 v01(gf[i4].x, gf[i4].y), v23(gf[i4].z, gf[i4].w);
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const uint2 u = uf[r][i4];
+        F2 E01 = fma2(unbias2(ws[2 * i4][2 * r], ws[2 * i4][2 * r + 1]), nsws[r], F2(Act<T>::get(u.x, 0), Act<T>::get(u.x, 1)));
+        F2 E23 = fma2(unbias2(ws[2 * i4 + 1][2 * r], ws[2 * i4 + 1][2 * r + 1]), nsws[r], F2(Act<T>::get(u.y, 0), Act<T>::get(u.y, 1)));
+        E01 = mul2(E01, f01);
+        E23 = mul2(E23, f23);
+        float e0, e1, e2, e3;
+        E01.get(e0, e1);
+        E23.get(e2, e3);
+        const uint32_t p01 = Act<T>::pack2(e0, e1), p23 = Act<T>::pack2(e2, e3);  // e_local: rounded to the activation type
+        uint8_t* dst = s_ew + (g + 8 * r) * C + t0 + 4 * i4;
+        *reinterpret_cast<uint32_t*>(dst + 1024) = codes4<Q127>(F2(Act<T>::get(p01, 0), Act<T>::get(p01, 1)),
+                                                                F2(Act<T>::get(p23, 0), Act<T>::get(p23, 1)), isel[r], a.qmax);
+        if (gate) {
+          E01 = mul2(E01, v01);
+          E23 = mul2(E23, v23);
+        }
+        *reinterpret_cast<uint32_t*>(dst) = codes4<Q127>(E01, E23, isew[r], a.qmax);
+      }
+    }
+    group_sync();
+
+    // ---- 4. e_local rows out (1 KB per group, contiguous); write product and carry update
+    {
+      uint4* eout = reinterpret_cast<uint4*>(a.elT + ((tile0 + c) * V + v0 + 16 * gv) * C);
+#pragma unroll
+      for (int i = ks * 32 + lane; i < 64; i += 32 * KS)
+        if (ok) eout[i] = *reinterpret_cast<const uint4*>(s_ew + 1024 + 16 * i);
+    }
+    const uint4 ea = *reinterpret_cast<const uint4*>(s_ew + g * C + 16 * j);
+    const uint4 eb = *reinterpret_cast<const uint4*>(s_ew + (g + 8) * C + 16 * j);
+    const float gs = !DIAG && a.use_g ? expf(*reinterpret_cast<const float*>(st + S::kD + 12)) : 1.0f;
+    const F2 gs2(gs, gs);
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt) {
+        const uint4 k4 = EARLY ? kf[EARLY ? nt : 0] : *reinterpret_cast<const uint4*>(krow + (32 * b + 2 * nt) * C);
+        int acc[4];
+        mma_s8_biased(acc, ea.x, eb.x, ea.y, eb.y, k4.x, k4.y);
+        mma_s8(acc, ea.z, eb.z, ea.w, eb.w, k4.z, k4.w);
+        F2 gm = gs2;
+        if (DIAG) gm.v = *reinterpret_cast<const unsigned long long*>(st + S::kD + 4 * (kc0 + 32 * b + 2 * nt));
+        F2 sk = skw[NB == 1 ? nt : 0];
+        if (NB > 1) sk.v = *reinterpret_cast<const unsigned long long*>(s_skw + kc0 + 32 * b + 2 * nt);
+        carry[b][0][nt] = fma2(carry[b][0][nt], gm, mul2(mul2(unbias2(acc[0], acc[1]), sk), sew[0]));
+        carry[b][1][nt] = fma2(carry[b][1][nt], gm, mul2(mul2(unbias2(acc[2], acc[3]), sk), sew[1]));
+      }
+    }
+    __syncwarp();
+    if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bars + 8 * (NS + slot)) : "memory");
+    if (++slot == NS) { slot = 0; phase ^= 1; }
+  }
+  if (!ok) atomicExch(a.status, 1);
+
+  if (a.final_state != nullptr && ok) {
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float* r0 = a.final_state + ((size_t)bh * K + kc0 + 32 * b + 2 * i) * V;
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          float x, y;
+          carry[b][r][i].get(x, y);
+          r0[r ? vb : va] = x;
+          r0[V + (r ? vb : va)] = y;
+        }
+      }
+    }
+  }
+}
+
+// ------------------------------------------------------------------------------------------------ state pass, canonical storage
 template <int ROWB>
 __device__ __forceinline__ int swz_row(int row, int chunk) {
   if (ROWB == 128) return row * 128 + ((chunk ^ ((row & 1) << 2)) << 4);
   return row * 64 + (chunk << 4);
 }
 
-template <typename T, int K, int V, bool DIAG>
-__global__ void __launch_bounds__(128) zoo_state_delta_kernel(DeltaStateArgs a) {
-  pdl_enter();
-  constexpr int C = 64, BV = 32;
-  constexpr int NTK = K / 32;  // key n-tiles per warp in the carry layout
-  constexpr int KK = K / 64;
-  __shared__ __align__(128) uint8_t s_h[BV * K];
-  __shared__ __align__(128) uint8_t s_ew[BV * C];
-  __shared__ __align__(128) uint8_t s_el[BV * C];
-
-  const int v0 = blockIdx.x * BV;
-  const int bh = blockIdx.y, h = bh % a.H;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int g = lane >> 2, j = lane & 3;
-  const int kw0 = warp * (K / 4);
-  const int kown = kw0 + 2 * NTK * j;  // first of the 2*NTK consecutive key channels this thread owns
-
-  // carry rows (value channels, local index) and their scales
-  float sew_r[4], iss_r[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int vl = 16 * (i >> 1) + g + 8 * (i & 1);
-    sew_r[i] = a.sew[h * V + v0 + vl];
-    iss_r[i] = 1.0f / a.ss[h * V + v0 + vl];
-  }
-  float skw[2 * NTK];
-#pragma unroll
-  for (int i = 0; i < 2 * NTK; ++i) skw[i] = a.skw[h * K + kown + i];
-  // E columns: eight consecutive value channels v0 + 8j .. + 7
-  float ss_c[8], isel_c[8], isew_c[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    ss_c[i] = a.ss[h * V + v0 + 8 * j + i];
-    isel_c[i] = 1.0f / a.sel[h * V + v0 + 8 * j + i];
-    isew_c[i] = 1.0f / a.sew[h * V + v0 + 8 * j + i];
-  }
-  const float sw = a.sw[h];
-
-  int krow[NTK];
-#pragma unroll
-  for (int nt = 0; nt < NTK; ++nt) krow[nt] = kw0 + 2 * NTK * (g >> 1) + 2 * nt + (g & 1);
-
-  const size_t base_tile = (size_t)bh * a.NT;
-  const int ta = 16 * warp + g, tb = ta + 8;
-  const T* up = reinterpret_cast<const T*>(a.u);
-
-  float carry[2][NTK][4];
-#pragma unroll
-  for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-    for (int nt = 0; nt < NTK; ++nt) {
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const size_t kk_ = (size_t)bh * K + kown + 2 * nt + e;
-        carry[mt][nt][e] = a.initial_state ? a.initial_state[kk_ * V + v0 + 16 * mt + g] : 0.f;
-        carry[mt][nt][2 + e] = a.initial_state ? a.initial_state[kk_ * V + v0 + 16 * mt + g + 8] : 0.f;
-      }
-    }
-
-  uint4 wa[KK], wb[KK], ua, ub, kb[NTK];
-  float fwa, fwb, gca, gcb, glast;
-  auto fetch = [&](int c, uint4 (&wa_)[KK], uint4 (&wb_)[KK], uint4& ua_, uint4& ub_, uint4 (&kb_)[NTK], float& fwa_,
-                   float& fwb_, float& gca_, float& gcb_, float& gl_) {
-    const size_t tile = base_tile + c;
-    const int8_t* wqc = a.wq + tile * (size_t)(C * K);
-#pragma unroll
-    for (int kk = 0; kk < KK; ++kk) {
-      wa_[kk] = __ldg(reinterpret_cast<const uint4*>(wqc + ta * K + 64 * kk + 16 * j));
-      wb_[kk] = __ldg(reinterpret_cast<const uint4*>(wqc + tb * K + 64 * kk + 16 * j));
-    }
-    ua_ = __ldg(reinterpret_cast<const uint4*>(up + (tile * C + ta) * V + v0 + 8 * j));
-    ub_ = __ldg(reinterpret_cast<const uint4*>(up + (tile * C + tb) * V + v0 + 8 * j));
-    const int8_t* kwc = a.kwT + tile * (size_t)(K * C);
-#pragma unroll
-    for (int nt = 0; nt < NTK; ++nt) kb_[nt] = __ldg(reinterpret_cast<const uint4*>(kwc + krow[nt] * C + 16 * j));
-    fwa_ = __ldg(a.fw + tile * C + ta);
-    fwb_ = __ldg(a.fw + tile * C + tb);
-    if (DIAG) {  // gca/gcb carry the log envelope of the two token rows; the carry decay is per key channel
-      gca_ = __ldg(a.genv + tile * C + ta);
-      gcb_ = __ldg(a.genv + tile * C + tb);
-      gl_ = 0.f;
-    } else {
-      gca_ = a.use_g ? __ldg(a.gc + tile * C + ta) : 0.f;
-      gcb_ = a.use_g ? __ldg(a.gc + tile * C + tb) : 0.f;
-      gl_ = a.use_g ? __ldg(a.gc + tile * C + C - 1) : 0.f;
-    }
-  };
-  fetch(0, wa, wb, ua, ub, kb, fwa, fwb, gca, gcb, glast);
-
-  for (int c = 0; c < a.NT; ++c) {
-    const size_t tile = base_tile + c;
-    uint4 nwa[KK], nwb[KK], nua = ua, nub = ub, nkb[NTK];
-    float nfwa = 0.f, nfwb = 0.f, ngca = 0.f, ngcb = 0.f, ngl = 0.f;
-#pragma unroll
-    for (int kk = 0; kk < KK; ++kk) { nwa[kk] = wa[kk]; nwb[kk] = wb[kk]; }
-#pragma unroll
-    for (int nt = 0; nt < NTK; ++nt) nkb[nt] = kb[nt];
-    if (c + 1 < a.NT) fetch(c + 1, nwa, nwb, nua, nub, nkb, nfwa, nfwb, ngca, ngcb, ngl);
-
-    // ---- 1. INT8 copy of the carry entering the chunk: global stored state + shared B operand
-    {
-      int8_t* hc = a.hT + tile * (size_t)(V * K);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int mt = i >> 1, hi = i & 1;
-        const int vl = 16 * mt + g + 8 * hi;
-        int cd[2 * NTK];
-#pragma unroll
-        for (int nt = 0; nt < NTK; ++nt) {
-          cd[2 * nt] = q8_lower127(carry[mt][nt][2 * hi], iss_r[i]);  // upper clamp: the saturating pack below
-          cd[2 * nt + 1] = q8_lower127(carry[mt][nt][2 * hi + 1], iss_r[i]);
-        }
-        uint8_t* sdst = s_h + swz_row<K>(vl, kown >> 4) + (kown & 15);
-        int8_t* gdst = hc + (size_t)state_row_of_channel(v0 + vl) * K + kown;
-        if (NTK == 4) {
-          const uint2 w = make_uint2(pack_sat_s8x2(cd[1], cd[0], pack_sat_s8x2(cd[3], cd[2], 0u)),
-                                     pack_sat_s8x2(cd[5 % (2 * NTK)], cd[4 % (2 * NTK)],
-                                                   pack_sat_s8x2(cd[7 % (2 * NTK)], cd[6 % (2 * NTK)], 0u)));
-          *reinterpret_cast<uint2*>(sdst) = w;
-          *reinterpret_cast<uint2*>(gdst) = w;
-        } else {
-          const uint32_t w = pack_sat_s8x2(cd[1], cd[0], pack_sat_s8x2(cd[3], cd[2], 0u));
-          *reinterpret_cast<uint32_t*>(sdst) = w;
-          *reinterpret_cast<uint32_t*>(gdst) = w;
-        }
-      }
-    }
-    __syncthreads();
-
-    // ---- 2. ws = wq . hq ; E ; e_local / e_write codes
-    {
-      int acc[4][4];
-#pragma unroll
-      for (int nt = 0; nt < 4; ++nt) {
-        acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0;
-        const int vr = 8 * (g >> 1) + 2 * nt + (g & 1);
-#pragma unroll
-        for (int kk = 0; kk < KK; ++kk) {
-          const uint4 bs = *reinterpret_cast<const uint4*>(s_h + swz_row<K>(vr, 4 * kk + j));
-          mma_s8(acc[nt], wa[kk].x, wb[kk].x, wa[kk].y, wb[kk].y, bs.x, bs.y);
-          mma_s8(acc[nt], wa[kk].z, wb[kk].z, wa[kk].w, wb[kk].w, bs.z, bs.w);
-        }
-      }
-      float Ua[8], Ub[8];
-      Act<T>::unpack8(ua, Ua);
-      Act<T>::unpack8(ub, Ub);
-      const float fva = DIAG ? expf(a.eta * gca) : (a.use_g ? expf(a.eta * (glast - gca)) : 1.f);
-      const float fvb = DIAG ? expf(a.eta * gcb) : (a.use_g ? expf(a.eta * (glast - gcb)) : 1.f);
-#pragma unroll
-      for (int nt = 0; nt < 4; ++nt) {
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int i = 2 * nt + e;
-          const int vl = 8 * j + i;
-          const float wsa = __fmul_rn(__fmul_rn((float)acc[nt][e], sw), ss_c[i]);
-          const float wsb = __fmul_rn(__fmul_rn((float)acc[nt][2 + e], sw), ss_c[i]);
-          const float Ea = __fmul_rn(__fsub_rn(Ua[i], wsa), fwa);
-          const float Eb = __fmul_rn(__fsub_rn(Ub[i], wsb), fwb);
-          s_el[vl * C + ta] = (uint8_t)q8(Act<T>::round(Ea), isel_c[i], a.qmax);
-          s_el[vl * C + tb] = (uint8_t)q8(Act<T>::round(Eb), isel_c[i], a.qmax);
-          s_ew[vl * C + ta] = (uint8_t)q8(__fmul_rn(Ea, fva), isew_c[i], a.qmax);
-          s_ew[vl * C + tb] = (uint8_t)q8(__fmul_rn(Eb, fvb), isew_c[i], a.qmax);
-        }
-      }
-    }
-    __syncthreads();
-
-    // ---- 3. write product and carry update; e_local tile out
-    {
-      reinterpret_cast<uint4*>(a.elT + tile * (size_t)(V * C) + (size_t)v0 * C)[tid] = reinterpret_cast<const uint4*>(s_el)[tid];
-      float gamv[2 * NTK];
-      if (DIAG) {
-#pragma unroll
-        for (int i = 0; i < 2 * NTK; ++i) gamv[i] = expf(__ldg(a.gcl + tile * K + kown + i));
-      } else {
-        const float gs = a.use_g ? expf(glast) : 1.0f;
-#pragma unroll
-        for (int i = 0; i < 2 * NTK; ++i) gamv[i] = gs;
-      }
-#pragma unroll
-      for (int mt = 0; mt < 2; ++mt) {
-        const uint4 ea = *reinterpret_cast<const uint4*>(s_ew + (16 * mt + g) * C + 16 * j);
-        const uint4 eb = *reinterpret_cast<const uint4*>(s_ew + (16 * mt + g + 8) * C + 16 * j);
-#pragma unroll
-        for (int nt = 0; nt < NTK; ++nt) {
-          int acc[4] = {0, 0, 0, 0};
-          mma_s8(acc, ea.x, eb.x, ea.y, eb.y, kb[nt].x, kb[nt].y);
-          mma_s8(acc, ea.z, eb.z, ea.w, eb.w, kb[nt].z, kb[nt].w);
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const float ta_ = __fmul_rn(__fmul_rn((float)acc[e], skw[2 * nt + e]), sew_r[2 * mt]);
-            const float tb_ = __fmul_rn(__fmul_rn((float)acc[2 + e], skw[2 * nt + e]), sew_r[2 * mt + 1]);
-            carry[mt][nt][e] = fmaf(carry[mt][nt][e], gamv[2 * nt + e], ta_);
-            carry[mt][nt][2 + e] = fmaf(carry[mt][nt][2 + e], gamv[2 * nt + e], tb_);
-          }
-        }
-      }
-    }
-#pragma unroll
-    for (int kk = 0; kk < KK; ++kk) { wa[kk] = nwa[kk]; wb[kk] = nwb[kk]; }
-#pragma unroll
-    for (int nt = 0; nt < NTK; ++nt) kb[nt] = nkb[nt];
-    ua = nua; ub = nub; fwa = nfwa; fwb = nfwb; gca = ngca; gcb = ngcb; glast = ngl;
-  }
-
-  if (a.final_state != nullptr) {
-    float* fs = a.final_state + (size_t)bh * K * V;
-#pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-      for (int nt = 0; nt < NTK; ++nt)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int kk_ = kown + 2 * nt + e;
-          fs[(size_t)kk_ * V + v0 + 16 * mt + g] = carry[mt][nt][e];
-          fs[(size_t)kk_ * V + v0 + 16 * mt + g + 8] = carry[mt][nt][2 + e];
-        }
-  }
-}
-
-// ------------------------------------------------------------------------------------------------ state pass, canonical storage
 // Delta-rule state pass when v arrives rotated by R_V and the state is stored canonical (zoo/gated_delta_rule.py,
 // zoo/kda.py with unrot=; reference.py:218-227). Per chunk:
 //   ws   = fp16(dequant(W_q . S_q)) . R_V            the canonical state read, taken into the rotated value basis
@@ -495,8 +599,8 @@ __global__ void __launch_bounds__(256) zoo_state_delta_unrot_kernel(DeltaStateAr
       const int8_t* wqc = a.wq + tile * (size_t)(C * K);
 #pragma unroll
       for (int kk = 0; kk < KK; ++kk) {
-        wa[kk] = __ldg(reinterpret_cast<const uint4*>(wqc + ta * K + 64 * kk + 16 * j));
-        wb[kk] = __ldg(reinterpret_cast<const uint4*>(wqc + tb * K + 64 * kk + 16 * j));
+        wa[kk] = __ldg(reinterpret_cast<const uint4*>(wqc + wq_offset(ta, 64 * kk + 16 * j)));
+        wb[kk] = __ldg(reinterpret_cast<const uint4*>(wqc + wq_offset(tb, 64 * kk + 16 * j)));
       }
     }
     const float fwa = __ldg(a.fw + tile * C + ta), fwb = __ldg(a.fw + tile * C + tb);
@@ -556,8 +660,8 @@ __global__ void __launch_bounds__(256) zoo_state_delta_unrot_kernel(DeltaStateAr
 
     // ---- 3. read rotation, E, codes
     {
-      const float fva = DIAG ? expf(a.eta * gca) : (a.use_g ? expf(a.eta * (glast - gca)) : 1.f);
-      const float fvb = DIAG ? expf(a.eta * gcb) : (a.use_g ? expf(a.eta * (glast - gcb)) : 1.f);
+      const float fva = DIAG ? gca : (a.use_g ? expf(a.eta * (glast - gca)) : 1.f);
+      const float fvb = DIAG ? gcb : (a.use_g ? expf(a.eta * (glast - gcb)) : 1.f);
 #pragma unroll
       for (int n2 = 0; n2 < NT2; ++n2) {
         const int nt = NT2 * vh + n2;
@@ -573,16 +677,8 @@ __global__ void __launch_bounds__(256) zoo_state_delta_unrot_kernel(DeltaStateAr
                   *reinterpret_cast<const uint32_t*>(brow + 16 * kk + 8 + 2 * j));
         }
         const int vc = 8 * nt + 2 * j;
-        const uint32_t ura = __ldg(reinterpret_cast<const uint32_t*>(up + (tile * C + ta) * V + vc));
-        const uint32_t urb = __ldg(reinterpret_cast<const uint32_t*>(up + (tile * C + tb) * V + vc));
-        float Ua[2], Ub[2];
-        if (std::is_same<T, __half>::value) {
-          const float2 fa = __half22float2(*reinterpret_cast<const __half2*>(&ura)), fb = __half22float2(*reinterpret_cast<const __half2*>(&urb));
-          Ua[0] = fa.x; Ua[1] = fa.y; Ub[0] = fb.x; Ub[1] = fb.y;
-        } else {
-          Ua[0] = __uint_as_float(ura << 16); Ua[1] = __uint_as_float(ura & 0xffff0000u);
-          Ub[0] = __uint_as_float(urb << 16); Ub[1] = __uint_as_float(urb & 0xffff0000u);
-        }
+        const T* uc = up + (tile * V + vc) * C;
+        const float Ua[2] = {Act<T>::to(uc[ta]), Act<T>::to(uc[C + ta])}, Ub[2] = {Act<T>::to(uc[tb]), Act<T>::to(uc[C + tb])};
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           const int vl = vc + e;
@@ -630,8 +726,8 @@ __global__ void __launch_bounds__(256) zoo_state_delta_unrot_kernel(DeltaStateAr
     if (owner) {
       float gam[2] = {1.f, 1.f};
       if (DIAG) {
-        gam[0] = expf(__ldg(a.gcl + tile * K + ka));
-        gam[1] = expf(__ldg(a.gcl + tile * K + kb_));
+        gam[0] = __ldg(a.gcl + tile * K + ka);
+        gam[1] = __ldg(a.gcl + tile * K + kb_);
       } else if (a.use_g) {
         gam[0] = gam[1] = expf(glast);
       }
@@ -690,7 +786,7 @@ static int dispatch_delta_prep(const lq_zoo_problem* p, const DeltaPrepArgs& d, 
 int run_prologue_delta(const lq_zoo_problem* p, const lq_zoo_workspace* ws, cudaStream_t st) {
   DeltaPrepArgs d;
   fill_prologue_args(p, ws, d.pro);
-  d.beta = p->beta; d.sw = p->sw; d.wq = ws->wq; d.u = ws->u; d.fw = ws->fw; d.sigma = p->sigma; d.tau = p->tau;
+  d.beta = p->beta; d.sw = p->sw; d.wq = ws->wq; d.u = ws->u; d.fw = ws->fw; d.genv = ws->genv; d.sigma = p->sigma; d.tau = p->tau;
   if (p->act_dtype == LQ_F16) return dispatch_delta_prep<__half>(p, d, st);
   if (p->act_dtype == LQ_BF16) return dispatch_delta_prep<__nv_bfloat16>(p, d, st);
   return fail(LQ_ERR_UNSUPPORTED, "delta prologue: activation dtype must be f16 or bf16");
@@ -713,6 +809,22 @@ static int launch_delta_state_unrot(const lq_zoo_problem* p, const DeltaStateArg
   return check_launch("zoo_state_delta_unrot_kernel");
 }
 
+template <typename T, int K, bool Q127, int KS_, int GV, int NS, int MINB>
+static cudaError_t launch_delta_state_v(const lq_zoo_problem* p, const DeltaStateArgs& a, cudaStream_t st) {
+  constexpr int KS = KS_ < K / 32 ? KS_ : K / 32;
+  const dim3 grid(p->V / 16 / GV, p->B * p->H);
+  constexpr size_t smem = delta_state_smem<K, KS, GV, NS>();
+  if (p->decay == LQ_DECAY_DIAGONAL) return launch_opt_in(zoo_state_delta_kernel<T, K, KS, GV, NS, MINB, true, Q127>, grid, 32 * (KS * GV + 1), smem, st, a);
+  return launch_opt_in(zoo_state_delta_kernel<T, K, KS, GV, NS, MINB, false, Q127>, grid, 32 * (KS * GV + 1), smem, st, a);
+}
+template <typename T, int K, bool Q127>
+static cudaError_t launch_delta_state(const lq_zoo_problem* p, const DeltaStateArgs& a, cudaStream_t st) {
+  // Up to two groups of 16 value rows per SM: one group per CTA, a warp per 32 key channels (the shortest step). More: two
+  // warps per group and two groups per CTA (fewer instructions per group; three CTAs per SM).
+  if ((long long)p->B * p->H * (p->V / 16) <= 296) return launch_delta_state_v<T, K, Q127, 4, 1, 2, 1>(p, a, st);
+  return launch_delta_state_v<T, K, Q127, 2, 2, 2, 3>(p, a, st);
+}
+
 template <typename T>
 static int dispatch_delta_state(const lq_zoo_problem* p, const DeltaStateArgs& a, cudaStream_t st) {
   if (p->unrot_t != nullptr) {  // canonical storage: one CTA per (batch, head) owns the whole state
@@ -722,17 +834,12 @@ static int dispatch_delta_state(const lq_zoo_problem* p, const DeltaStateArgs& a
     if (p->K == 128 && p->V == 128) return launch_delta_state_unrot<T, 128, 128>(p, a, st);
     return fail(LQ_ERR_UNSUPPORTED, "delta state: K and V must be 64 or 128");
   }
-  dim3 grid(p->V / 32, p->B * p->H), block(128);
-  const bool diag = p->decay == LQ_DECAY_DIAGONAL;
-#define LQ_LAUNCH_DSTATE(KK_, VV_)                                                         \
-  if (diag) launch(zoo_state_delta_kernel<T, KK_, VV_, true>, grid, block, 0, st, a);          \
-  else launch(zoo_state_delta_kernel<T, KK_, VV_, false>, grid, block, 0, st, a)
-  if (p->K == 64 && p->V == 64) { LQ_LAUNCH_DSTATE(64, 64); }
-  else if (p->K == 64 && p->V == 128) { LQ_LAUNCH_DSTATE(64, 128); }
-  else if (p->K == 128 && p->V == 64) { LQ_LAUNCH_DSTATE(128, 64); }
-  else if (p->K == 128 && p->V == 128) { LQ_LAUNCH_DSTATE(128, 128); }
+  const bool q127 = p->qmax == 127.f;
+  cudaError_t e;
+  if (p->K == 64) e = q127 ? launch_delta_state<T, 64, true>(p, a, st) : launch_delta_state<T, 64, false>(p, a, st);
+  else if (p->K == 128) e = q127 ? launch_delta_state<T, 128, true>(p, a, st) : launch_delta_state<T, 128, false>(p, a, st);
   else return fail(LQ_ERR_UNSUPPORTED, "delta state: K and V must be 64 or 128");
-#undef LQ_LAUNCH_DSTATE
+  if (e != cudaSuccess) return fail(LQ_ERR_LAUNCH, "zoo_state_delta_kernel: %s", cudaGetErrorString(e));
   return check_launch("zoo_state_delta_kernel");
 }
 
@@ -740,8 +847,9 @@ int run_state_delta(const lq_zoo_problem* p, const lq_zoo_workspace* ws, cudaStr
   DeltaStateArgs a;
   a.wq = ws->wq; a.kwT = ws->kwT; a.u = ws->u; a.fw = ws->fw; a.gc = ws->gc;
   a.skw = p->skw; a.sw = p->sw; a.sel = p->sel; a.sew = p->sew; a.ss = p->sstate;
-  a.hT = ws->hT; a.elT = ws->vlT; a.final_state = p->final_state; a.initial_state = p->initial_state; a.gcl = ws->gcl; a.genv = ws->genv;
-  a.H = p->H; a.NT = p->T / p->chunk; a.use_g = p->g != nullptr; a.eta = p->eta; a.qmax = p->qmax;
+  a.hT = ws->hT; a.elT = ws->vlT; a.status = p->status != nullptr ? p->status : ws->status;
+  a.final_state = p->final_state; a.initial_state = p->initial_state; a.gcl = ws->gcl; a.genv = ws->genv;
+  a.H = p->H; a.NT = p->T / p->chunk; a.V = p->V; a.use_g = p->g != nullptr; a.eta = p->eta; a.qmax = p->qmax;
   if (p->act_dtype == LQ_F16) return dispatch_delta_state<__half>(p, a, st);
   if (p->act_dtype == LQ_BF16) return dispatch_delta_state<__nv_bfloat16>(p, a, st);
   return fail(LQ_ERR_UNSUPPORTED, "delta state: activation dtype must be f16 or bf16");

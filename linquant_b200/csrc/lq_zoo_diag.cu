@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(256) zoo_diag_rows_kernel(DiagArgs a) {
       f = (float)acc;
       s_gc[t * LD + tid] = f;
     }
-    a.gcl[tile * K + tid] = f;
+    a.gcl[tile * K + tid] = expf(f);
   }
   __syncthreads();
   for (int i = tid; i < C * (K / 4); i += 256) {
@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(256) zoo_diag_rows_kernel(DiagArgs a) {
     for (int d = 16; d > 0; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
     if (lane == 0) {
       s_le[t] = m;
-      a.genv[tile * C + t] = m;
+      a.genv[tile * C + t] = expf(a.eta * m);
     }
   }
   __syncthreads();
@@ -775,8 +775,8 @@ __global__ void __launch_bounds__(256) zoo_kda_wy_kernel(DiagArgs a) {
       const int col = n0 + 8 * nt + 2 * j4;
       const int a0 = q8(Act<T>::round(acc[nt][0]), inv_sw, a.qmax), a1 = q8(Act<T>::round(acc[nt][1]), inv_sw, a.qmax);
       const int b0 = q8(Act<T>::round(acc[nt][2]), inv_sw, a.qmax), b1 = q8(Act<T>::round(acc[nt][3]), inv_sw, a.qmax);
-      *reinterpret_cast<uint16_t*>(a.wq + (tile * C + ia) * K + col) = (uint16_t)((a0 & 0xff) | ((a1 & 0xff) << 8));
-      *reinterpret_cast<uint16_t*>(a.wq + (tile * C + ib) * K + col) = (uint16_t)((b0 & 0xff) | ((b1 & 0xff) << 8));
+      *reinterpret_cast<uint16_t*>(a.wq + tile * (C * K) + wq_offset(ia, col)) = (uint16_t)((a0 & 0xff) | ((a1 & 0xff) << 8));
+      *reinterpret_cast<uint16_t*>(a.wq + tile * (C * K) + wq_offset(ib, col)) = (uint16_t)((b0 & 0xff) | ((b1 & 0xff) << 8));
     }
   }
   __syncthreads();  // v staged by all threads
@@ -795,8 +795,11 @@ __global__ void __launch_bounds__(256) zoo_kda_wy_kernel(DiagArgs a) {
 #pragma unroll
     for (int nt = 0; nt < NTU; ++nt) {
       const int col = n0 + 8 * nt + 2 * j4;
-      *reinterpret_cast<uint32_t*>(up + (tile * C + ia) * V + col) = Act<T>::pack2(acc[nt][0], acc[nt][1]);
-      *reinterpret_cast<uint32_t*>(up + (tile * C + ib) * V + col) = Act<T>::pack2(acc[nt][2], acc[nt][3]);
+      T* uc = up + (tile * V + col) * C;  // [V][C]: the token index contiguous
+      uc[ia] = Act<T>::from(acc[nt][0]);
+      uc[C + ia] = Act<T>::from(acc[nt][1]);
+      uc[ib] = Act<T>::from(acc[nt][2]);
+      uc[C + ib] = Act<T>::from(acc[nt][3]);
     }
   }
 }

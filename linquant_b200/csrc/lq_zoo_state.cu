@@ -21,7 +21,7 @@ namespace lq {
 struct StateArgs {
   const int8_t *kwT, *vwT;
   const float *gc, *skw, *svw, *ss;
-  const float* gcl;  // diagonal decay: [BH,NT,K] cumulative log-decay at the chunk end, per key channel
+  const float* gcl;  // diagonal decay: [BH,NT,K] decay factor of the chunk, per key channel
   int8_t* hT;
   float* final_state;  // [B,H,K,V] or null
   const float* initial_state;  // [B,H,K,V] or null
@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(128, DEPTH == 3 ? 2 : 4) zoo_state_linear_kern
     float gamv[NC];
     if constexpr (DIAG) {
 #pragma unroll
-      for (int i = 0; i < NC; ++i) gamv[i] = expf(t.gk[i]);
+      for (int i = 0; i < NC; ++i) gamv[i] = t.gk[i];
     } else {
       const float gs = a.use_g ? expf(t.gl) : 1.0f;
 #pragma unroll

@@ -126,8 +126,8 @@ __global__ void __launch_bounds__(128) zoo_state_linear_unrot_kernel(StateUnrotA
     // un-rotation on the tensor cores, folded into the carry
     float gam[2] = {1.f, 1.f};
     if (DIAG) {
-      gam[0] = expf(a.gcl[((size_t)bh * a.NT + c) * K + k0 + g]);
-      gam[1] = expf(a.gcl[((size_t)bh * a.NT + c) * K + k0 + g + 8]);
+      gam[0] = a.gcl[((size_t)bh * a.NT + c) * K + k0 + g];
+      gam[1] = a.gcl[((size_t)bh * a.NT + c) * K + k0 + g + 8];
     } else if (a.use_g) {
       gam[0] = gam[1] = expf(gc[(size_t)c * C + (C - 1)]);
     }
