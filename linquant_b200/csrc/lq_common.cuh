@@ -220,6 +220,61 @@ __device__ __forceinline__ void s8x4_to_h2x2(uint32_t w, uint32_t& h01, uint32_t
   h23 = *reinterpret_cast<uint32_t*>(&hb);
 }
 
+// two fp32 values in one register pair: one instruction for both (each rounded on its own, as the scalar forms)
+struct F2 {
+  unsigned long long v;
+  __device__ __forceinline__ F2() {}
+  __device__ __forceinline__ F2(float x, float y) { asm("mov.b64 %0, {%1, %2};\n" : "=l"(v) : "f"(x), "f"(y)); }
+  __device__ __forceinline__ void get(float& x, float& y) const { asm("mov.b64 {%0, %1}, %2;\n" : "=f"(x), "=f"(y) : "l"(v)); }
+};
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) { F2 r; asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+__device__ __forceinline__ F2 add2(F2 a, F2 b) { F2 r; asm("add.rn.f32x2 %0, %1, %2;\n" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) { F2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v)); return r; }
+
+__device__ __forceinline__ F2 sub2(F2 a, F2 b) { F2 r; asm("sub.rn.f32x2 %0, %1, %2;\n" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+
+// four codes of two pairs, packed: the rule of q8 (fp32 product, clamp, half away from zero)
+template <bool Q127>
+__device__ __forceinline__ uint32_t codes4(F2 x01, F2 x23, F2 inv, float qmax) {
+  float y[4], h[4];
+  mul2(x01, inv).get(y[0], y[1]);
+  mul2(x23, inv).get(y[2], y[3]);
+  int c[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    y[i] = fmaxf(y[i], Q127 ? -127.f : -qmax);  // at 127 the upper clamp is the saturating pack
+    if (!Q127) y[i] = fminf(y[i], qmax);
+    h[i] = copysignf(0.5f, y[i]);
+  }
+  add2(F2(y[0], y[1]), F2(h[0], h[1])).get(y[0], y[1]);
+  add2(F2(y[2], y[3]), F2(h[2], h[3])).get(y[2], y[3]);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) c[i] = __float2int_rz(y[i]);
+  return pack_sat_s8x2(c[1], c[0], pack_sat_s8x2(c[3], c[2], 0u));
+}
+// INT8 products accumulate on top of the bit pattern of 1.5 * 2^23 (|sum| <= 128 * 127 * 127 < 2^22): the accumulator read as
+// a float is 1.5 * 2^23 + sum, and one subtraction gives the sum exactly, two at a time
+__device__ __forceinline__ void mma_s8_biased(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
+               : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0x4B400000));
+}
+__device__ __forceinline__ F2 unbias2(int a, int b) { return add2(F2(__int_as_float(a), __int_as_float(b)), F2(-12582912.f, -12582912.f)); }
+
+// an fp32 value as three bf16 values, biggest first (8 + 8 + 8 bits: the sum is exact), two to a word; eight values
+__device__ __forceinline__ void split3(const float (&x)[8], uint32_t (&hi)[4], uint32_t (&mid)[4], uint32_t (&lo)[4]) {
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    hi[p] = Act<__nv_bfloat16>::pack2(x[2 * p], x[2 * p + 1]);
+    const F2 r = sub2(F2(x[2 * p], x[2 * p + 1]), F2(__uint_as_float(hi[p] << 16), __uint_as_float(hi[p] & 0xffff0000u)));
+    float a, b;
+    r.get(a, b);
+    mid[p] = Act<__nv_bfloat16>::pack2(a, b);
+    sub2(r, F2(__uint_as_float(mid[p] << 16), __uint_as_float(mid[p] & 0xffff0000u))).get(a, b);
+    lo[p] = Act<__nv_bfloat16>::pack2(a, b);
+  }
+}
+
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
   uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");

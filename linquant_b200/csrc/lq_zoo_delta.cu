@@ -189,45 +189,6 @@ struct DeltaStateArgs {
   float eta, qmax;
 };
 
-// two fp32 values in one register pair: one instruction for both (each rounded on its own, as the scalar forms)
-struct F2 {
-  unsigned long long v;
-  __device__ __forceinline__ F2() {}
-  __device__ __forceinline__ F2(float x, float y) { asm("mov.b64 %0, {%1, %2};\n" : "=l"(v) : "f"(x), "f"(y)); }
-  __device__ __forceinline__ void get(float& x, float& y) const { asm("mov.b64 {%0, %1}, %2;\n" : "=f"(x), "=f"(y) : "l"(v)); }
-};
-__device__ __forceinline__ F2 mul2(F2 a, F2 b) { F2 r; asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
-__device__ __forceinline__ F2 add2(F2 a, F2 b) { F2 r; asm("add.rn.f32x2 %0, %1, %2;\n" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
-__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) { F2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v)); return r; }
-
-// four codes of two pairs, packed: the rule of q8 (fp32 product, clamp, half away from zero)
-template <bool Q127>
-__device__ __forceinline__ uint32_t codes4(F2 x01, F2 x23, F2 inv, float qmax) {
-  float y[4], h[4];
-  mul2(x01, inv).get(y[0], y[1]);
-  mul2(x23, inv).get(y[2], y[3]);
-  int c[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    y[i] = fmaxf(y[i], Q127 ? -127.f : -qmax);  // at 127 the upper clamp is the saturating pack
-    if (!Q127) y[i] = fminf(y[i], qmax);
-    h[i] = copysignf(0.5f, y[i]);
-  }
-  add2(F2(y[0], y[1]), F2(h[0], h[1])).get(y[0], y[1]);
-  add2(F2(y[2], y[3]), F2(h[2], h[3])).get(y[2], y[3]);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) c[i] = __float2int_rz(y[i]);
-  return pack_sat_s8x2(c[1], c[0], pack_sat_s8x2(c[3], c[2], 0u));
-}
-// INT8 products accumulate on top of the bit pattern of 1.5 * 2^23 (|sum| <= 128 * 127 * 127 < 2^22): the accumulator read as
-// a float is 1.5 * 2^23 + sum, and one subtraction gives the sum exactly, two at a time
-__device__ __forceinline__ void mma_s8_biased(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
-               : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
-               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0x4B400000));
-}
-__device__ __forceinline__ F2 unbias2(int a, int b) { return add2(F2(__int_as_float(a), __int_as_float(b)), F2(-12582912.f, -12582912.f)); }
-
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst), "l"(src), "r"(bytes),
                "r"(bar)

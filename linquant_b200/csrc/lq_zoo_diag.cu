@@ -221,262 +221,292 @@ __global__ void __launch_bounds__(256) zoo_diag_rows_kernel(DiagArgs a) {
 }
 
 // ------------------------------------------------------------------------------------------------ A matrix
+// Eight warps, no data shared but the log-decay tile and the codes of the off-diagonal operands; every operand element is
+// made in the register of the MMA fragment that contracts it. In all tiles a lane holds of its two rows (g, g + 8 of 16) the
+// channels 32 m + 8 j .. + 7 (one 16-byte load each): the contraction index may be dealt to the MMA slots in any order as
+// long as both operands agree.
+//   warps 0 - 3   diagonal block I = warp: both operands' codes, times exp(g - a) and exp(a - g) around the block's first row
+//                 a, each split into three bf16 pieces (exact), six products (big to small down to 2^-16) on the tensor cores
+//   warps 4 - 7   the nine re-scaled operand tiles of the off-diagonal block rows: fp16 rounding, Hadamard rotation, codes; then
+//                 (one barrier of these four warps) the six 16 x 16 INT8 products
+// The 2^7 (2^6) Hadamard transform is split over the channel bits: bits 0, 1, 3, 4 are the sixteen slots of an m16n8k16 product
+// with the +-1 matrix (exact operands, fp32 accumulation), the others a butterfly between a lane's own registers.
+// Bound by instruction issue. The kernel before it (operands through shared memory, shuffle butterflies, 3xTF32 with the
+// split in the product loop: 42 k warp instructions and 27 block barriers per chunk) took 2070 us for 256 (b, h) x 128 chunks at K = 128; this one 1637.
 template <typename T, int K>
 __global__ void __launch_bounds__(256) zoo_diag_amat_kernel(DiagArgs a) {
   pdl_enter();
-  constexpr int C = 64, LD = K + 4, SUB = 16;
+  constexpr int C = 64, LD = K + 4, SUB = 16, M = K / 32;
   extern __shared__ __align__(16) uint8_t smem_raw[];
-  float* s_gc = reinterpret_cast<float*>(smem_raw);
-  float* s_A = s_gc + C * LD;
-  float* s_hw = s_A + C * 65;
-  int8_t* s_qc = reinterpret_cast<int8_t*>(s_hw + C);
-  int8_t* s_kc = s_qc + C * K;
-  int8_t* s_qa = s_kc + C * K;
-  int8_t* s_ka = s_qa + SUB * K;
+  float* s_gc = reinterpret_cast<float*>(smem_raw);                          // [C][LD]
+  float* s_sgn = s_gc + C * LD;                                              // [K] rotation signs / sqrt(K) on the fp16 grid
+  float* s_hw = s_sgn + K;                                                   // [C]
+  uint4* s_code = reinterpret_cast<uint4*>(s_hw + C);                        // [9 tiles][M][32 lanes]: row g (eh 0, 1), row g + 8
 
   const int c = blockIdx.x, bh = blockIdx.y;
   const int b = bh / a.H, h = bh % a.H;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int g = lane >> 2, j4 = lane & 3;
+  const int g = lane >> 2, j = lane & 3;
   const size_t tile = (size_t)bh * a.NT + c;
   const float e_hw = (1.f - a.sigma) * a.tau;
   const bool use_hw = a.beta != nullptr && e_hw != 0.f;
   const bool rot = a.signs != nullptr;
-
-  constexpr int LPR = K / 8, G = 32 / LPR;
-  const int r = lane % LPR, grp = lane / LPR;
   const T* qp = reinterpret_cast<const T*>(a.q);
   const T* kp = reinterpret_cast<const T*>(a.k);
-  auto grow = [&](int t) { return (((size_t)b * a.T + (size_t)c * C + t) * a.H + h) * K + 8 * r; };
+  auto grow = [&](int t) { return (((size_t)b * a.T + (size_t)c * C + t) * a.H + h) * K + 8 * j; };
 
-  // The rows of the bare operands (diagonal blocks) are requested first of all, so that their trip to memory runs
-  // beside that of the log-decay tile; every row load of the thread is issued before the first is used.
-  constexpr int NIT = C / (8 * G);
-  uint4 rq0[NIT], rk0[NIT];
-#pragma unroll
-  for (int u = 0; u < NIT; ++u) {
-    const int t = warp * G + grp + 8 * G * u;
-    rq0[u] = __ldg(reinterpret_cast<const uint4*>(qp + grow(t)));
-    rk0[u] = __ldg(reinterpret_cast<const uint4*>(kp + grow(t)));
-  }
   load_gc_tile<K, K / 32>(a.gc + tile * (size_t)(C * K), s_gc);
-  for (int i = tid; i < C * 65; i += 256) s_A[i] = 0.f;
-  if (tid < C) {
-    s_hw[tid] = use_hw ? pow_exact01(a.beta[((size_t)b * a.T + (size_t)c * C + tid) * a.H + h], e_hw) : 1.f;
-  }
-  __syncthreads();
-
-  const float inv_sq = 1.0f / a.sq[h], inv_sk = 1.0f / a.sk[h];
-  const float sqk = __fmul_rn(a.sq[h], a.sk[h]);
-#pragma unroll
-  for (int u = 0; u < NIT; ++u) {
-    const int t = warp * G + grp + 8 * G * u;
-    float x[8];
-    int cd[8];
-    Act<T>::unpack8(rq0[u], x);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) cd[j] = q8(__fmul_rn(x[j], a.scale), inv_sq, a.qmax);
-    *reinterpret_cast<uint2*>(s_qc + t * K + 8 * r) = make_uint2(pack4(cd[0], cd[1], cd[2], cd[3]), pack4(cd[4], cd[5], cd[6], cd[7]));
-    Act<T>::unpack8(rk0[u], x);
-    if (use_hw) {
-      const float hw = s_hw[t];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) x[j] = Act<T>::round(__fmul_rn(x[j], hw));
-    }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) cd[j] = q8(x[j], inv_sk, a.qmax);
-    *reinterpret_cast<uint2*>(s_kc + t * K + 8 * r) = make_uint2(pack4(cd[0], cd[1], cd[2], cd[3]), pack4(cd[4], cd[5], cd[6], cd[7]));
-  }
-
-  // off-diagonal blocks: rows [16I, 16I+16) against columns [0, 16I), operands re-scaled around the anchor row 16I
-  float sgn[8];
-  {
+  if (tid < C) s_hw[tid] = use_hw ? pow_exact01(a.beta[((size_t)b * a.T + (size_t)c * C + tid) * a.H + h], e_hw) : 1.f;
+  if (tid >= 128 && tid < 128 + K) {
     const float n16 = __half2float(__float2half_rn(K == 64 ? 0.125f : 0.08838834764831845f));
-#pragma unroll
-    for (int j = 0; j < 8; ++j) sgn[j] = rot ? a.signs[8 * r + j] * n16 : 1.f;
+    s_sgn[tid - 128] = rot ? a.signs[tid - 128] * n16 : 1.f;
   }
-  for (int I = 1; I < C / SUB; ++I) {
-    float anc[8];
+  __syncthreads();
+
+  const float fq = 1.0f / a.sq[h], fk = 1.0f / a.sk[h];
+  const float sqk = __fmul_rn(a.sq[h], a.sk[h]);
+  __half* A = a.amat + tile * (size_t)(C * C);
+  auto lds8 = [&](const float* p, float (&v)[8]) {
+    *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(p);
+    *reinterpret_cast<float4*>(v + 4) = *reinterpret_cast<const float4*>(p + 4);
+  };
+
+  if (warp < 4) {
+    // ---------------------------------------------------------------------------------- diagonal block
+    const int t0 = SUB * warp;
+    uint4 rq[2][M], rk[2][M];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) anc[j] = s_gc[(SUB * I) * LD + 8 * r + j];
-    const int R = SUB + SUB * I;
-    uint4 rrow[NIT];  // this thread's rows of the block row, requested together
+    for (int r = 0; r < 2; ++r)
 #pragma unroll
-    for (int u = 0; u < NIT; ++u) {
-      const int rr = warp * G + grp + 8 * G * u;
-      if (rr < R) rrow[u] = __ldg(reinterpret_cast<const uint4*>((rr < SUB ? qp : kp) + grow(rr < SUB ? SUB * I + rr : rr - SUB)));
-    }
+      for (int m = 0; m < M; ++m) {
+        rq[r][m] = __ldg(reinterpret_cast<const uint4*>(qp + grow(t0 + g + 8 * r) + 32 * m));
+        rk[r][m] = __ldg(reinterpret_cast<const uint4*>(kp + grow(t0 + g + 8 * r) + 32 * m));
+      }
+    auto key = [&](const uint4& raw, int t, float (&x)[8]) {  // the readout key of one row piece
+      Act<T>::unpack8(raw, x);
+      if (use_hw) {
+        const float hw = s_hw[t];
 #pragma unroll
-    for (int u = 0; u < NIT; ++u) {
-      const int rr = warp * G + grp + 8 * G * u;
-      if (rr >= R) break;
-      const bool isq = rr < SUB;
-      const int t = isq ? SUB * I + rr : rr - SUB;
-      float x[8];
-      int cd[8];
-      Act<T>::unpack8(rrow[u], x);
-      if (isq) {
+        for (int e = 0; e < 8; ++e) x[e] = Act<T>::round(__fmul_rn(x[e], hw));
+      }
+    };
+    // the weight exp(g_i - g_j) factors around the first row unless the decay across the block is so strong (beyond e^60) that
+    // the second factor could leave fp32
+    float spread = 0.f;
+    for (int n = lane; n < K; n += 32) spread = fmaxf(spread, __fsub_rn(s_gc[t0 * LD + n], s_gc[(t0 + SUB - 1) * LD + n]));
+    const bool exact = __any_sync(0xffffffffu, spread > 60.f);
+    float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+    if (!exact) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) x[j] = __fmul_rn(__fmul_rn(x[j], __expf(__fsub_rn(s_gc[t * LD + 8 * r + j], anc[j]))), a.scale);
-      } else {
-        if (use_hw) {
-          const float hw = s_hw[t];
+      for (int m = 0; m < M; ++m) {
+        float an[8];
+        lds8(s_gc + t0 * LD + 32 * m + 8 * j, an);
+        uint32_t qh[2][4], qm[2][4], ql[2][4], kh[2][4], km[2][4], kl[2][4];  // [row half][pair of channels]
 #pragma unroll
-          for (int j = 0; j < 8; ++j) x[j] = Act<T>::round(__fmul_rn(x[j], hw));
+        for (int r = 0; r < 2; ++r) {
+          const int t = t0 + g + 8 * r;
+          float x[8], gv[8], e1[8];
+          lds8(s_gc + t * LD + 32 * m + 8 * j, gv);
+          Act<T>::unpack8(rq[r][m], x);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            e1[e] = __fsub_rn(gv[e], an[e]);
+            x[e] = __fmul_rn((float)q8(__fmul_rn(x[e], a.scale), fq, a.qmax), __expf(e1[e]));
+          }
+          split3(x, qh[r], qm[r], ql[r]);
+          key(rk[r][m], t, x);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) x[e] = __fmul_rn((float)q8(x[e], fk, a.qmax), __expf(-e1[e]));
+          split3(x, kh[r], km[r], kl[r]);
         }
 #pragma unroll
-        for (int j = 0; j < 8; ++j) x[j] = __fmul_rn(x[j], __expf(__fsub_rn(anc[j], s_gc[t * LD + 8 * r + j])));
+        for (int eh = 0; eh < 2; ++eh) {
+          const int p = 2 * eh;
+          auto mma = [&](float (&d)[4], const uint32_t (&qa)[2][4], const uint32_t (&kb)[4]) {
+            mma_bf16(d, qa[0][p], qa[1][p], qa[0][p + 1], qa[1][p + 1], kb[p], kb[p + 1]);
+          };
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt) {
+            mma(acc[nt], ql, kh[nt]);
+            mma(acc[nt], qh, kl[nt]);
+            mma(acc[nt], qm, km[nt]);
+            mma(acc[nt], qm, kh[nt]);
+            mma(acc[nt], qh, km[nt]);
+            mma(acc[nt], qh, kh[nt]);
+          }
+        }
       }
-      if (rot) {
+    } else {
+      // one exp per (i, j, channel), a lane for each of its eight (i, j) of the accumulator layout
+      for (int n = 0; n < K; ++n) {
+        float qc[2], kc[2][2], gi[2], gj[2][2];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) x[j] = __half2float(__float2half_rn(x[j]));
-        fwht8<LPR>(x, r);
+        for (int r = 0; r < 2; ++r) {
+          const int t = t0 + g + 8 * r;
+          gi[r] = s_gc[t * LD + n];
+          qc[r] = (float)q8(__fmul_rn(Act<T>::to(qp[grow(t) - 8 * j + n]), a.scale), fq, a.qmax);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) x[j] = __fmul_rn(x[j], sgn[j]);
+          for (int e = 0; e < 2; ++e) {
+            const int tj = t0 + 8 * r + 2 * j + e;
+            gj[r][e] = s_gc[tj * LD + n];
+            float x = Act<T>::to(kp[grow(tj) - 8 * j + n]);
+            if (use_hw) x = Act<T>::round(__fmul_rn(x, s_hw[tj]));
+            kc[r][e] = (float)q8(x, fk, a.qmax);
+          }
+        }
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            acc[nt][i] = fmaf(__fmul_rn(qc[i >> 1], kc[nt][i & 1]), __expf(gi[i >> 1] - gj[nt][i & 1]), acc[nt][i]);
       }
-      const float inv = isq ? inv_sq : inv_sk;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) cd[j] = q8(x[j], inv, a.qmax);
-      int8_t* dst = isq ? (s_qa + rr * K) : (s_ka + (rr - SUB) * K);
-      *reinterpret_cast<uint2*>(dst + 8 * r) = make_uint2(pack4(cd[0], cd[1], cd[2], cd[3]), pack4(cd[4], cd[5], cd[6], cd[7]));
     }
-    __syncthreads();
-    if (warp < 2 * I) {
-      int acc[4] = {0, 0, 0, 0};
 #pragma unroll
-      for (int kk = 0; kk < K / 64; ++kk) {
-        const uint4 qa = *reinterpret_cast<const uint4*>(s_qa + g * K + 64 * kk + 16 * j4);
-        const uint4 qb = *reinterpret_cast<const uint4*>(s_qa + (g + 8) * K + 64 * kk + 16 * j4);
-        const uint4 kb = *reinterpret_cast<const uint4*>(s_ka + (8 * warp + g) * K + 64 * kk + 16 * j4);
-        mma_s8(acc, qa.x, qb.x, qa.y, qb.y, kb.x, kb.y);
-        mma_s8(acc, qa.z, qb.z, qa.w, qb.w, kb.z, kb.w);
-      }
+    for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        s_A[(SUB * I + g) * 65 + 8 * warp + 2 * j4 + e] = __fmul_rn((float)acc[e], sqk);
-        s_A[(SUB * I + g + 8) * 65 + 8 * warp + 2 * j4 + e] = __fmul_rn((float)acc[2 + e], sqk);
+      for (int r = 0; r < 2; ++r) {
+        const int i = g + 8 * r, jj = 8 * nt + 2 * j;
+        const float x0 = jj <= i ? __fmul_rn(acc[nt][2 * r], sqk) : 0.f, x1 = jj + 1 <= i ? __fmul_rn(acc[nt][2 * r + 1], sqk) : 0.f;
+        *reinterpret_cast<uint32_t*>(A + (t0 + i) * C + t0 + jj) = Act<__half>::pack2(x0, x1);
       }
-    }
-    __syncthreads();
+    return;
   }
 
-  // diagonal blocks: A_ij = s_q s_k sum_n q^_in k^_jn exp(g_in - g_jn), i >= j inside a 16 x 16 block. The weight factors
-  // around the block's first row a: exp(g_in - a_n) exp(a_n - g_jn). The first factor is <= 1; the second is >= 1 and grows
-  // with the decay across at most 15 tokens, so per block the spread max_n (a_n - g_last,n) decides: up to 60 (a factor
-  // below 1.2e26, far inside fp32) the block is two sets of 16 scaled rows (one exp per row element, 16 x fewer) and a
-  // 16 x 16 x K fp32 product; beyond it (decays as strong as the g x 40 cases) the block takes one exp per (i, j, n).
-  float* s_qd = reinterpret_cast<float*>(s_ka + 48 * K);  // [16][LD] q^ exp(g_i - a), then [16][LD] k^ exp(a - g_j)
-  float* s_kd = s_qd + SUB * LD;
-  __shared__ int s_exact[C / SUB];
-  if (tid < C / SUB) s_exact[tid] = 0;
-  __syncthreads();
-  for (int i = tid; i < (C / SUB) * K; i += 256) {
-    const int I = i / K, n = i - I * K;
-    if (__fsub_rn(s_gc[(SUB * I) * LD + n], s_gc[(SUB * I + SUB - 1) * LD + n]) > 60.f) s_exact[I] = 1;
-  }
-  __syncthreads();
-  for (int I = 0; I < C / SUB; ++I) {
-    if (s_exact[I]) {  // 136 (i >= j) pairs, eight lanes per pair, four channels per lane and step (128-bit loads)
-      for (int pass = 0; pass < 5; ++pass) {
-        const int rem_raw = pass * 32 + (tid >> 3);
-        const bool valid = rem_raw < 136;  // the last pass has idle pairs: they compute a clamped pair and store nothing
-        const int rem = valid ? rem_raw : 135;
-        {
-          int i = (int)((sqrtf(8.f * rem + 1.f) - 1.f) * 0.5f);
-          while ((i + 1) * (i + 2) / 2 <= rem) ++i;
-          while (i * (i + 1) / 2 > rem) --i;
-          const int jj = rem - i * (i + 1) / 2;
-          const int ti = SUB * I + i, tj = SUB * I + jj;
-          const int l8 = tid & 7;
-          float sum = 0.f;
+  // ------------------------------------------------------------------------------------ off-diagonal operand tiles
+  // tile I - 1: the sixteen query rows of block row I; tiles 3 + (I - 1) I / 2 + J: key rows of block J, both around row 16 I
+  const int w4 = warp - 4;
+  const uint32_t had = [&]() {  // (-1)^popc(s & n) for slots s = 2j, 2j + 1 and column n = g, as two halves
+    const uint32_t s0 = (__popc((2 * j) & g) & 1) ? 0xBC00u : 0x3C00u, s1 = (__popc((2 * j + 1) & g) & 1) ? 0xBC00u : 0x3C00u;
+    return s0 | (s1 << 16);
+  }();
+  const bool q127 = a.qmax == 127.f;
+  for (int it = w4; it < 9; it += 4) {
+    const bool isq = it < 3;
+    const int u = it - 3;
+    const int I = isq ? it + 1 : (u < 1 ? 1 : u < 3 ? 2 : 3);
+    const int t0 = SUB * (isq ? I : u - (I - 1) * I / 2);
+    const T* src = isq ? qp : kp;
+    uint4 raw[2][M];
 #pragma unroll
-          for (int n4 = 0; n4 < K / 32; ++n4) {
-            const int n = 4 * l8 + 32 * n4;  // the eight lanes of a pair read 128 consecutive bytes of a gc row
-            const float4 gi = *reinterpret_cast<const float4*>(s_gc + ti * LD + n);
-            const float4 gj = *reinterpret_cast<const float4*>(s_gc + tj * LD + n);
-            const uint32_t qw = *reinterpret_cast<const uint32_t*>(s_qc + ti * K + n) ^ 0x80808080u;
-            const uint32_t kw = *reinterpret_cast<const uint32_t*>(s_kc + tj * K + n) ^ 0x80808080u;
-            sum = fmaf(__fmul_rn(s8_to_float<0>(qw), s8_to_float<0>(kw)), __expf(gi.x - gj.x), sum);
-            sum = fmaf(__fmul_rn(s8_to_float<1>(qw), s8_to_float<1>(kw)), __expf(gi.y - gj.y), sum);
-            sum = fmaf(__fmul_rn(s8_to_float<2>(qw), s8_to_float<2>(kw)), __expf(gi.z - gj.z), sum);
-            sum = fmaf(__fmul_rn(s8_to_float<3>(qw), s8_to_float<3>(kw)), __expf(gi.w - gj.w), sum);
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int m = 0; m < M; ++m) raw[r][m] = __ldg(reinterpret_cast<const uint4*>(src + grow(t0 + g + 8 * r) + 32 * m));
+    F2 y[M][2][2][2];  // [m][eh][row half][channel pair]
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+      float an[8], x[2][8];
+      lds8(s_gc + SUB * I * LD + 32 * m + 8 * j, an);
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const int t = t0 + g + 8 * r;
+        float gv[8];
+        lds8(s_gc + t * LD + 32 * m + 8 * j, gv);
+        Act<T>::unpack8(raw[r][m], x[r]);
+        if (isq) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) x[r][e] = __fmul_rn(__fmul_rn(x[r][e], __expf(__fsub_rn(gv[e], an[e]))), a.scale);
+        } else {
+          if (use_hw) {
+            const float hw = s_hw[t];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) x[r][e] = Act<T>::round(__fmul_rn(x[r][e], hw));
           }
-          sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-          sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-          sum += __shfl_xor_sync(0xffffffffu, sum, 4);
-          if (l8 == 0 && valid) s_A[ti * 65 + tj] = __fmul_rn(sum, sqk);
-        }
-      }
-      __syncthreads();
-      continue;
-    }
-    // scaled rows: thread = (row of the block, 4-channel piece); 2 x 16 x K elements over 256 threads
-    for (int i = tid; i < SUB * (K / 4); i += 256) {
-      const int rr = i / (K / 4), n = 4 * (i - rr * (K / 4));
-      const int t = SUB * I + rr;
-      const float4 an = *reinterpret_cast<const float4*>(s_gc + (SUB * I) * LD + n);
-      const float4 gt = *reinterpret_cast<const float4*>(s_gc + t * LD + n);
-      const uint32_t qw = *reinterpret_cast<const uint32_t*>(s_qc + t * K + n) ^ 0x80808080u;
-      const uint32_t kw = *reinterpret_cast<const uint32_t*>(s_kc + t * K + n) ^ 0x80808080u;
-      *reinterpret_cast<float4*>(s_qd + rr * LD + n) =
-          make_float4(__fmul_rn(s8_to_float<0>(qw), __expf(gt.x - an.x)), __fmul_rn(s8_to_float<1>(qw), __expf(gt.y - an.y)),
-                      __fmul_rn(s8_to_float<2>(qw), __expf(gt.z - an.z)), __fmul_rn(s8_to_float<3>(qw), __expf(gt.w - an.w)));
-      *reinterpret_cast<float4*>(s_kd + rr * LD + n) =
-          make_float4(__fmul_rn(s8_to_float<0>(kw), __expf(an.x - gt.x)), __fmul_rn(s8_to_float<1>(kw), __expf(an.y - gt.y)),
-                      __fmul_rn(s8_to_float<2>(kw), __expf(an.z - gt.z)), __fmul_rn(s8_to_float<3>(kw), __expf(an.w - gt.w)));
-    }
-    __syncthreads();
-    {  // 16 x 16 x K product on the tensor cores, 3xTF32 (both factors split into a TF32 part and a TF32 remainder: the
-       // products are good to about 2^-21). Warp w contracts the channels [K/8 w, K/8 (w + 1)); the eight partial blocks
-       // are parked behind the scaled rows and summed in a fixed order.
-      float* s_part = s_kd + SUB * LD;  // [8 warps][16][16]
-      float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
-      for (int kk = 0; kk < K / 64; ++kk) {
-        const int c0 = (K / 8) * warp + 8 * kk + j4, c1 = c0 + 4;
-        const float xa[4] = {s_qd[g * LD + c0], s_qd[(g + 8) * LD + c0], s_qd[g * LD + c1], s_qd[(g + 8) * LD + c1]};
-        uint32_t ab[4], as_[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          ab[e] = tf32_rna(xa[e]);
-          as_[e] = tf32_rna(xa[e] - __uint_as_float(ab[e]));
-        }
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt) {
-          const float y0 = s_kd[(8 * nt + g) * LD + c0], y1 = s_kd[(8 * nt + g) * LD + c1];
-          const uint32_t b0 = tf32_rna(y0), b1 = tf32_rna(y1);
-          const uint32_t s0 = tf32_rna(y0 - __uint_as_float(b0)), s1 = tf32_rna(y1 - __uint_as_float(b1));
-          mma_tf32(acc[nt], as_[0], as_[1], as_[2], as_[3], b0, b1);
-          mma_tf32(acc[nt], ab[0], ab[1], ab[2], ab[3], s0, s1);
-          mma_tf32(acc[nt], ab[0], ab[1], ab[2], ab[3], b0, b1);
+          for (int e = 0; e < 8; ++e) x[r][e] = __fmul_rn(x[r][e], __expf(__fsub_rn(an[e], gv[e])));
         }
       }
 #pragma unroll
-      for (int nt = 0; nt < 2; ++nt) {
-        float* pw = s_part + warp * 256;
-        pw[g * 16 + 8 * nt + 2 * j4] = acc[nt][0];
-        pw[g * 16 + 8 * nt + 2 * j4 + 1] = acc[nt][1];
-        pw[(g + 8) * 16 + 8 * nt + 2 * j4] = acc[nt][2];
-        pw[(g + 8) * 16 + 8 * nt + 2 * j4 + 1] = acc[nt][3];
-      }
-      __syncthreads();
-      {
-        const int i = tid >> 4, jj = tid & 15;
-        if (jj <= i) {
-          float sum = 0.f;
+      for (int eh = 0; eh < 2; ++eh) {
+        if (rot) {
+          uint32_t f[2][2];
 #pragma unroll
-          for (int w = 0; w < 8; ++w) sum += s_part[w * 256 + tid];
-          s_A[(SUB * I + i) * 65 + SUB * I + jj] = __fmul_rn(sum, sqk);
+          for (int r = 0; r < 2; ++r) {
+            f[r][0] = Act<__half>::pack2(x[r][4 * eh], x[r][4 * eh + 1]);
+            f[r][1] = Act<__half>::pack2(x[r][4 * eh + 2], x[r][4 * eh + 3]);
+          }
+          float d0[4] = {0.f, 0.f, 0.f, 0.f}, d1[4] = {0.f, 0.f, 0.f, 0.f};
+          mma_f16(d0, f[0][0], f[1][0], f[0][1], f[1][1], had, had);
+          mma_f16(d1, f[0][0], f[1][0], f[0][1], f[1][1], had, had ^ 0x80008000u);
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            y[m][eh][r][0] = F2(d0[2 * r], d0[2 * r + 1]);
+            y[m][eh][r][1] = F2(d1[2 * r], d1[2 * r + 1]);
+          }
+        } else {
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            y[m][eh][r][0] = F2(x[r][4 * eh], x[r][4 * eh + 1]);
+            y[m][eh][r][1] = F2(x[r][4 * eh + 2], x[r][4 * eh + 3]);
+          }
         }
       }
     }
-    __syncthreads();
+    if (rot) {  // the remaining channel bits: 2 (eh), 5 and 6 (m)
+      const F2 neg(-1.f, -1.f);
+      auto fly = [&](F2& p, F2& q) {
+        const F2 s = add2(p, q);
+        q = fma2(q, neg, p);
+        p = s;
+      };
+#pragma unroll
+      for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+#pragma unroll
+          for (int m = 0; m < M; ++m) fly(y[m][0][r][e], y[m][1][r][e]);
+#pragma unroll
+          for (int eh = 0; eh < 2; ++eh) {
+#pragma unroll
+            for (int m = 0; m < M; m += 2) fly(y[m][eh][r][e], y[m + 1][eh][r][e]);
+            if (M == 4) {
+              fly(y[0][eh][r][e], y[2 % M][eh][r][e]);
+              fly(y[1][eh][r][e], y[3 % M][eh][r][e]);
+            }
+          }
+        }
+    }
+    const float inv1 = isq ? fq : fk;
+    const F2 inv(inv1, inv1);
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+      uint32_t w[2][2];
+#pragma unroll
+      for (int eh = 0; eh < 2; ++eh) {
+        const float4 sg = *reinterpret_cast<const float4*>(s_sgn + 32 * m + 8 * j + 4 * eh);
+        const F2 s0(sg.x, sg.y), s1(sg.z, sg.w);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const F2 y0 = rot ? mul2(y[m][eh][r][0], s0) : y[m][eh][r][0], y1 = rot ? mul2(y[m][eh][r][1], s1) : y[m][eh][r][1];
+          w[r][eh] = q127 ? codes4<true>(y0, y1, inv, 127.f) : codes4<false>(y0, y1, inv, a.qmax);
+        }
+      }
+      s_code[(it * M + m) * 32 + lane] = make_uint4(w[0][0], w[1][0], w[0][1], w[1][1]);
+    }
   }
-  __syncthreads();
-  uint32_t* out = reinterpret_cast<uint32_t*>(a.amat + tile * (size_t)(C * C));
-  for (int i = tid; i < C * 32; i += 256) {
-    const int row = i >> 5, cp = i & 31;
-    out[i] = Act<__half>::pack2(s_A[row * 65 + 2 * cp], s_A[row * 65 + 2 * cp + 1]);
+  asm volatile("bar.sync 1, 128;\n" ::: "memory");
+  for (int u = w4; u < 6; u += 4) {  // block (I, J)
+    const int I = u < 1 ? 1 : u < 3 ? 2 : 3, J = u - (I - 1) * I / 2;
+    int acc[2][4];
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+      const uint4 qa = s_code[((I - 1) * M + m) * 32 + lane], kb = s_code[((3 + u) * M + m) * 32 + lane];
+      if (m == 0) {
+        mma_s8_first(acc[0], qa.x, qa.y, qa.z, qa.w, kb.x, kb.z);
+        mma_s8_first(acc[1], qa.x, qa.y, qa.z, qa.w, kb.y, kb.w);
+      } else {
+        mma_s8(acc[0], qa.x, qa.y, qa.z, qa.w, kb.x, kb.z);
+        mma_s8(acc[1], qa.x, qa.y, qa.z, qa.w, kb.y, kb.w);
+      }
+    }
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const int i = g + 8 * r, jj = 8 * nt + 2 * j;
+        *reinterpret_cast<uint32_t*>(A + (SUB * I + i) * C + SUB * J + jj) =
+            Act<__half>::pack2(__fmul_rn((float)acc[nt][2 * r], sqk), __fmul_rn((float)acc[nt][2 * r + 1], sqk));
+        *reinterpret_cast<uint32_t*>(A + (SUB * J + i) * C + SUB * I + jj) = 0u;  // the block above the diagonal
+      }
   }
 }
 
@@ -834,7 +864,7 @@ static int run_diag_T(const lq_zoo_problem* p, const DiagArgs& a, bool delta, in
     return launch_big_smem(zoo_diag_rows_kernel<T, K, V, false>, "zoo_diag_rows_kernel", grid, smem, a, st);
   }
   if (stage == 1) {
-    const size_t smem = sizeof(float) * (64 * (K + 4) + 64 * 65 + 64 + 2 * 16 * (K + 4) + 8 * 256) + (size_t)(64 * K * 2 + 16 * K + 48 * K);
+    const size_t smem = sizeof(float) * (64 * (K + 4) + K + 64) + (size_t)9 * (K / 32) * 512;
     return launch_big_smem(zoo_diag_amat_kernel<T, K>, "zoo_diag_amat_kernel", grid, smem, a, st);
   }
   const size_t smem = sizeof(float) * (64 * ((K + 4) > (V + 8) ? (K + 4) : (V + 8)) + 64 * (K + 4) + 2 * 64 * 68 + 128 + 8 * 256);
