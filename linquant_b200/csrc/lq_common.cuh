@@ -233,6 +233,16 @@ __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) { F2 r; asm("fma.rn.f32x2 %
 
 __device__ __forceinline__ F2 sub2(F2 a, F2 b) { F2 r; asm("sub.rn.f32x2 %0, %1, %2;\n" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
 
+// e^x of two values as 2^(x log2 e), one hardware exponential each; a result below 2^-126 is zero (the non-flushing form takes
+// three more instructions a value to keep it)
+__device__ __forceinline__ F2 exp_pair(F2 x) {
+  float a, b;
+  mul2(x, F2(1.44269504f, 1.44269504f)).get(a, b);
+  asm("ex2.approx.ftz.f32 %0, %0;\n" : "+f"(a));
+  asm("ex2.approx.ftz.f32 %0, %0;\n" : "+f"(b));
+  return F2(a, b);
+}
+
 // four codes of two pairs, packed: the rule of q8 (fp32 product, clamp, half away from zero)
 template <bool Q127>
 __device__ __forceinline__ uint32_t codes4(F2 x01, F2 x23, F2 inv, float qmax) {
@@ -252,6 +262,15 @@ __device__ __forceinline__ uint32_t codes4(F2 x01, F2 x23, F2 inv, float qmax) {
   for (int i = 0; i < 4; ++i) c[i] = __float2int_rz(y[i]);
   return pack_sat_s8x2(c[1], c[0], pack_sat_s8x2(c[3], c[2], 0u));
 }
+// the codes of a pair (the rule of q8) as fp32 values
+__device__ __forceinline__ F2 code_pair(F2 x, float inv, float qmax) {
+  float y0, y1;
+  mul2(x, F2(inv, inv)).get(y0, y1);
+  y0 = fminf(fmaxf(y0, -qmax), qmax);
+  y1 = fminf(fmaxf(y1, -qmax), qmax);
+  add2(F2(y0, y1), F2(copysignf(0.5f, y0), copysignf(0.5f, y1))).get(y0, y1);
+  return F2(truncf(y0), truncf(y1));
+}
 // INT8 products accumulate on top of the bit pattern of 1.5 * 2^23 (|sum| <= 128 * 127 * 127 < 2^22): the accumulator read as
 // a float is 1.5 * 2^23 + sum, and one subtraction gives the sum exactly, two at a time
 __device__ __forceinline__ void mma_s8_biased(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
@@ -261,18 +280,20 @@ __device__ __forceinline__ void mma_s8_biased(int (&c)[4], uint32_t a0, uint32_t
 }
 __device__ __forceinline__ F2 unbias2(int a, int b) { return add2(F2(__int_as_float(a), __int_as_float(b)), F2(-12582912.f, -12582912.f)); }
 
-// an fp32 value as three bf16 values, biggest first (8 + 8 + 8 bits: the sum is exact), two to a word; eight values
+// two fp32 values as three bf16 pairs, biggest first (8 + 8 + 8 bits: the sum is exact)
+__device__ __forceinline__ void split3_pair(F2 x, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  float a, b;
+  x.get(a, b);
+  hi = Act<__nv_bfloat16>::pack2(a, b);
+  const F2 r = sub2(x, F2(__uint_as_float(hi << 16), __uint_as_float(hi & 0xffff0000u)));
+  r.get(a, b);
+  mid = Act<__nv_bfloat16>::pack2(a, b);
+  sub2(r, F2(__uint_as_float(mid << 16), __uint_as_float(mid & 0xffff0000u))).get(a, b);
+  lo = Act<__nv_bfloat16>::pack2(a, b);
+}
 __device__ __forceinline__ void split3(const float (&x)[8], uint32_t (&hi)[4], uint32_t (&mid)[4], uint32_t (&lo)[4]) {
 #pragma unroll
-  for (int p = 0; p < 4; ++p) {
-    hi[p] = Act<__nv_bfloat16>::pack2(x[2 * p], x[2 * p + 1]);
-    const F2 r = sub2(F2(x[2 * p], x[2 * p + 1]), F2(__uint_as_float(hi[p] << 16), __uint_as_float(hi[p] & 0xffff0000u)));
-    float a, b;
-    r.get(a, b);
-    mid[p] = Act<__nv_bfloat16>::pack2(a, b);
-    sub2(r, F2(__uint_as_float(mid[p] << 16), __uint_as_float(mid[p] & 0xffff0000u))).get(a, b);
-    lo[p] = Act<__nv_bfloat16>::pack2(a, b);
-  }
+  for (int p = 0; p < 4; ++p) split3_pair(F2(x[2 * p], x[2 * p + 1]), hi[p], mid[p], lo[p]);
 }
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {

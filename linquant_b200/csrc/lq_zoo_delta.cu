@@ -33,22 +33,49 @@ struct DeltaPrepArgs {
   float sigma, tau;
 };
 
-template <typename T, int K, int V>
-__global__ void __launch_bounds__(256) zoo_prologue_delta_kernel(DeltaPrepArgs d) {
+// Shared memory: the rotated keys (activation dtype, or fp32 where D_QK is given without a rotation and they are not rounded),
+// the raw values, and a work area that holds G and T = (I + G)^-1, then the fragments of T diag(cw) for W and U.
+template <typename T, int K, int V, bool KF32>
+struct DeltaPrepSmem {
+  typedef typename std::conditional<KF32, float, T>::type KT;
+  static constexpr int LDK = K + (KF32 ? 4 : 8), LDV = V + 8;
+  static constexpr int kK = 4 * (6 * 64 + 4 * K), kV = kK + (int)sizeof(KT) * 64 * LDK, kWork = kV + 2 * 64 * LDV;
+  static constexpr int kBytes = kWork + 4 * 2 * 64 * 68;
+};
+
+// One CTA per chunk, four steps between block barriers:
+//   1  four warps a 16-token tile of k each, four of q: D_QK, Hadamard rotation (sixteen slots of an m16n8k16 product with
+//      the +-1 matrix, the rest a butterfly between the lane's own registers; fp32 operands as three bf16 pieces, exact),
+//      rounding; q codes out, k to shared memory
+//   2  k codes from shared memory (a thread holds four tokens x eight channels, so that the transposed codes are whole words)
+//      and the Gram blocks (exact products of 16-bit keys, fp32 accumulation)
+//   3  the blocked inverse
+//   4  W and U on three-piece products (lq_wy.cuh)
+// Bound by instruction issue and the latency of the inverse. The kernel before it (shuffle Hadamard, fp32 staging, TF32
+// operands split in the product loop; 112 KB of shared memory) took 774 us for 64 (b, h) x 128 chunks at K = V = 128
+// with D_QK; this one 490. Three CTAs per SM at 80 registers spill and gave 867 against 851 us for the whole call.
+template <typename T, int K, int V, bool KF32>
+__global__ void __launch_bounds__(256, 2) zoo_prologue_delta_kernel(DeltaPrepArgs d) {
   pdl_enter();
-  constexpr int C = kChunk, LDK = K + 8, LDV = V + 8;
+  typedef DeltaPrepSmem<T, K, V, KF32> S;
+  typedef typename S::KT KT;
+  constexpr int C = kChunk, LDK = S::LDK, LDV = S::LDV, M = K / 32, KS = K / 64;
+  constexpr bool F16 = std::is_same<T, __half>::value;
   extern __shared__ __align__(16) uint8_t smem_raw[];
   float* s_gc = reinterpret_cast<float*>(smem_raw);
   float* s_fk = s_gc + C;
   float* s_bs = s_fk + C;
   float* s_b1 = s_bs + C;
   float* s_hw = s_b1 + C;
-  float* s_cwW = s_hw + C;  // beta^sigma * exp(gc)
-  float* s_kf = s_cwW + C;
-  float* s_vf = s_kf + C * LDK;
-  float* s_G = s_vf + C * LDV;
+  float* s_cwW = s_hw + C;   // beta^sigma * exp(gc)
+  float* s_ikw = s_cwW + C;  // [K] 1 / k_write scale
+  float* s_sgn = s_ikw + K;  // [K] rotation signs / sqrt(K)
+  float* s_dq = s_sgn + K;   // [2][K] D_QK of q, of k
+  KT* s_k = reinterpret_cast<KT*>(smem_raw + S::kK);
+  T* s_v = reinterpret_cast<T*>(smem_raw + S::kV);
+  float* s_G = reinterpret_cast<float*>(smem_raw + S::kWork);
   float* s_T = s_G + C * 68;
-  uint32_t(*s_kw)[17] = reinterpret_cast<uint32_t(*)[17]>(s_T + C * 68);
+  uint4* s_frag = reinterpret_cast<uint4*>(smem_raw + S::kWork);  // W's fragments, then U's
 
   const PrologueArgs& a = d.pro;
   const int c = blockIdx.x, bh = blockIdx.y;
@@ -56,8 +83,25 @@ __global__ void __launch_bounds__(256) zoo_prologue_delta_kernel(DeltaPrepArgs d
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, j = lane & 3;
   const size_t tile = (size_t)bh * a.NT + c;
+  const size_t tok0 = ((size_t)b * a.T + (size_t)c * C) * a.H + h;
   const float e_hw = (1.f - d.sigma) * d.tau;
+  const bool rot = !KF32 && a.signs != nullptr, dqk = KF32 || a.dqk != nullptr;
 
+  // every global row of the CTA is requested before the first is used
+  const bool isq = warp >= 4;
+  const int t0 = 16 * (warp & 3);
+  const T* src = reinterpret_cast<const T*>(isq ? a.q : a.k);
+  uint4 raw[2][M];
+#pragma unroll
+  for (int r = 0; r < 2; ++r)
+#pragma unroll
+    for (int m = 0; m < M; ++m)
+      raw[r][m] = __ldg(reinterpret_cast<const uint4*>(src + (tok0 + (size_t)(t0 + g + 8 * r) * a.H) * K + 32 * m + 8 * j));
+  for (int i = tid; i < C * V / 8; i += 256) {
+    const int t = i / (V / 8), n = 8 * (i % (V / 8));
+    cp_async16(s_v + t * LDV + n, reinterpret_cast<const T*>(a.v) + (tok0 + (size_t)t * a.H) * V + n);
+  }
+  cp_async_commit();
   if (warp == 0) {
     if (a.g != nullptr) {
       chunk_decay_scan(a.g, b, c, h, a.T, a.H, s_gc);
@@ -66,13 +110,21 @@ __global__ void __launch_bounds__(256) zoo_prologue_delta_kernel(DeltaPrepArgs d
       s_gc[lane + 32] = 0.f;
     }
   }
+  if (tid >= 256 - K) {
+    const int n = tid - (256 - K);
+    s_ikw[n] = 1.0f / a.skw[h * K + n];
+    s_sgn[n] = rot ? a.signs[n] * (K == 64 ? 0.125f : 0.08838834764831845f) : 1.f;
+    const float dm = dqk ? a.dqk[h * K + n] : 1.f;
+    s_dq[n] = dm;
+    s_dq[K + n] = 1.0f / dm;
+  }
   __syncthreads();
   if (tid < C) {
     const float dd = s_gc[C - 1] - s_gc[tid];
     s_fk[tid] = a.g ? expf((1.0f - a.eta) * dd) : 1.0f;
     a.gc[tile * C + tid] = s_gc[tid];
     d.genv[tile * C + tid] = a.g ? expf(a.eta * dd) : 1.0f;
-    const float bt = d.beta[((size_t)b * a.T + (size_t)c * C + tid) * a.H + h];
+    const float bt = d.beta[tok0 + (size_t)tid * a.H];
     const float bs = pow_exact01(bt, d.sigma);
     s_bs[tid] = bs;
     s_b1[tid] = pow_exact01(bt, 1.f - d.sigma);
@@ -80,99 +132,240 @@ __global__ void __launch_bounds__(256) zoo_prologue_delta_kernel(DeltaPrepArgs d
     s_cwW[tid] = a.g ? bs * expf(s_gc[tid]) : bs;
     d.fw[tile * C + tid] = pow_exact01(bt, (1.f - d.sigma) * (1.f - d.tau));
   }
+
+  // ---- 1. rows of q (codes) or k (to shared memory)
+  {
+    const uint32_t one = F16 && !dqk ? 0x3C00u : 0x3F80u;
+    const uint32_t had = [&]() {  // (-1)^popc(s & n) for slots s = 2j, 2j + 1 and column n = g
+      const uint32_t s0 = one | ((__popc((2 * j) & g) & 1) << 15), s1 = one | ((__popc((2 * j + 1) & g) & 1) << 15);
+      return s0 | (s1 << 16);
+    }();
+    const uint32_t hadn = had ^ 0x80008000u;
+    const float* dq = s_dq + (isq ? 0 : K);
+    F2 y[M][2][2][2];  // [m][eh][row half][channel pair]: channel 32 m + 8 j + 4 eh + 2 pair + (0, 1)
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+      uint32_t pc[2][3][4];  // [row half][piece][channel pair of eight]
+      float x[2][8];
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        if (dqk || !rot) Act<T>::unpack8(raw[r][m], x[r]);
+        if (dqk) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) x[r][e] = __fmul_rn(x[r][e], dq[32 * m + 8 * j + e]);
+          if (rot) split3(x[r], pc[r][0], pc[r][1], pc[r][2]);
+        } else {
+          pc[r][0][0] = raw[r][m].x; pc[r][0][1] = raw[r][m].y; pc[r][0][2] = raw[r][m].z; pc[r][0][3] = raw[r][m].w;
+        }
+      }
+#pragma unroll
+      for (int eh = 0; eh < 2; ++eh) {
+        if (rot) {
+          float d0[4] = {0.f, 0.f, 0.f, 0.f}, d1[4] = {0.f, 0.f, 0.f, 0.f};
+          auto mma = [&](int i) {
+            const uint32_t a0 = pc[0][i][2 * eh], a1 = pc[1][i][2 * eh], a2 = pc[0][i][2 * eh + 1], a3 = pc[1][i][2 * eh + 1];
+            mma_bf16(d0, a0, a1, a2, a3, had, had);
+            mma_bf16(d1, a0, a1, a2, a3, had, hadn);
+          };
+          if (dqk) {
+            mma(2);
+            mma(1);
+            mma(0);
+          } else if (F16) {
+            mma_f16(d0, pc[0][0][2 * eh], pc[1][0][2 * eh], pc[0][0][2 * eh + 1], pc[1][0][2 * eh + 1], had, had);
+            mma_f16(d1, pc[0][0][2 * eh], pc[1][0][2 * eh], pc[0][0][2 * eh + 1], pc[1][0][2 * eh + 1], had, hadn);
+          } else {
+            mma(0);
+          }
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            y[m][eh][r][0] = F2(d0[2 * r], d0[2 * r + 1]);
+            y[m][eh][r][1] = F2(d1[2 * r], d1[2 * r + 1]);
+          }
+        } else {
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            y[m][eh][r][0] = F2(x[r][4 * eh], x[r][4 * eh + 1]);
+            y[m][eh][r][1] = F2(x[r][4 * eh + 2], x[r][4 * eh + 3]);
+          }
+        }
+      }
+    }
+    if (rot) {  // the remaining channel bits: 2 (eh), 5 and 6 (m)
+      const F2 neg(-1.f, -1.f);
+      auto fly = [&](F2& p, F2& q) {
+        const F2 s = add2(p, q);
+        q = fma2(q, neg, p);
+        p = s;
+      };
+#pragma unroll
+      for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+#pragma unroll
+          for (int m = 0; m < M; ++m) fly(y[m][0][r][e], y[m][1][r][e]);
+#pragma unroll
+          for (int eh = 0; eh < 2; ++eh) {
+#pragma unroll
+            for (int m = 0; m < M; m += 2) fly(y[m][eh][r][e], y[m + 1][eh][r][e]);
+            if (M == 4) {
+              fly(y[0][eh][r][e], y[2 % M][eh][r][e]);
+              fly(y[1][eh][r][e], y[3 % M][eh][r][e]);
+            }
+          }
+        }
+    }
+    const float inv_sq = 1.0f / a.sq[h];
+    const F2 inv(inv_sq, inv_sq), scale(a.scale, a.scale);
+#pragma unroll
+    for (int m = 0; m < M; ++m)
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const int t = t0 + g + 8 * r;
+        uint32_t w[4];  // the eight channels, rounded to the activation dtype
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+          F2& yy = y[m][p >> 1][r][p & 1];
+          if constexpr (!KF32) {  // not rotated: the factor is 1 and the values are of the activation dtype
+            const float2 sg = *reinterpret_cast<const float2*>(s_sgn + 32 * m + 8 * j + 2 * p);
+            float x0, x1;
+            mul2(yy, F2(sg.x, sg.y)).get(x0, x1);
+            w[p] = Act<T>::pack2(x0, x1);
+            yy = F2(Act<T>::get(w[p], 0), Act<T>::get(w[p], 1));
+          }
+        }
+        if (isq) {
+          uint32_t cd[2];
+#pragma unroll
+          for (int eh = 0; eh < 2; ++eh) {
+            const F2 x01 = mul2(y[m][eh][r][0], scale), x23 = mul2(y[m][eh][r][1], scale);
+            cd[eh] = codes4<false>(x01, x23, inv, a.qmax);
+          }
+          *reinterpret_cast<uint2*>(a.qq + (tile * C + t) * K + 32 * m + 8 * j) = make_uint2(cd[0], cd[1]);
+        } else if constexpr (KF32) {
+          float x[8];
+#pragma unroll
+          for (int p = 0; p < 4; ++p) y[m][p >> 1][r][p & 1].get(x[2 * p], x[2 * p + 1]);
+          *reinterpret_cast<float4*>(s_k + t * LDK + 32 * m + 8 * j) = make_float4(x[0], x[1], x[2], x[3]);
+          *reinterpret_cast<float4*>(s_k + t * LDK + 32 * m + 8 * j + 4) = make_float4(x[4], x[5], x[6], x[7]);
+        } else {
+          *reinterpret_cast<uint4*>(s_k + t * LDK + 32 * m + 8 * j) = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+      }
+  }
   __syncthreads();
 
-  // the v rows are requested before the q / k rows are processed, and staged afterwards
-  const T* vp = reinterpret_cast<const T*>(a.v);
-  constexpr int NV = C * (V / 8) / 256;
-  uint4 rv[NV];
+  // ---- 2. k codes: four tokens x eight channels a thread
+  if (warp < 2 * M) {
+    const int tg = 8 * (warp & 1) + g, n0 = 8 * (4 * (warp >> 1) + j);
+    const float inv_sk = 1.0f / a.sk[h];
+    const F2 inv(inv_sk, inv_sk);
+    float x[4][8];
 #pragma unroll
-  for (int u = 0; u < NV; ++u) {
-    const int i = tid + 256 * u, t = i / (V / 8), seg = i % (V / 8);
-    rv[u] = __ldg(reinterpret_cast<const uint4*>(vp + (((size_t)b * a.T + (size_t)c * C + t) * a.H + h) * V + 8 * seg));
-  }
-  prologue_qk_rows<T, K>(a, b, c, h, tile, s_fk, e_hw != 0.f ? s_hw : nullptr, s_kf, LDK, s_kw);
+    for (int i = 0; i < 4; ++i) {
+      const int t = 4 * tg + i;
+      if constexpr (KF32) {
+        *reinterpret_cast<float4*>(x[i]) = *reinterpret_cast<const float4*>(s_k + t * LDK + n0);
+        *reinterpret_cast<float4*>(x[i] + 4) = *reinterpret_cast<const float4*>(s_k + t * LDK + n0 + 4);
+      } else {
+        Act<T>::unpack8(*reinterpret_cast<const uint4*>(s_k + t * LDK + n0), x[i]);
+      }
+      if (e_hw != 0.f) {
+        const float hw = s_hw[t];
 #pragma unroll
-  for (int u = 0; u < NV; ++u) {
-    const int i = tid + 256 * u, t = i / (V / 8), seg = i % (V / 8);
-    float x[8];
-    Act<T>::unpack8(rv[u], x);
-    *reinterpret_cast<float4*>(s_vf + t * LDV + 8 * seg) = make_float4(x[0], x[1], x[2], x[3]);
-    *reinterpret_cast<float4*>(s_vf + t * LDV + 8 * seg + 4) = make_float4(x[4], x[5], x[6], x[7]);
+        for (int e = 0; e < 8; ++e) x[i][e] = Act<T>::round(__fmul_rn(x[i][e], hw));
+      }
+      uint32_t cd[2];
+#pragma unroll
+      for (int eh = 0; eh < 2; ++eh) {
+        const F2 x01(x[i][4 * eh], x[i][4 * eh + 1]), x23(x[i][4 * eh + 2], x[i][4 * eh + 3]);
+        cd[eh] = codes4<false>(x01, x23, inv, a.qmax);
+      }
+      *reinterpret_cast<uint2*>(a.kl + (tile * C + kl_row_of_token(t)) * K + n0) = make_uint2(cd[0], cd[1]);
+    }
+    const float4 fk = *reinterpret_cast<const float4*>(s_fk + 4 * tg);
+    const F2 fk01(fk.x, fk.y), fk23(fk.z, fk.w);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const float iw = s_ikw[n0 + e];
+      const F2 x01 = mul2(F2(x[0][e], x[1][e]), fk01), x23 = mul2(F2(x[2][e], x[3][e]), fk23), ikw(iw, iw);
+      *reinterpret_cast<uint32_t*>(a.kwT + (tile * K + n0 + e) * C + 4 * tg) =
+          codes4<false>(x01, x23, ikw, a.qmax);
+    }
   }
-  __syncthreads();
-
-  // Work split of the three triangular products. Row tile mt (16 tokens) of G, W and U contracts over 2 mt + 2 steps
-  // of eight tokens, so the cost grows 1 : 2 : 3 : 4 with mt: every warp takes the row tiles pr and 3 - pr (five steps on
-  // average instead of up to eight) and one quarter of the columns.
-  const int pr = warp & 1, qd = warp >> 1;
-  // ---- Gram matrix (strictly lower triangle): 8-column tiles nt <= 2 mt + 1 of row tile mt, ten per pair of row tiles,
-  // dealt round-robin to the pair's four warps. Tiles above the diagonal blocks are never read and stay unwritten.
-  for (int u = qd; u < 10; u += 4) {
-    const int lo = 2 * pr + 2;  // tiles of the lighter row tile of the pair
-    const int mt = u < lo ? pr : 3 - pr, nt = u < lo ? u : u - lo;
-    const int ia = 16 * mt + g, ib = ia + 8;
+  // ---- Gram matrix (strictly lower triangle): the twenty 16 x 8 tiles on and below the diagonal blocks
+  for (int u = warp; u < 20; u += 8) {
+    const int blk = u >> 1, I = blk < 1 ? 0 : blk < 3 ? 1 : blk < 6 ? 2 : 3, J = blk - I * (I + 1) / 2, tj = 16 * J + 8 * (u & 1);
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int kk = 0; kk < K / 8; ++kk) {
-      const int c0 = 8 * kk + j;
-      mma_tf32(acc, __float_as_uint(s_kf[ia * LDK + c0]), __float_as_uint(s_kf[ib * LDK + c0]),
-               __float_as_uint(s_kf[ia * LDK + c0 + 4]), __float_as_uint(s_kf[ib * LDK + c0 + 4]),
-               __float_as_uint(s_kf[(8 * nt + g) * LDK + c0]), __float_as_uint(s_kf[(8 * nt + g) * LDK + c0 + 4]));
+#pragma unroll
+    for (int kk = 0; kk < K / 16; ++kk) {
+      if constexpr (KF32) {  // fp32 keys: three pieces each, six products
+        const float* ra = s_k + (16 * I + g) * LDK + 16 * kk + 2 * j;
+        const float* rb = s_k + (tj + g) * LDK + 16 * kk + 2 * j;
+        uint32_t pa[3][4], pb[3][2];
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+          const float2 x = *reinterpret_cast<const float2*>(ra + (p & 1) * 8 * LDK + (p >> 1) * 8);
+          split3_pair(F2(x.x, x.y), pa[0][p], pa[1][p], pa[2][p]);
+        }
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+          const float2 x = *reinterpret_cast<const float2*>(rb + 8 * p);
+          split3_pair(F2(x.x, x.y), pb[0][p], pb[1][p], pb[2][p]);
+        }
+        auto mma = [&](int i, int k2) { mma_bf16(acc, pa[i][0], pa[i][1], pa[i][2], pa[i][3], pb[k2][0], pb[k2][1]); };
+        mma(2, 0);
+        mma(0, 2);
+        mma(1, 1);
+        mma(1, 0);
+        mma(0, 1);
+        mma(0, 0);
+      } else {
+        uint32_t qa[4], kb[2];
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(qa[0]), "=r"(qa[1]), "=r"(qa[2]), "=r"(qa[3])
+                     : "r"(smem_u32(s_k + (16 * I + (lane & 15)) * LDK + 16 * kk + 8 * (lane >> 4))) : "memory");
+        asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];\n" : "=r"(kb[0]), "=r"(kb[1])
+                     : "r"(smem_u32(s_k + (tj + (lane & 7)) * LDK + 16 * kk + 8 * ((lane >> 3) & 1))) : "memory");
+        if constexpr (F16) mma_f16(acc, qa[0], qa[1], qa[2], qa[3], kb[0], kb[1]);
+        else mma_bf16(acc, qa[0], qa[1], qa[2], qa[3], kb[0], kb[1]);
+      }
     }
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int jj = 8 * nt + 2 * j + e;
-      s_G[ia * 68 + jj] = (ia > jj) ? s_bs[ia] * s_b1[jj] * acc[e] * expf(s_gc[ia] - s_gc[jj]) : 0.f;
-      s_G[ib * 68 + jj] = (ib > jj) ? s_bs[ib] * s_b1[jj] * acc[2 + e] * expf(s_gc[ib] - s_gc[jj]) : 0.f;
+    for (int r = 0; r < 2; ++r) {
+      const int i = 16 * I + g + 8 * r, jj = tj + 2 * j;
+      float v[2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) v[e] = jj + e < i ? s_bs[i] * s_b1[jj + e] * acc[2 * r + e] * expf(s_gc[i] - s_gc[jj + e]) : 0.f;
+      *reinterpret_cast<float2*>(s_G + i * 68 + jj) = make_float2(v[0], v[1]);
     }
   }
+  cp_async_wait<0>();
   __syncthreads();
+  // ---- 3.
   wy_solve(s_G, s_T);
+  // ---- 4. W = T diag(beta^sigma exp(gc)) k  -> w_read codes;  U = T diag(beta^sigma) v  -> activation dtype
+  wy_fragments2(s_T, s_cwW, s_bs, s_frag, warp, lane);  // in the place of G and T
   __syncthreads();
-  const float inv_sw = 1.0f / d.sw[h];
-  T* up = reinterpret_cast<T*>(d.u);
+  {
+    constexpr int NB = KF32 ? 3 : F16 ? 2 : 1;
+    const int n0 = (K / 8) * warp;
+    float acc[4][KS][4];
+    wy_product3<KS, NB>(acc, s_frag, lane, [&](int ks, uint32_t (&bp)[NB][KS][2]) {
+      if constexpr (KF32) {
 #pragma unroll
-  for (int half = 0; half < 2; ++half) {
-    const int mt = half == 0 ? pr : 3 - pr;
-    const int ia = 16 * mt + g, ib = ia + 8;
-    // ---- W = T diag(beta^sigma exp(gc)) k  -> w_read codes
-    {
-      constexpr int NTW = K / 32;
-      float acc[NTW][4];
+        for (int nt = 0; nt < KS; ++nt)
 #pragma unroll
-      for (int nt = 0; nt < NTW; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
-      const int n0 = qd * (K / 4);
-      wy_product<NTW>(acc, s_T, s_cwW, s_kf, LDK, mt, n0, g, j);
-#pragma unroll
-      for (int nt = 0; nt < NTW; ++nt) {
-        const int col = n0 + 8 * nt + 2 * j;
-        const int a0 = q8(Act<T>::round(acc[nt][0]), inv_sw, a.qmax), a1 = q8(Act<T>::round(acc[nt][1]), inv_sw, a.qmax);
-        const int b0 = q8(Act<T>::round(acc[nt][2]), inv_sw, a.qmax), b1 = q8(Act<T>::round(acc[nt][3]), inv_sw, a.qmax);
-        *reinterpret_cast<uint16_t*>(d.wq + tile * (C * K) + wq_offset(ia, col)) = (uint16_t)((a0 & 0xff) | ((a1 & 0xff) << 8));
-        *reinterpret_cast<uint16_t*>(d.wq + tile * (C * K) + wq_offset(ib, col)) = (uint16_t)((b0 & 0xff) | ((b1 & 0xff) << 8));
+          for (int s = 0; s < 2; ++s) {
+            const float* kp = s_k + (16 * ks + 8 * s + 2 * j) * LDK + n0 + 8 * nt + g;
+            split3_pair(F2(kp[0], kp[LDK]), bp[0][nt][s], bp[1][nt][s], bp[2][nt][s]);
+          }
+      } else {
+        wy_pieces16<T, KS>(bp, s_k + 16 * ks * LDK + n0, LDK, lane);
       }
-    }
-    // ---- U = T diag(beta^sigma) v  -> activation dtype
-    {
-      constexpr int NTU = V / 32;
-      float acc[NTU][4];
-#pragma unroll
-      for (int nt = 0; nt < NTU; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
-      const int n0 = qd * (V / 4);
-      wy_product<NTU>(acc, s_T, s_bs, s_vf, LDV, mt, n0, g, j);
-#pragma unroll
-      for (int nt = 0; nt < NTU; ++nt) {
-        const int col = n0 + 8 * nt + 2 * j;
-        T* uc = up + (tile * V + col) * C;  // [V][C]: the token index contiguous
-        uc[ia] = Act<T>::from(acc[nt][0]);
-        uc[C + ia] = Act<T>::from(acc[nt][1]);
-        uc[ib] = Act<T>::from(acc[nt][2]);
-        uc[C + ib] = Act<T>::from(acc[nt][3]);
-      }
-    }
+    });
+    wy_store_w<T, KS>(acc, d.wq + tile * (C * K), n0, 1.0f / d.sw[h], a.qmax, lane);
   }
-  uint32_t* kw_out = reinterpret_cast<uint32_t*>(a.kwT + tile * (size_t)(K * C));
-  for (int i = tid; i < K * 16; i += 256) kw_out[i] = s_kw[i >> 4][i & 15];
+  wy_u<T, V>(s_frag + 30 * 32, s_v, LDV, reinterpret_cast<T*>(d.u) + tile * (size_t)(V * C), warp, lane);
 }
 
 // ------------------------------------------------------------------------------------------------ state pass
@@ -727,10 +920,11 @@ void fill_prologue_args(const lq_zoo_problem* p, const lq_zoo_workspace* ws, Pro
 
 template <typename T, int K, int V>
 static int launch_delta_prep(const DeltaPrepArgs& d, int BH, cudaStream_t st) {
-  constexpr size_t smem = sizeof(float) * (6 * 64 + 64 * (K + 8) + 64 * (V + 8) + 2 * 64 * 68) + sizeof(uint32_t) * K * 17;
-  cudaError_t e = cudaFuncSetAttribute(zoo_prologue_delta_kernel<T, K, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return fail(LQ_ERR_LAUNCH, "delta prologue: cannot opt in to %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
-  launch(zoo_prologue_delta_kernel<T, K, V>, dim3(d.pro.NT, BH), 256, smem, st, d);
+  const dim3 grid(d.pro.NT, BH);
+  const bool kf32 = d.pro.dqk != nullptr && d.pro.signs == nullptr;  // rescaled and not rotated: the keys are not rounded
+  const cudaError_t e = kf32 ? launch_opt_in(zoo_prologue_delta_kernel<T, K, V, true>, grid, 256, DeltaPrepSmem<T, K, V, true>::kBytes, st, d)
+                             : launch_opt_in(zoo_prologue_delta_kernel<T, K, V, false>, grid, 256, DeltaPrepSmem<T, K, V, false>::kBytes, st, d);
+  if (e != cudaSuccess) return fail(LQ_ERR_LAUNCH, "delta prologue: launch failed: %s", cudaGetErrorString(e));
   return check_launch("zoo_prologue_delta_kernel");
 }
 

@@ -232,7 +232,9 @@ __global__ void __launch_bounds__(256) zoo_diag_rows_kernel(DiagArgs a) {
 // The 2^7 (2^6) Hadamard transform is split over the channel bits: bits 0, 1, 3, 4 are the sixteen slots of an m16n8k16 product
 // with the +-1 matrix (exact operands, fp32 accumulation), the others a butterfly between a lane's own registers.
 // Bound by instruction issue. The kernel before it (operands through shared memory, shuffle butterflies, 3xTF32 with the
-// split in the product loop: 42 k warp instructions and 27 block barriers per chunk) took 2070 us for 256 (b, h) x 128 chunks at K = 128; this one 1637.
+// split in the product loop: 42 k warp instructions and 27 block barriers per chunk) took 2070 us for 256 (b, h) x 128 chunks at
+// K = 128, this one 1637; with pairwise exponentials, the channel loop of the diagonal blocks rolled (unrolled, waiting for instructions
+// was the first stall) and one form of the code rule 1236.
 template <typename T, int K>
 __global__ void __launch_bounds__(256) zoo_diag_amat_kernel(DiagArgs a) {
   pdl_enter();
@@ -274,14 +276,15 @@ __global__ void __launch_bounds__(256) zoo_diag_amat_kernel(DiagArgs a) {
   if (warp < 4) {
     // ---------------------------------------------------------------------------------- diagonal block
     const int t0 = SUB * warp;
-    uint4 rq[2][M], rk[2][M];
+    uint4 nq[2], nk[2];  // the rows of the next 32 channels
+    const T* rowp[2][2];
 #pragma unroll
-    for (int r = 0; r < 2; ++r)
-#pragma unroll
-      for (int m = 0; m < M; ++m) {
-        rq[r][m] = __ldg(reinterpret_cast<const uint4*>(qp + grow(t0 + g + 8 * r) + 32 * m));
-        rk[r][m] = __ldg(reinterpret_cast<const uint4*>(kp + grow(t0 + g + 8 * r) + 32 * m));
-      }
+    for (int r = 0; r < 2; ++r) {
+      rowp[r][0] = qp + grow(t0 + g + 8 * r);
+      rowp[r][1] = kp + grow(t0 + g + 8 * r);
+      nq[r] = __ldg(reinterpret_cast<const uint4*>(rowp[r][0]));
+      nk[r] = __ldg(reinterpret_cast<const uint4*>(rowp[r][1]));
+    }
     auto key = [&](const uint4& raw, int t, float (&x)[8]) {  // the readout key of one row piece
       Act<T>::unpack8(raw, x);
       if (use_hw) {
@@ -297,27 +300,35 @@ __global__ void __launch_bounds__(256) zoo_diag_amat_kernel(DiagArgs a) {
     const bool exact = __any_sync(0xffffffffu, spread > 60.f);
     float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
     if (!exact) {
-#pragma unroll
+#pragma unroll 1  // 600 instructions a pass: unrolled, the kernel waits for its instructions
       for (int m = 0; m < M; ++m) {
         float an[8];
         lds8(s_gc + t0 * LD + 32 * m + 8 * j, an);
         uint32_t qh[2][4], qm[2][4], ql[2][4], kh[2][4], km[2][4], kl[2][4];  // [row half][pair of channels]
+        const uint4 rq[2] = {nq[0], nq[1]}, rk[2] = {nk[0], nk[1]};
+        if (m + 1 < M) {
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            nq[r] = __ldg(reinterpret_cast<const uint4*>(rowp[r][0] + 32 * (m + 1)));
+            nk[r] = __ldg(reinterpret_cast<const uint4*>(rowp[r][1] + 32 * (m + 1)));
+          }
+        }
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
           const int t = t0 + g + 8 * r;
-          float x[8], gv[8], e1[8];
+          float x[8], gv[8];
+          F2 e1[4];
           lds8(s_gc + t * LD + 32 * m + 8 * j, gv);
-          Act<T>::unpack8(rq[r][m], x);
+          Act<T>::unpack8(rq[r], x);
 #pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            e1[e] = __fsub_rn(gv[e], an[e]);
-            x[e] = __fmul_rn((float)q8(__fmul_rn(x[e], a.scale), fq, a.qmax), __expf(e1[e]));
+          for (int p = 0; p < 4; ++p) {
+            e1[p] = sub2(F2(gv[2 * p], gv[2 * p + 1]), F2(an[2 * p], an[2 * p + 1]));
+            split3_pair(mul2(code_pair(mul2(F2(x[2 * p], x[2 * p + 1]), F2(a.scale, a.scale)), fq, a.qmax), exp_pair(e1[p])), qh[r][p], qm[r][p], ql[r][p]);
           }
-          split3(x, qh[r], qm[r], ql[r]);
-          key(rk[r][m], t, x);
+          key(rk[r], t, x);
 #pragma unroll
-          for (int e = 0; e < 8; ++e) x[e] = __fmul_rn((float)q8(x[e], fk, a.qmax), __expf(-e1[e]));
-          split3(x, kh[r], km[r], kl[r]);
+          for (int p = 0; p < 4; ++p)
+            split3_pair(mul2(code_pair(F2(x[2 * p], x[2 * p + 1]), fk, a.qmax), exp_pair(mul2(e1[p], F2(-1.f, -1.f)))), kh[r][p], km[r][p], kl[r][p]);
         }
 #pragma unroll
         for (int eh = 0; eh < 2; ++eh) {
@@ -379,7 +390,6 @@ __global__ void __launch_bounds__(256) zoo_diag_amat_kernel(DiagArgs a) {
     const uint32_t s0 = (__popc((2 * j) & g) & 1) ? 0xBC00u : 0x3C00u, s1 = (__popc((2 * j + 1) & g) & 1) ? 0xBC00u : 0x3C00u;
     return s0 | (s1 << 16);
   }();
-  const bool q127 = a.qmax == 127.f;
   for (int it = w4; it < 9; it += 4) {
     const bool isq = it < 3;
     const int u = it - 3;
@@ -404,7 +414,8 @@ __global__ void __launch_bounds__(256) zoo_diag_amat_kernel(DiagArgs a) {
         Act<T>::unpack8(raw[r][m], x[r]);
         if (isq) {
 #pragma unroll
-          for (int e = 0; e < 8; ++e) x[r][e] = __fmul_rn(__fmul_rn(x[r][e], __expf(__fsub_rn(gv[e], an[e]))), a.scale);
+          for (int e = 0; e < 8; e += 2)
+            mul2(mul2(F2(x[r][e], x[r][e + 1]), exp_pair(sub2(F2(gv[e], gv[e + 1]), F2(an[e], an[e + 1])))), F2(a.scale, a.scale)).get(x[r][e], x[r][e + 1]);
         } else {
           if (use_hw) {
             const float hw = s_hw[t];
@@ -412,7 +423,8 @@ __global__ void __launch_bounds__(256) zoo_diag_amat_kernel(DiagArgs a) {
             for (int e = 0; e < 8; ++e) x[r][e] = Act<T>::round(__fmul_rn(x[r][e], hw));
           }
 #pragma unroll
-          for (int e = 0; e < 8; ++e) x[r][e] = __fmul_rn(x[r][e], __expf(__fsub_rn(an[e], gv[e])));
+          for (int e = 0; e < 8; e += 2)
+            mul2(F2(x[r][e], x[r][e + 1]), exp_pair(sub2(F2(an[e], an[e + 1]), F2(gv[e], gv[e + 1])))).get(x[r][e], x[r][e + 1]);
         }
       }
 #pragma unroll
@@ -477,7 +489,7 @@ __global__ void __launch_bounds__(256) zoo_diag_amat_kernel(DiagArgs a) {
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
           const F2 y0 = rot ? mul2(y[m][eh][r][0], s0) : y[m][eh][r][0], y1 = rot ? mul2(y[m][eh][r][1], s1) : y[m][eh][r][1];
-          w[r][eh] = q127 ? codes4<true>(y0, y1, inv, 127.f) : codes4<false>(y0, y1, inv, a.qmax);
+          w[r][eh] = codes4<false>(y0, y1, inv, a.qmax);
         }
       }
       s_code[(it * M + m) * 32 + lane] = make_uint4(w[0][0], w[1][0], w[0][1], w[1][1]);
@@ -512,326 +524,209 @@ __global__ void __launch_bounds__(256) zoo_diag_amat_kernel(DiagArgs a) {
 
 // ------------------------------------------------------------------------------------------------ KDA WY prep
 // Gram matrix G[i][j] = beta_i^sigma beta_j^(1-sigma) sum_n k[i,n] k[j,n] exp(gc[i,n] - gc[j,n]), i > j, in 16-token
-// secondary chunks like the A matrix: inside a diagonal block every (i, j, n) takes its own exp (exponent <= 0);
-// for block row I against the earlier tokens the operands are re-scaled around the anchor row 16 I,
-//   kd[i,n] = k[i,n] exp(gc[i,n] - gc[16I,n]),  ke[j,n] = k[j,n] exp(gc[16I,n] - gc[j,n])   (both factors <= 1),
-// and contracted on the tensor cores as 3xTF32 (big*big + big*small + small*big), which keeps fp32-grade products.
-// W and U are T diag(beta^sigma) times k exp(gc) (3xTF32, both operands split) and times v (exact in TF32).
-template <typename T, int K>
-__device__ __forceinline__ void kda_scaled_rows(const DiagArgs& a, int b, int c, int h, const float* s_gc, float* s_x,
-                                                int anchor_row, int first_row, int nrows, int dst_row, bool toward_anchor) {
-  // rows [first_row, first_row + nrows) of k, times exp(gc[row] - gc[anchor]) (toward_anchor) or exp(gc[anchor] - gc[row]),
-  // or times exp(gc[row]) when anchor_row < 0; written as fp32 to s_x rows dst_row ...
-  constexpr int C = 64, LD = K + 4, LPR = K / 8, MAXIT = C * LPR / 256;
-  const T* kp = reinterpret_cast<const T*>(a.k);
-  // every row piece of the thread is requested before the first is used (at most MAXIT of them: nrows <= 64)
-  uint4 raw[MAXIT];
-#pragma unroll
-  for (int it = 0; it < MAXIT; ++it) {
-    const int i = threadIdx.x + 256 * it;
-    if (i < nrows * LPR) {
-      const int rr = i / LPR, seg = i % LPR;
-      raw[it] = __ldg(reinterpret_cast<const uint4*>(kp + (((size_t)b * a.T + (size_t)c * C + first_row + rr) * a.H + h) * K + 8 * seg));
-    }
-  }
-#pragma unroll
-  for (int it = 0; it < MAXIT; ++it) {
-    const int i = threadIdx.x + 256 * it;
-    if (i >= nrows * LPR) break;
-    const int rr = i / LPR, seg = i % LPR;
-    const int t = first_row + rr;
-    float x[8];
-    Act<T>::unpack8(raw[it], x);
-    const float4 g0 = *reinterpret_cast<const float4*>(s_gc + t * LD + 8 * seg);
-    const float4 g1 = *reinterpret_cast<const float4*>(s_gc + t * LD + 8 * seg + 4);
-    float gv[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
-    if (anchor_row >= 0) {
-      const float4 a0 = *reinterpret_cast<const float4*>(s_gc + anchor_row * LD + 8 * seg);
-      const float4 a1 = *reinterpret_cast<const float4*>(s_gc + anchor_row * LD + 8 * seg + 4);
-      const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-#pragma unroll
-      for (int e = 0; e < 8; ++e) gv[e] = toward_anchor ? __fsub_rn(gv[e], av[e]) : __fsub_rn(av[e], gv[e]);
-    }
-    float y[8];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) y[e] = __fmul_rn(x[e], __expf(gv[e]));
-    *reinterpret_cast<float4*>(s_x + (dst_row + rr) * LD + 8 * seg) = make_float4(y[0], y[1], y[2], y[3]);
-    *reinterpret_cast<float4*>(s_x + (dst_row + rr) * LD + 8 * seg + 4) = make_float4(y[4], y[5], y[6], y[7]);
-  }
-}
+// secondary chunks like the A matrix: for block row I the weight factors around its first row a = 16 I,
+//   kd[i,n] = k[i,n] exp(gc[i,n] - gc[a,n])  (<= 1),   ke[j,n] = k[j,n] exp(gc[a,n] - gc[j,n])  (<= 1 for the earlier blocks),
+// each split into three bf16 pieces (exact) and contracted in six products on the tensor cores. A warp takes a quarter of the
+// channels and block rows 0 and 3, or 1 and 2: seven operand tiles each, made in the registers of the fragments that
+// contract them (a lane holds K/16 consecutive channels of its two rows), and the four quarters are added in a fixed order.
+// W = T diag(beta^sigma) (k exp(gc)) and U = T diag(beta^sigma) v follow on the same three-piece products (lq_wy.cuh).
+// Bound by instruction issue. The kernel before it (operands through shared memory once per block row, 3xTF32 with the split
+// in the product loop, 30 block barriers: 58 k warp instructions a chunk) took 3480 us for 256 (b, h) x 128 chunks at
+// K = V = 128; this one 1692 (1826 before its exponentials and the codes of W were taken in pairs).
+template <int K, int V>
+struct KdaWySmem {
+  static constexpr int LD = K + 4, LDR = K + 8, LDV = V + 8;  // fp32 log-decays, raw k rows, raw v rows
+  static constexpr int kGc = 0, kK = kGc + 4 * 64 * LD, kV = kK + 2 * 64 * LDR;
+  static constexpr int kWork = kV + 2 * 64 * LDV;  // quarter sums of the Gram blocks; then G | T; then the fragments of T in G's place
+  static constexpr int kBeta = kWork + 4 * 10 * 1024, kBytes = kBeta + 4 * 128;
+};
+template <int K, int V>
+constexpr size_t kda_wy_smem() { return KdaWySmem<K, V>::kBytes; }
 
 template <typename T, int K, int V>
-__global__ void __launch_bounds__(256) zoo_kda_wy_kernel(DiagArgs a) {
+__global__ void __launch_bounds__(256, 2) zoo_kda_wy_kernel(DiagArgs a) {
   pdl_enter();
-  constexpr int C = 64, LD = K + 4, LDV = V + 8, SUB = 16;
-  constexpr int REG0 = C * (LD > LDV ? LD : LDV);
+  typedef KdaWySmem<K, V> S;
+  constexpr int C = 64, LD = S::LD, LDR = S::LDR, LDV = S::LDV, SUB = 16, CH = K / 16, KS = K / 64;
+  static_assert(2 * C * 68 * 4 <= 4 * 10 * 1024 && 30 * 512 <= C * 68 * 4, "aliases of the work area");
   extern __shared__ __align__(16) uint8_t smem_raw[];
-  float* s_gc = reinterpret_cast<float*>(smem_raw);  // gc tile; v (fp32) once the decayed keys are formed
-  float* s_x = s_gc + REG0;                          // k (fp32), then anchored operands, then k exp(gc)
-  float* s_G = s_x + C * LD;
+  float* s_gc = reinterpret_cast<float*>(smem_raw + S::kGc);
+  T* s_k = reinterpret_cast<T*>(smem_raw + S::kK);
+  T* s_v = reinterpret_cast<T*>(smem_raw + S::kV);
+  float4* s_part = reinterpret_cast<float4*>(smem_raw + S::kWork);  // [quarter][block][n-tile][lane]
+  float* s_G = reinterpret_cast<float*>(smem_raw + S::kWork);
   float* s_T = s_G + C * 68;
-  float* s_bs = s_T + C * 68;
+  uint4* s_frag = reinterpret_cast<uint4*>(smem_raw + S::kWork);
+  float* s_bs = reinterpret_cast<float*>(smem_raw + S::kBeta);
   float* s_b1 = s_bs + C;
-  float* s_part = s_b1 + C;  // [8 warps][16][16] partial diagonal blocks
-  float* s_vf = s_gc;
 
   const int c = blockIdx.x, bh = blockIdx.y;
   const int b = bh / a.H, h = bh % a.H;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int g = lane >> 2, j4 = lane & 3;
+  const int g = lane >> 2, j = lane & 3;
   const size_t tile = (size_t)bh * a.NT + c;
+  const size_t tok0 = ((size_t)b * a.T + (size_t)c * C) * a.H + h;
 
-  load_gc_tile<K>(a.gc + tile * (size_t)(C * K), s_gc);
-  {
-    const T* kp = reinterpret_cast<const T*>(a.k);
-    constexpr int NIT = C * (K / 8) / 256;
-    uint4 raw[NIT];
-#pragma unroll
-    for (int it = 0; it < NIT; ++it) {
-      const int i = tid + 256 * it, t = i / (K / 8), seg = i % (K / 8);
-      raw[it] = __ldg(reinterpret_cast<const uint4*>(kp + (((size_t)b * a.T + (size_t)c * C + t) * a.H + h) * K + 8 * seg));
-    }
-#pragma unroll
-    for (int it = 0; it < NIT; ++it) {
-      const int i = tid + 256 * it, t = i / (K / 8), seg = i % (K / 8);
-      float x[8];
-      Act<T>::unpack8(raw[it], x);
-      *reinterpret_cast<float4*>(s_x + t * LD + 8 * seg) = make_float4(x[0], x[1], x[2], x[3]);
-      *reinterpret_cast<float4*>(s_x + t * LD + 8 * seg + 4) = make_float4(x[4], x[5], x[6], x[7]);
-    }
+  for (int i = tid; i < C * K / 4; i += 256) {
+    const int t = i / (K / 4), n = 4 * (i % (K / 4));
+    cp_async16(s_gc + t * LD + n, a.gc + (tile * C + t) * K + n);
   }
+  for (int i = tid; i < C * K / 8; i += 256) {
+    const int t = i / (K / 8), n = 8 * (i % (K / 8));
+    cp_async16(s_k + t * LDR + n, reinterpret_cast<const T*>(a.k) + (tok0 + (size_t)t * a.H) * K + n);
+  }
+  cp_async_commit();
+  for (int i = tid; i < C * V / 8; i += 256) {
+    const int t = i / (V / 8), n = 8 * (i % (V / 8));
+    cp_async16(s_v + t * LDV + n, reinterpret_cast<const T*>(a.v) + (tok0 + (size_t)t * a.H) * V + n);
+  }
+  cp_async_commit();
   if (tid < C) {
-    const float bt = a.beta[((size_t)b * a.T + (size_t)c * C + tid) * a.H + h];
+    const float bt = a.beta[tok0 + (size_t)tid * a.H];
     s_bs[tid] = pow_exact01(bt, a.sigma);
     s_b1[tid] = pow_exact01(bt, 1.f - a.sigma);
     a.fw[tile * C + tid] = pow_exact01(bt, (1.f - a.sigma) * (1.f - a.tau));
   }
-  for (int i = tid; i < C * 68; i += 256) s_G[i] = 0.f;
+  cp_async_wait<1>();
   __syncthreads();
 
-  // ---- diagonal blocks (strictly lower pairs of each 16 x 16 block). As in the A matrix the per-channel weight
-  // exp(gc_in - gc_jn) factors around the block's first row a into exp(gc_in - a_n) (<= 1) and exp(a_n - gc_jn) (>= 1): two
-  // sets of 16 scaled rows (in the space of T, which is not needed yet) and a 16 x 16 x K fp32 product. A block whose
-  // decay spread max_n (a_n - gc_last,n) exceeds 60 keeps one exp per (i, j, n).
+  // ---- Gram blocks, one quarter of the channels
   {
-    float* s_kq = s_T;             // [16][LD] k exp(gc_i - a)
-    float* s_kk = s_T + SUB * LD;  // [16][LD] k exp(a - gc_j)
-    __shared__ int s_exact[C / SUB];
-    if (tid < C / SUB) s_exact[tid] = 0;
-    __syncthreads();
-    for (int i = tid; i < (C / SUB) * K; i += 256) {
-      const int I = i / K, n = i - I * K;
-      if (__fsub_rn(s_gc[(SUB * I) * LD + n], s_gc[(SUB * I + SUB - 1) * LD + n]) > 60.f) s_exact[I] = 1;
-    }
-    __syncthreads();
-    for (int I = 0; I < C / SUB; ++I) {
-      if (s_exact[I]) {  // 120 strictly-lower pairs, eight lanes per pair
-        for (int pass = 0; pass < 4; ++pass) {
-          const int rem_raw = pass * 32 + (tid >> 3);
-          const bool valid = rem_raw < 120;  // idle pairs of the last pass compute a clamped pair and store nothing
-          const int rem = valid ? rem_raw : 119;
-          int i = (int)((sqrtf(8.f * rem + 1.f) + 1.f) * 0.5f);
-          while (i * (i + 1) / 2 <= rem) ++i;
-          while (i * (i - 1) / 2 > rem) --i;
-          const int jj = rem - i * (i - 1) / 2;
-          const int ti = SUB * I + i, tj = SUB * I + jj;
-          const int l8 = tid & 7;
-          float sum = 0.f;
+    const int n0 = (K / 4) * (warp & 3) + CH * j;
+    auto ldg = [&](int t, float (&x)[CH]) {
 #pragma unroll
-          for (int n4 = 0; n4 < K / 32; ++n4) {
-            const int n = 4 * l8 + 32 * n4;  // the eight lanes of a pair read 128 consecutive bytes of each row
-            const float4 gi = *reinterpret_cast<const float4*>(s_gc + ti * LD + n), gj = *reinterpret_cast<const float4*>(s_gc + tj * LD + n);
-            const float4 xi = *reinterpret_cast<const float4*>(s_x + ti * LD + n), xj = *reinterpret_cast<const float4*>(s_x + tj * LD + n);
-            sum = fmaf(xi.x * xj.x, __expf(gi.x - gj.x), sum);
-            sum = fmaf(xi.y * xj.y, __expf(gi.y - gj.y), sum);
-            sum = fmaf(xi.z * xj.z, __expf(gi.z - gj.z), sum);
-            sum = fmaf(xi.w * xj.w, __expf(gi.w - gj.w), sum);
-          }
-          sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-          sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-          sum += __shfl_xor_sync(0xffffffffu, sum, 4);
-          if (l8 == 0 && valid) s_G[ti * 68 + tj] = s_bs[ti] * s_b1[tj] * sum;
+      for (int e = 0; e < CH; e += 4) *reinterpret_cast<float4*>(x + e) = *reinterpret_cast<const float4*>(s_gc + t * LD + n0 + e);
+    };
+    auto ldk = [&](int t, float (&x)[CH]) {
+      if constexpr (CH == 8) {
+        Act<T>::unpack8(*reinterpret_cast<const uint4*>(s_k + t * LDR + n0), x);
+      } else {
+        const uint2 w = *reinterpret_cast<const uint2*>(s_k + t * LDR + n0);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) x[e] = Act<T>::get(e < 2 ? w.x : w.y, e & 1);
+      }
+    };
+    for (int half = 0; half < 2; ++half) {
+      const int I = warp < 4 ? 3 * half : 1 + half;
+      float an[CH];
+      ldg(SUB * I, an);
+      uint32_t ah[2][CH / 2], am[2][CH / 2], al[2][CH / 2];  // [row half][pair of channels]
+      float lowest = 0.f;
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        float x[CH], gv[CH];
+        ldg(SUB * I + g + 8 * r, gv);
+        ldk(SUB * I + g + 8 * r, x);
+#pragma unroll
+        for (int p = 0; p < CH / 2; ++p) {
+          const F2 d = sub2(F2(gv[2 * p], gv[2 * p + 1]), F2(an[2 * p], an[2 * p + 1]));
+          float d0, d1;
+          d.get(d0, d1);
+          lowest = fminf(lowest, fminf(d0, d1));
+          split3_pair(mul2(F2(x[2 * p], x[2 * p + 1]), exp_pair(d)), ah[r][p], am[r][p], al[r][p]);
         }
-        __syncthreads();
-        continue;
       }
-      for (int i = tid; i < SUB * (K / 4); i += 256) {
-        const int rr = i / (K / 4), n = 4 * (i - rr * (K / 4));
-        const int t = SUB * I + rr;
-        const float4 an = *reinterpret_cast<const float4*>(s_gc + (SUB * I) * LD + n);
-        const float4 gt = *reinterpret_cast<const float4*>(s_gc + t * LD + n);
-        const float4 xv = *reinterpret_cast<const float4*>(s_x + t * LD + n);
-        *reinterpret_cast<float4*>(s_kq + rr * LD + n) = make_float4(__fmul_rn(xv.x, __expf(gt.x - an.x)), __fmul_rn(xv.y, __expf(gt.y - an.y)),
-                                                                     __fmul_rn(xv.z, __expf(gt.z - an.z)), __fmul_rn(xv.w, __expf(gt.w - an.w)));
-        *reinterpret_cast<float4*>(s_kk + rr * LD + n) = make_float4(__fmul_rn(xv.x, __expf(an.x - gt.x)), __fmul_rn(xv.y, __expf(an.y - gt.y)),
-                                                                     __fmul_rn(xv.z, __expf(an.z - gt.z)), __fmul_rn(xv.w, __expf(an.w - gt.w)));
-      }
-      __syncthreads();
-      {  // 16 x 16 x K product on the tensor cores, 3xTF32, as in the A matrix: warp w contracts the channels
-         // [K/8 w, K/8 (w + 1)), the eight partial blocks are summed in a fixed order
+      // the factors of the diagonal block stay in fp32's range unless the decay across it is beyond e^60
+      const bool exact = __any_sync(0xffffffffu, lowest < -60.f);
+      for (int J = 0; J <= I; ++J) {
         float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+        if (J < I || !exact) {
+          uint32_t bh_[2][CH / 2], bm[2][CH / 2], bl[2][CH / 2];
 #pragma unroll
-        for (int kk = 0; kk < K / 64; ++kk) {
-          const int c0 = (K / 8) * warp + 8 * kk + j4, c1 = c0 + 4;
-          const float xa[4] = {s_kq[g * LD + c0], s_kq[(g + 8) * LD + c0], s_kq[g * LD + c1], s_kq[(g + 8) * LD + c1]};
-          uint32_t ab[4], as_[4];
+          for (int r = 0; r < 2; ++r) {
+            float x[CH], gv[CH];
+            ldg(SUB * J + g + 8 * r, gv);
+            ldk(SUB * J + g + 8 * r, x);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            ab[e] = tf32_rna(xa[e]);
-            as_[e] = tf32_rna(xa[e] - __uint_as_float(ab[e]));
+            for (int p = 0; p < CH / 2; ++p) {
+              const F2 w = exp_pair(sub2(F2(an[2 * p], an[2 * p + 1]), F2(gv[2 * p], gv[2 * p + 1])));
+              split3_pair(mul2(F2(x[2 * p], x[2 * p + 1]), w), bh_[r][p], bm[r][p], bl[r][p]);
+            }
           }
+          auto mma = [&](const uint32_t (&qa)[2][CH / 2], const uint32_t (&kb)[2][CH / 2], int p) {
 #pragma unroll
-          for (int nt = 0; nt < 2; ++nt) {
-            const float y0 = s_kk[(8 * nt + g) * LD + c0], y1 = s_kk[(8 * nt + g) * LD + c1];
-            const uint32_t b0 = tf32_rna(y0), b1 = tf32_rna(y1);
-            const uint32_t s0 = tf32_rna(y0 - __uint_as_float(b0)), s1 = tf32_rna(y1 - __uint_as_float(b1));
-            mma_tf32(acc[nt], as_[0], as_[1], as_[2], as_[3], b0, b1);
-            mma_tf32(acc[nt], ab[0], ab[1], ab[2], ab[3], s0, s1);
-            mma_tf32(acc[nt], ab[0], ab[1], ab[2], ab[3], b0, b1);
+            for (int nt = 0; nt < 2; ++nt) mma_bf16(acc[nt], qa[0][p], qa[1][p], qa[0][p + 1], qa[1][p + 1], kb[nt][p], kb[nt][p + 1]);
+          };
+#pragma unroll
+          for (int p = 0; p < CH / 2; p += 2) {
+            mma(al, bh_, p);
+            mma(ah, bl, p);
+            mma(am, bm, p);
+            mma(am, bh_, p);
+            mma(ah, bm, p);
+            mma(ah, bh_, p);
+          }
+        } else {
+          // one exp per (i, j, channel), a lane for each of its eight (i, j) of the accumulator layout
+          for (int n = (K / 4) * (warp & 3); n < (K / 4) * (warp & 3) + K / 4; ++n) {
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const int ti = SUB * I + g + 8 * (e >> 1), tj = SUB * I + 8 * nt + 2 * j + (e & 1);
+                const float w = tj < ti ? __expf(s_gc[ti * LD + n] - s_gc[tj * LD + n]) : 0.f;
+                acc[nt][e] = fmaf(Act<T>::to(s_k[ti * LDR + n]) * Act<T>::to(s_k[tj * LDR + n]), w, acc[nt][e]);
+              }
           }
         }
+        const int blk = I * (I + 1) / 2 + J;
 #pragma unroll
-        for (int nt = 0; nt < 2; ++nt) {
-          float* pw = s_part + warp * 256;
-          pw[g * 16 + 8 * nt + 2 * j4] = acc[nt][0];
-          pw[g * 16 + 8 * nt + 2 * j4 + 1] = acc[nt][1];
-          pw[(g + 8) * 16 + 8 * nt + 2 * j4] = acc[nt][2];
-          pw[(g + 8) * 16 + 8 * nt + 2 * j4 + 1] = acc[nt][3];
-        }
-        __syncthreads();
-        const int i = tid >> 4, jj = tid & 15;
-        if (jj < i) {
-          float sum = 0.f;
-#pragma unroll
-          for (int w = 0; w < 8; ++w) sum += s_part[w * 256 + tid];
-          const int ti = SUB * I + i;
-          s_G[ti * 68 + SUB * I + jj] = s_bs[ti] * s_b1[SUB * I + jj] * sum;
-        }
+        for (int nt = 0; nt < 2; ++nt)
+          s_part[(((warp & 3) * 10 + blk) * 2 + nt) * 32 + lane] = make_float4(acc[nt][0], acc[nt][1], acc[nt][2], acc[nt][3]);
       }
-      __syncthreads();
     }
   }
-
-  // ---- off-diagonal blocks: block row I against tokens [0, 16 I), anchored at row 16 I
-  for (int I = 1; I < C / SUB; ++I) {
-    kda_scaled_rows<T, K>(a, b, c, h, s_gc, s_x, SUB * I, 0, SUB * I, 0, false);        // ke -> rows 0 .. 16I-1
-    kda_scaled_rows<T, K>(a, b, c, h, s_gc, s_x, SUB * I, SUB * I, SUB, 48, true);      // kd -> rows 48 .. 63
-    __syncthreads();
-    // 2 I column tiles of eight tokens x four quarters of the channels = 8 I units of work, dealt to the eight warps
-    // (one column tile per warp would leave 8 - 2 I warps idle); the quarter sums are parked in the space of T, which is
-    // not needed before the solve, and added in a fixed order.
-    for (int u = warp; u < 8 * I; u += 8) {
-      const int nt = u >> 2, kq = u & 3;
-      float acc[4] = {0.f, 0.f, 0.f, 0.f};
-      const float* ra = s_x + (48 + g) * LD;
-      const float* rb = s_x + (56 + g) * LD;
-      const float* rn = s_x + (8 * nt + g) * LD;
-#pragma unroll
-      for (int ks = 0; ks < K / 32; ++ks) {
-        const int c0 = 8 * (kq * (K / 32) + ks) + j4, c1 = c0 + 4;
-        const float xa[4] = {ra[c0], rb[c0], ra[c1], rb[c1]};
-        const float xb[2] = {rn[c0], rn[c1]};
-        uint32_t ab[4], as_[4], bb[2], bs_[2];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          ab[e] = tf32_rna(xa[e]);
-          as_[e] = tf32_rna(xa[e] - __uint_as_float(ab[e]));
-        }
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          bb[e] = tf32_rna(xb[e]);
-          bs_[e] = tf32_rna(xb[e] - __uint_as_float(bb[e]));
-        }
-        mma_tf32(acc, as_[0], as_[1], as_[2], as_[3], bb[0], bb[1]);
-        mma_tf32(acc, ab[0], ab[1], ab[2], ab[3], bs_[0], bs_[1]);
-        mma_tf32(acc, ab[0], ab[1], ab[2], ab[3], bb[0], bb[1]);
-      }
-      float* pp = s_T + u * 128;  // [16 rows][8 columns]
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        pp[g * 8 + 2 * j4 + e] = acc[e];
-        pp[(g + 8) * 8 + 2 * j4 + e] = acc[2 + e];
-      }
-    }
-    __syncthreads();
-    for (int el = tid; el < 256 * I; el += 256) {
-      const int i = el / (16 * I), jj = el - i * (16 * I);
-      const float* pp = s_T + (4 * (jj >> 3)) * 128 + i * 8 + (jj & 7);
-      const float sum = ((pp[0] + pp[128]) + pp[256]) + pp[384];
-      const int ia = SUB * I + i;
-      s_G[ia * 68 + jj] = s_bs[ia] * s_b1[jj] * sum;
-    }
-    __syncthreads();
-  }
-  wy_solve(s_G, s_T);
-  // decayed keys k * exp(gc) (the Gram passes are done); then the gc region is free for v
-  kda_scaled_rows<T, K>(a, b, c, h, s_gc, s_x, -1, 0, C, 0, false);
   __syncthreads();
-  {
-    const T* vp = reinterpret_cast<const T*>(a.v);
-    constexpr int NIT = C * (V / 8) / 256;
-    uint4 raw[NIT];
+  {  // 10 blocks x 2 n-tiles x 32 lanes, summed in registers: G takes the place of the quarter sums
+    float4 sum[3];
 #pragma unroll
-    for (int it = 0; it < NIT; ++it) {
-      const int i = tid + 256 * it, t = i / (V / 8), seg = i % (V / 8);
-      raw[it] = __ldg(reinterpret_cast<const uint4*>(vp + (((size_t)b * a.T + (size_t)c * C + t) * a.H + h) * V + 8 * seg));
+    for (int it = 0; it < 3; ++it) {
+      const int f = tid + 256 * it;
+      if (f < 640) {
+        const float4 p0 = s_part[f], p1 = s_part[640 + f], p2 = s_part[1280 + f], p3 = s_part[1920 + f];
+        sum[it] = make_float4(((p0.x + p1.x) + p2.x) + p3.x, ((p0.y + p1.y) + p2.y) + p3.y, ((p0.z + p1.z) + p2.z) + p3.z,
+                              ((p0.w + p1.w) + p2.w) + p3.w);
+      }
     }
+    cp_async_wait<0>();  // v: seen by all after the barriers of the solve
+    __syncthreads();
 #pragma unroll
-    for (int it = 0; it < NIT; ++it) {
-      const int i = tid + 256 * it, t = i / (V / 8), seg = i % (V / 8);
-      float x[8];
-      Act<T>::unpack8(raw[it], x);
-      *reinterpret_cast<float4*>(s_vf + t * LDV + 8 * seg) = make_float4(x[0], x[1], x[2], x[3]);
-      *reinterpret_cast<float4*>(s_vf + t * LDV + 8 * seg + 4) = make_float4(x[4], x[5], x[6], x[7]);
+    for (int it = 0; it < 3; ++it) {
+      const int f = tid + 256 * it;
+      if (f < 640) {
+        const int blk = f >> 6, I = blk < 1 ? 0 : blk < 3 ? 1 : blk < 6 ? 2 : 3, J = blk - I * (I + 1) / 2;
+        const int i = SUB * I + g, jj = SUB * J + 8 * ((f >> 5) & 1) + 2 * j;
+        const float c0 = s_b1[jj], c1 = s_b1[jj + 1];
+        *reinterpret_cast<float2*>(s_G + i * 68 + jj) = make_float2(jj < i ? s_bs[i] * c0 * sum[it].x : 0.f, jj + 1 < i ? s_bs[i] * c1 * sum[it].y : 0.f);
+        *reinterpret_cast<float2*>(s_G + (i + 8) * 68 + jj) =
+            make_float2(jj < i + 8 ? s_bs[i + 8] * c0 * sum[it].z : 0.f, jj + 1 < i + 8 ? s_bs[i + 8] * c1 * sum[it].w : 0.f);
+      }
     }
   }
-  // Row tile mt of W and U contracts over 2 mt + 2 steps of eight tokens: every warp takes the row tiles pr and 3 - pr
-  // (five steps on average instead of up to eight) and one quarter of the columns.
-  const int pr = warp & 1, qd = warp >> 1;
-  const float inv_sw = 1.0f / a.sw[h];
+  __syncthreads();
+  wy_solve(s_G, s_T);
+  wy_fragments(s_T, s_bs, s_frag, warp, lane);  // in the place of G
+  __syncthreads();
   // ---- W = T diag(beta^sigma) (k exp(gc))  -> w_read codes
+  {
+    const int n0 = (K / 8) * warp;
+    float acc[4][KS][4];
+    wy_product3<KS, 3>(acc, s_frag, lane, [&](int ks, uint32_t (&bp)[3][KS][2]) {
+      uint32_t raw[KS][2];
+      wy_ldmatrix<KS>(raw, s_k + 16 * ks * LDR + n0, LDR, lane);
 #pragma unroll
-  for (int half = 0; half < 2; ++half) {
-    const int mt = half == 0 ? pr : 3 - pr;
-    constexpr int NTW = K / 32;
-    float acc[NTW][4];
+      for (int nt = 0; nt < KS; ++nt)
 #pragma unroll
-    for (int nt = 0; nt < NTW; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
-    const int n0 = qd * (K / 4);
-    wy_product_split<NTW>(acc, s_T, s_bs, s_x, LD, mt, n0, g, j4);
-    const int ia = 16 * mt + g, ib = ia + 8;
-#pragma unroll
-    for (int nt = 0; nt < NTW; ++nt) {
-      const int col = n0 + 8 * nt + 2 * j4;
-      const int a0 = q8(Act<T>::round(acc[nt][0]), inv_sw, a.qmax), a1 = q8(Act<T>::round(acc[nt][1]), inv_sw, a.qmax);
-      const int b0 = q8(Act<T>::round(acc[nt][2]), inv_sw, a.qmax), b1 = q8(Act<T>::round(acc[nt][3]), inv_sw, a.qmax);
-      *reinterpret_cast<uint16_t*>(a.wq + tile * (C * K) + wq_offset(ia, col)) = (uint16_t)((a0 & 0xff) | ((a1 & 0xff) << 8));
-      *reinterpret_cast<uint16_t*>(a.wq + tile * (C * K) + wq_offset(ib, col)) = (uint16_t)((b0 & 0xff) | ((b1 & 0xff) << 8));
-    }
+        for (int s = 0; s < 2; ++s) {
+          const float* gp = s_gc + (16 * ks + 8 * s + 2 * j) * LD + n0 + 8 * nt + g;
+          split3_pair(mul2(F2(Act<T>::get(raw[nt][s], 0), Act<T>::get(raw[nt][s], 1)), exp_pair(F2(gp[0], gp[LD]))), bp[0][nt][s], bp[1][nt][s],
+                      bp[2][nt][s]);
+        }
+    });
+    wy_store_w<T, KS>(acc, a.wq + tile * (C * K), n0, 1.0f / a.sw[h], a.qmax, lane);
   }
-  __syncthreads();  // v staged by all threads
-  // ---- U = T diag(beta^sigma) v (v is exact in TF32)
-  T* up = reinterpret_cast<T*>(a.u);
-#pragma unroll
-  for (int half = 0; half < 2; ++half) {
-    const int mt = half == 0 ? pr : 3 - pr;
-    constexpr int NTU = V / 32;
-    float acc[NTU][4];
-#pragma unroll
-    for (int nt = 0; nt < NTU; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
-    const int n0 = qd * (V / 4);
-    wy_product<NTU>(acc, s_T, s_bs, s_vf, LDV, mt, n0, g, j4);
-    const int ia = 16 * mt + g, ib = ia + 8;
-#pragma unroll
-    for (int nt = 0; nt < NTU; ++nt) {
-      const int col = n0 + 8 * nt + 2 * j4;
-      T* uc = up + (tile * V + col) * C;  // [V][C]: the token index contiguous
-      uc[ia] = Act<T>::from(acc[nt][0]);
-      uc[C + ia] = Act<T>::from(acc[nt][1]);
-      uc[ib] = Act<T>::from(acc[nt][2]);
-      uc[C + ib] = Act<T>::from(acc[nt][3]);
-    }
-  }
+  // ---- U = T diag(beta^sigma) v
+  wy_u<T, V>(s_frag, s_v, LDV, reinterpret_cast<T*>(a.u) + tile * (size_t)(V * C), warp, lane);
 }
 
 // ------------------------------------------------------------------------------------------------ launchers
@@ -867,8 +762,7 @@ static int run_diag_T(const lq_zoo_problem* p, const DiagArgs& a, bool delta, in
     const size_t smem = sizeof(float) * (64 * (K + 4) + K + 64) + (size_t)9 * (K / 32) * 512;
     return launch_big_smem(zoo_diag_amat_kernel<T, K>, "zoo_diag_amat_kernel", grid, smem, a, st);
   }
-  const size_t smem = sizeof(float) * (64 * ((K + 4) > (V + 8) ? (K + 4) : (V + 8)) + 64 * (K + 4) + 2 * 64 * 68 + 128 + 8 * 256);
-  return launch_big_smem(zoo_kda_wy_kernel<T, K, V>, "zoo_kda_wy_kernel", grid, smem, a, st);
+  return launch_big_smem(zoo_kda_wy_kernel<T, K, V>, "zoo_kda_wy_kernel", grid, kda_wy_smem<K, V>(), a, st);
 }
 
 template <typename T>
