@@ -284,13 +284,16 @@ __global__ void __launch_bounds__(256, 2) zoo_prologue_delta_kernel(DeltaPrepArg
       *reinterpret_cast<uint2*>(a.kl + (tile * C + kl_row_of_token(t)) * K + n0) = make_uint2(cd[0], cd[1]);
     }
     const float4 fk = *reinterpret_cast<const float4*>(s_fk + 4 * tg);
-    const F2 fk01(fk.x, fk.y), fk23(fk.z, fk.w);
+    const F2 f[4] = {F2(fk.x, fk.x), F2(fk.y, fk.y), F2(fk.z, fk.z), F2(fk.w, fk.w)};
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const float iw = s_ikw[n0 + e];
-      const F2 x01 = mul2(F2(x[0][e], x[1][e]), fk01), x23 = mul2(F2(x[2][e], x[3][e]), fk23), ikw(iw, iw);
-      *reinterpret_cast<uint32_t*>(a.kwT + (tile * K + n0 + e) * C + 4 * tg) =
-          codes4<false>(x01, x23, ikw, a.qmax);
+    for (int p = 0; p < 4; ++p) {  // codes of channel pairs, then words of four tokens
+      F2 w[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) w[i] = mul2(F2(x[i][2 * p], x[i][2 * p + 1]), f[i]);
+      const F2 ikw(s_ikw[n0 + 2 * p], s_ikw[n0 + 2 * p + 1]);
+      const uint32_t lo = codes4<false>(w[0], w[1], ikw, a.qmax), hi = codes4<false>(w[2], w[3], ikw, a.qmax);
+      *reinterpret_cast<uint32_t*>(a.kwT + (tile * K + n0 + 2 * p) * C + 4 * tg) = __byte_perm(lo, hi, 0x6420);
+      *reinterpret_cast<uint32_t*>(a.kwT + (tile * K + n0 + 2 * p + 1) * C + 4 * tg) = __byte_perm(lo, hi, 0x7531);
     }
   }
   // ---- Gram matrix (strictly lower triangle): the twenty 16 x 8 tiles on and below the diagonal blocks

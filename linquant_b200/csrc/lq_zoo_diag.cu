@@ -48,174 +48,169 @@ __device__ __forceinline__ void load_gc_tile(const float* gc_tile, float* s_gc) 
 }
 
 // ------------------------------------------------------------------------------------------------ rows
+// Work items of a warp: 32 tokens x 32 channels of q and k, or of v; a thread takes four tokens x eight channels, so that the
+// transposed codes are whole words and go straight to global memory (32 contiguous bytes per channel). The q / k rows travel
+// during the decay scan. Bound by instruction issue and the scan's latency. The kernel before it (codes one at a time,
+// transposed through shared memory, rows requested after the scan) took 892 us for 256 (b, h) x 128 chunks at K = 128 (KDA)
+// and 88 us for 32 x 64 with K = V = 128 (GLA); this one 584
+// (0.98 of the time its 3.8 GB take at 6.55 TB/s) and 56.
+template <int K, int V>
+constexpr size_t diag_rows_smem() { return sizeof(float) * (64 * (K + 4) + 128 + K + 2 * V); }
+
 template <typename T, int K, int V, bool DELTA>
-__global__ void __launch_bounds__(256) zoo_diag_rows_kernel(DiagArgs a) {
+__global__ void __launch_bounds__(256, 3) zoo_diag_rows_kernel(DiagArgs a) {
   pdl_enter();
-  constexpr int C = 64, LD = K + 4;
+  constexpr int C = 64, LD = K + 4, NQK = K / 16;
   extern __shared__ __align__(16) uint8_t smem_raw[];
   float* s_gc = reinterpret_cast<float*>(smem_raw);
   float* s_le = s_gc + C * LD;
   float* s_hw = s_le + C;
-  uint32_t(*s_kw)[17] = reinterpret_cast<uint32_t(*)[17]>(s_hw + C);
-  uint32_t(*s_vl)[17] = s_kw + K;
-  uint32_t(*s_vw)[17] = s_vl + V;
+  float* s_ikw = s_hw + C;  // [K] 1 / scale
+  float* s_ivl = s_ikw + K;  // [V]
+  float* s_ivw = s_ivl + V;  // [V]
 
   const int c = blockIdx.x, bh = blockIdx.y;
   const int b = bh / a.H, h = bh % a.H;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const size_t tile = (size_t)bh * a.NT + c;
+  const size_t tok0 = ((size_t)b * a.T + (size_t)c * C) * a.H + h;
   const float e_hw = (1.f - a.sigma) * a.tau;
+  const int lt = 4 * (lane >> 2), ln = 8 * (lane & 3);  // the thread's first token and channel in an item
 
-  // stage the raw log-decays of the chunk (coalesced), then one thread per channel scans them in double
-  {
-    constexpr int NIT = C * (K / 4) / 256;
-    float4 v[NIT];
+  // the raw log-decays of the chunk, and the rows of the warp's q / k item
+  for (int i = tid; i < C * (K / 4); i += 256) {
+    const int t = i / (K / 4), n = 4 * (i % (K / 4));
+    cp_async16(s_gc + t * LD + n, a.g + (tok0 + (size_t)t * a.H) * K + n);
+  }
+  cp_async_commit();
+  uint4 rq[4], rk[4];
+  if (warp < NQK) {
+    const int t0 = 32 * (warp & 1) + lt, n0 = 32 * (warp >> 1) + ln;
 #pragma unroll
-    for (int it = 0; it < NIT; ++it) {
-      const int i = tid + 256 * it, t = i / (K / 4), c4 = i % (K / 4);
-      v[it] = __ldg(reinterpret_cast<const float4*>(a.g + (((size_t)b * a.T + (size_t)c * C + t) * a.H + h) * K) + c4);
-    }
-#pragma unroll
-    for (int it = 0; it < NIT; ++it) {
-      const int i = tid + 256 * it, t = i / (K / 4), c4 = i % (K / 4);
-      *reinterpret_cast<float4*>(s_gc + t * LD + 4 * c4) = v[it];
+    for (int i = 0; i < 4; ++i) {
+      const size_t row = (tok0 + (size_t)(t0 + i) * a.H) * K + n0;
+      rq[i] = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(a.q) + row));
+      rk[i] = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(a.k) + row));
     }
   }
-  if (DELTA && tid >= 128 && tid < 128 + C) {
-    const int t = tid - 128;
-    const float bt = a.beta[((size_t)b * a.T + (size_t)c * C + t) * a.H + h];
-    s_hw[t] = pow_exact01(bt, e_hw);
-  }
+  cp_async_wait<0>();
   __syncthreads();
+  // one thread per channel scans in double; the others form the reciprocal scales
   if (tid < K) {
     double acc = 0.0;
     float f = 0.f;
-#pragma unroll 8
-    for (int t = 0; t < C; ++t) {
-      acc += (double)s_gc[t * LD + tid];
-      f = (float)acc;
-      s_gc[t * LD + tid] = f;
+#pragma unroll 1
+    for (int t0 = 0; t0 < C; t0 += 16) {
+      float x[16];
+#pragma unroll
+      for (int t = 0; t < 16; ++t) x[t] = s_gc[(t0 + t) * LD + tid];
+#pragma unroll
+      for (int t = 0; t < 16; ++t) {
+        acc += (double)x[t];
+        f = (float)acc;
+        s_gc[(t0 + t) * LD + tid] = f;
+      }
     }
     a.gcl[tile * K + tid] = expf(f);
+  } else {
+    for (int i = tid - K; i < K; i += 256 - K) s_ikw[i] = 1.0f / a.skw[h * K + i];
+    if (!DELTA) {
+      for (int i = tid - K; i < V; i += 256 - K) {
+        s_ivl[i] = 1.0f / a.svl[h * V + i];
+        s_ivw[i] = 1.0f / a.svw[h * V + i];
+      }
+    } else if (tid >= 256 - C) {
+      const int t = tid - (256 - C);
+      s_hw[t] = pow_exact01(a.beta[tok0 + (size_t)t * a.H], e_hw);
+    }
   }
   __syncthreads();
   for (int i = tid; i < C * (K / 4); i += 256) {
     const int t = i / (K / 4), c4 = i % (K / 4);
     reinterpret_cast<float4*>(a.gc + (tile * C + t) * K)[c4] = *reinterpret_cast<const float4*>(s_gc + t * LD + 4 * c4);
   }
-  __syncthreads();
-  for (int tt = 0; tt < 8; ++tt) {
-    const int t = 8 * warp + tt;
-    float m = -INFINITY;
-    for (int n = lane; n < K; n += 32) m = fmaxf(m, s_gc[(C - 1) * LD + n] - s_gc[t * LD + n]);
+  if (a.eta != 0.f) {  // log envelope: with eta = 0 every gate is 1
+    for (int tt = 0; tt < 8; ++tt) {
+      const int t = 8 * warp + tt;
+      float m = -INFINITY;
+      for (int n = lane; n < K; n += 32) m = fmaxf(m, s_gc[(C - 1) * LD + n] - s_gc[t * LD + n]);
 #pragma unroll
-    for (int d = 16; d > 0; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
-    if (lane == 0) {
-      s_le[t] = m;
-      a.genv[tile * C + t] = expf(a.eta * m);
+      for (int d = 16; d > 0; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
+      if (lane == 0) {
+        s_le[t] = a.eta * m;
+        a.genv[tile * C + t] = expf(a.eta * m);
+      }
     }
+    __syncthreads();
+  } else if (tid < C) {
+    a.genv[tile * C + tid] = 1.f;
   }
-  __syncthreads();
 
-  {
-    constexpr int LPR = K / 8, G = 32 / LPR;
-    const int r = lane % LPR, grp = lane / LPR;
+  // words of four tokens from codes of channel pairs: channels n, n + 1 of tokens 0, 1 and of tokens 2, 3
+  auto put = [&](int8_t* dst, const F2 (&x)[4], F2 inv) {
+    const uint32_t lo = codes4<false>(x[0], x[1], inv, a.qmax), hi = codes4<false>(x[2], x[3], inv, a.qmax);
+    *reinterpret_cast<uint32_t*>(dst) = __byte_perm(lo, hi, 0x6420);
+    *reinterpret_cast<uint32_t*>(dst + C) = __byte_perm(lo, hi, 0x7531);
+  };
+  if (warp < NQK) {
+    const int t0 = 32 * (warp & 1) + lt, n0 = 32 * (warp >> 1) + ln;
     const float inv_sq = 1.0f / a.sq[h];
-    float inv_kw[8], gl[8];
+    const F2 inv(inv_sq, inv_sq), scale(a.scale, a.scale);
+    F2 gl[4], y[4][4];  // [token][channel pair]
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      inv_kw[j] = 1.0f / a.skw[h * K + 8 * r + j];
-      gl[j] = s_gc[(C - 1) * LD + 8 * r + j];
+    for (int p = 0; p < 4; ++p) gl[p] = F2(s_gc[(C - 1) * LD + n0 + 2 * p], s_gc[(C - 1) * LD + n0 + 2 * p + 1]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int t = t0 + i;
+      float x[8], gv[8];
+      *reinterpret_cast<float4*>(gv) = *reinterpret_cast<const float4*>(s_gc + t * LD + n0);
+      *reinterpret_cast<float4*>(gv + 4) = *reinterpret_cast<const float4*>(s_gc + t * LD + n0 + 4);
+      Act<T>::unpack8(rq[i], x);
+      uint32_t cd[2];
+#pragma unroll
+      for (int eh = 0; eh < 2; ++eh) {
+        const int e = 4 * eh;
+        cd[eh] = codes4<false>(mul2(mul2(F2(x[e], x[e + 1]), exp_pair(F2(gv[e], gv[e + 1]))), scale),
+                               mul2(mul2(F2(x[e + 2], x[e + 3]), exp_pair(F2(gv[e + 2], gv[e + 3]))), scale), inv, a.qmax);
+      }
+      *reinterpret_cast<uint2*>(a.qq + (tile * C + t) * K + n0) = make_uint2(cd[0], cd[1]);
+      Act<T>::unpack8(rk[i], x);
+      if (DELTA && e_hw != 0.f) {
+        const float hw = s_hw[t];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[e] = Act<T>::round(__fmul_rn(x[e], hw));
+      }
+      const float ele = a.eta != 0.f ? s_le[t] : 0.f;
+#pragma unroll
+      for (int p = 0; p < 4; ++p)
+        y[i][p] = mul2(F2(x[2 * p], x[2 * p + 1]), exp_pair(sub2(sub2(gl[p], F2(gv[2 * p], gv[2 * p + 1])), F2(ele, ele))));
     }
-    const T* qp = reinterpret_cast<const T*>(a.q);
-    const T* kp = reinterpret_cast<const T*>(a.k);
-    for (int tg = warp * G + grp; tg < C / 4; tg += 8 * G) {
-      uint32_t kwp[8];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) kwp[j] = 0u;
-      // the eight row loads of the group are in flight before the first is used
-      uint4 rq[4], rk[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const size_t row = (((size_t)b * a.T + (size_t)c * C + 4 * tg + i) * a.H + h) * K + 8 * r;
-        rq[i] = __ldg(reinterpret_cast<const uint4*>(qp + row));
-        rk[i] = __ldg(reinterpret_cast<const uint4*>(kp + row));
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int t = 4 * tg + i;
-        float x[8], gv[8];
-        int cd[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) gv[j] = s_gc[t * LD + 8 * r + j];
-        Act<T>::unpack8(rq[i], x);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) cd[j] = q8(__fmul_rn(__fmul_rn(x[j], __expf(gv[j])), a.scale), inv_sq, a.qmax);
-        *reinterpret_cast<uint2*>(a.qq + (tile * C + t) * K + 8 * r) =
-            make_uint2(pack4(cd[0], cd[1], cd[2], cd[3]), pack4(cd[4], cd[5], cd[6], cd[7]));
-        Act<T>::unpack8(rk[i], x);
-        if (DELTA && e_hw != 0.f) {
-          const float hw = s_hw[t];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) x[j] = Act<T>::round(__fmul_rn(x[j], hw));
-        }
-        const float ele = a.eta * s_le[t];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float w = __expf(__fsub_rn(__fsub_rn(gl[j], gv[j]), ele));
-          kwp[j] |= ((uint32_t)q8(__fmul_rn(x[j], w), inv_kw[j], a.qmax) & 0xffu) << (8 * i);
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < 8; ++j) s_kw[8 * r + j][tg] = kwp[j];
+    for (int p = 0; p < 4; ++p) {
+      const F2 w[4] = {y[0][p], y[1][p], y[2][p], y[3][p]};
+      put(a.kwT + (tile * K + n0 + 2 * p) * C + t0, w, F2(s_ikw[n0 + 2 * p], s_ikw[n0 + 2 * p + 1]));
     }
   }
-  if (!DELTA) {
-    constexpr int LPR = V / 8, G = 32 / LPR;
-    const int r = lane % LPR, grp = lane / LPR;
-    float inv_vl[8], inv_vw[8];
+  if (const int u = (warp + NQK) & 7; !DELTA && u < V / 16) {  // K = 64: the warps without a q / k item first
+    const int t0 = 32 * (u & 1) + lt, n0 = 32 * (u >> 1) + ln;
+    uint4 rv[4];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      inv_vl[j] = 1.0f / a.svl[h * V + 8 * r + j];
-      inv_vw[j] = 1.0f / a.svw[h * V + 8 * r + j];
+    for (int i = 0; i < 4; ++i) rv[i] = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(a.v) + (tok0 + (size_t)(t0 + i) * a.H) * V + n0));
+    float x[4][8], fv[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      Act<T>::unpack8(rv[i], x[i]);
+      fv[i] = a.eta != 0.f ? expf(s_le[t0 + i]) : 1.f;
     }
-    const T* vp = reinterpret_cast<const T*>(a.v);
-    for (int tg = warp * G + grp; tg < C / 4; tg += 8 * G) {
-      uint32_t vlp[8], vwp[8];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) vlp[j] = vwp[j] = 0u;
-      uint4 rv[4];  // the four row loads of the group are in flight before the first is used
+    for (int p = 0; p < 4; ++p) {
+      F2 w[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-        rv[i] = __ldg(reinterpret_cast<const uint4*>(vp + (((size_t)b * a.T + (size_t)c * C + 4 * tg + i) * a.H + h) * V + 8 * r));
+      for (int i = 0; i < 4; ++i) w[i] = F2(x[i][2 * p], x[i][2 * p + 1]);
+      put(a.vlT + (tile * V + n0 + 2 * p) * C + t0, w, F2(s_ivl[n0 + 2 * p], s_ivl[n0 + 2 * p + 1]));
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int t = 4 * tg + i;
-        float x[8];
-        Act<T>::unpack8(rv[i], x);
-        const float fv = expf(a.eta * s_le[t]);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          vlp[j] |= ((uint32_t)q8(x[j], inv_vl[j], a.qmax) & 0xffu) << (8 * i);
-          vwp[j] |= ((uint32_t)q8(__fmul_rn(x[j], fv), inv_vw[j], a.qmax) & 0xffu) << (8 * i);
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        s_vl[8 * r + j][tg] = vlp[j];
-        s_vw[8 * r + j][tg] = vwp[j];
-      }
-    }
-  }
-  __syncthreads();
-  uint32_t* kw_out = reinterpret_cast<uint32_t*>(a.kwT + tile * (size_t)(K * C));
-  for (int i = tid; i < K * 16; i += 256) kw_out[i] = s_kw[i >> 4][i & 15];
-  if (!DELTA) {
-    uint32_t* vl_out = reinterpret_cast<uint32_t*>(a.vlT + tile * (size_t)(V * C));
-    uint32_t* vw_out = reinterpret_cast<uint32_t*>(a.vwT + tile * (size_t)(V * C));
-    for (int i = tid; i < V * 16; i += 256) {
-      vl_out[i] = s_vl[i >> 4][i & 15];
-      vw_out[i] = s_vw[i >> 4][i & 15];
+      for (int i = 0; i < 4; ++i) w[i] = mul2(w[i], F2(fv[i], fv[i]));
+      put(a.vwT + (tile * V + n0 + 2 * p) * C + t0, w, F2(s_ivw[n0 + 2 * p], s_ivw[n0 + 2 * p + 1]));
     }
   }
 }
@@ -754,7 +749,7 @@ template <typename T, int K, int V>
 static int run_diag_T(const lq_zoo_problem* p, const DiagArgs& a, bool delta, int stage, cudaStream_t st) {
   dim3 grid(a.NT, p->B * p->H);
   if (stage == 0) {
-    const size_t smem = sizeof(float) * (64 * (K + 4) + 128) + sizeof(uint32_t) * 17 * (K + 2 * V);
+    constexpr size_t smem = diag_rows_smem<K, V>();
     if (delta) return launch_big_smem(zoo_diag_rows_kernel<T, K, V, true>, "zoo_diag_rows_kernel", grid, smem, a, st);
     return launch_big_smem(zoo_diag_rows_kernel<T, K, V, false>, "zoo_diag_rows_kernel", grid, smem, a, st);
   }
