@@ -1,14 +1,16 @@
 // Linear-family prologue, tensor-core version (used when no D_QK rescale is requested).
 //
 // Same outputs as zoo_prologue_linear_kernel, different machine mapping:
-//  * the signed Walsh-Hadamard rotation is an MMA of the activation rows (bf16/fp16, exact operands) with the +-1
-//    Sylvester matrix (exact in either dtype), fp32 accumulate. A warp owns 16 tokens; its A fragments are eight
-//    128-bit loads issued up front, the B fragments come from a per-CTA table in shared memory (one 64-bit load each);
-//  * MMA rows are mapped to tokens (2g, 2g+1) and MMA columns are permuted so that a thread ends up with eight
-//    consecutive channels of two consecutive tokens: row-major code tiles leave as 64-bit stores, transposed tiles
-//    as 16-bit stores into the shared-memory transposer;
+//  * a warp owns 16 tokens of q or of k. The transform is split over the channel bits: bits 0, 1, 3, 4 are the sixteen slots of
+//    an m16n8k16 product with the +-1 matrix (exact operands, fp32 accumulate), the others a butterfly between a lane's own
+//    registers;
+//  * MMA rows are mapped to tokens (2g, 2g+1) and a lane holds eight consecutive channels of both: row-major code tiles leave
+//    as 64-bit stores, transposed tiles as 16-bit stores into the shared-memory transposer;
 //  * the code rule keeps its arithmetic (fp32 x*inv, clamp, +-0.5, truncate) but saturates the upper side in the
-//    pack instruction, and a CTA walks several chunks so the table and the scale staging are amortised.
+//    pack instruction, two values to an instruction where there is one, and a CTA walks several chunks so the scale staging is
+//    amortised.
+// Bound by instruction issue. With the whole rotation as products (eight times as many of them) and codes one at a time, 64 (b, h) x
+// 64 chunks at K = V = 128 took 113 us; this form takes 102.
 // Arithmetic and references as in lq_zoo_prologue.cu.
 #include <type_traits>
 
@@ -16,50 +18,25 @@
 
 namespace lq {
 
-__device__ __forceinline__ uint32_t pack_sat2(int hi, int lo, uint32_t upper) { return pack_sat_s8x2(hi, lo, upper); }
-// code before the final saturation: with Q127 the upper clamp is left to the saturating pack
-template <bool Q127>
-__device__ __forceinline__ int code32(float x, float inv, float qmax) {
-  float y = __fmul_rn(x, inv);
-  y = fmaxf(y, -qmax);
-  if (!Q127) y = fminf(y, qmax);
-  return __float2int_rz(__fadd_rn(y, copysignf(0.5f, y)));
+template <typename T>
+__device__ __forceinline__ void unpack_pairs(const uint4& r, F2 (&x)[4]) {
+  float f[8];
+  Act<T>::unpack8(r, f);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) x[i] = F2(f[2 * i], f[2 * i + 1]);
 }
-__device__ __forceinline__ uint32_t pack4s(const int (&c)[8], int o) {
-  return pack_sat2(c[o + 1], c[o], pack_sat2(c[o + 3], c[o + 2], 0u));
-}
-
-// Hadamard product step: the B fragment arrives as one 64-bit register pair (the MMA wants its two B registers adjacent;
-// separate 32-bit operands chosen per step made the compiler copy them into place before every instruction), and the
-// first step of a chain takes C = 0 instead of zeroed accumulators.
-template <typename T, bool FIRST>
-__device__ __forceinline__ void mma_had(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint64_t bp) {
-  if (std::is_same<T, __half>::value) {
-    if (FIRST)
-      asm volatile("{\n.reg .b32 b0, b1;\nmov.b64 {b0, b1}, %8;\n"
-                   "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {b0,b1}, {%9,%9,%9,%9};\n}\n"
-                   : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "l"(bp), "f"(0.f));
-    else
-      asm volatile("{\n.reg .b32 b0, b1;\nmov.b64 {b0, b1}, %8;\n"
-                   "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {b0,b1}, {%0,%1,%2,%3};\n}\n"
-                   : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "l"(bp));
-  } else {
-    if (FIRST)
-      asm volatile("{\n.reg .b32 b0, b1;\nmov.b64 {b0, b1}, %8;\n"
-                   "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {b0,b1}, {%9,%9,%9,%9};\n}\n"
-                   : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "l"(bp), "f"(0.f));
-    else
-      asm volatile("{\n.reg .b32 b0, b1;\nmov.b64 {b0, b1}, %8;\n"
-                   "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {b0,b1}, {%0,%1,%2,%3};\n}\n"
-                   : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "l"(bp));
-  }
+// codes of channels n, n + 1 of token t (low half) and t + 1 into rows n, n + 1 of a transposer (17 words a row)
+__device__ __forceinline__ void put_pair(uint32_t* row, int t, uint32_t codes) {
+  const uint32_t w = __byte_perm(codes, 0u, 0x3120);
+  reinterpret_cast<uint16_t*>(row)[t >> 1] = (uint16_t)w;
+  reinterpret_cast<uint16_t*>(row + 17)[t >> 1] = (uint16_t)(w >> 16);
 }
 
 template <typename T, int K, int V, bool Q127>
 __global__ void __launch_bounds__(256, 2) zoo_prologue_linear_mma_kernel(PrologueArgs a, int n_tiles) {
   pdl_enter();
   constexpr int C = kChunk;
-  constexpr int KS = K / 16;
+  constexpr int M = K / 32, NVQ = V == 128 ? 3 : 2;
   constexpr int RAW_Q = C * K * 2, RAW_V = C * V * 2;
   extern __shared__ __align__(16) uint8_t smem_raw[];
   uint32_t(*s_kw)[17] = reinterpret_cast<uint32_t(*)[17]>(smem_raw);
@@ -82,20 +59,12 @@ __global__ void __launch_bounds__(256, 2) zoo_prologue_linear_mma_kernel(Prologu
   const T* kp = reinterpret_cast<const T*>(a.k);
   const T* vp = reinterpret_cast<const T*>(a.v);
 
-  // B fragments of the Sylvester matrix without a table. With input channel c = 32u + 8j + 4h + 2hi + e (k-step
-  // s = 2u + h, register hi, half e) and output channel n = 32(nt>>2) + 8(g>>1) + 2(nt&3) + (g&1), the sign
-  // (-1)^popc(c & n) splits into a per-lane part (e*g0 ^ j0*g1 ^ j1*g2), a part hi*(nt&1), and a part that depends
-  // on (s, nt) only. The last two are compile-time choices between the base register and its negation.
-  uint32_t hb0, hb0n;
-  {
+  // B fragment of the +-1 matrix on the sixteen slots: (-1)^popc(s & n) for slots s = 2j, 2j + 1 and column n = g
+  const uint32_t had = [&]() {
     const uint32_t one = std::is_same<T, __half>::value ? 0x3C00u : 0x3F80u;
-    const uint32_t L = ((j & 1) & ((g >> 1) & 1)) ^ (((j >> 1) & 1) & ((g >> 2) & 1));
-    hb0 = (one | (L << 15)) | ((one | ((L ^ (g & 1)) << 15)) << 16);
-    hb0n = hb0 ^ 0x80008000u;
-  }
-  // the four (b0, b1) sign combinations as register pairs, index 2*neg(b0) + neg(b1)
-  const uint64_t hbp[4] = {(uint64_t)hb0 | ((uint64_t)hb0 << 32), (uint64_t)hb0 | ((uint64_t)hb0n << 32),
-                           (uint64_t)hb0n | ((uint64_t)hb0 << 32), (uint64_t)hb0n | ((uint64_t)hb0n << 32)};
+    const uint32_t s0 = one | ((__popc((2 * j) & g) & 1) << 15), s1 = one | ((__popc((2 * j + 1) & g) & 1) << 15);
+    return s0 | (s1 << 16);
+  }();
 
   // persistent CTAs: tile t = (batch, chunk, head) with the head fastest, strided by the grid: every CTA gets the same
   // number of tiles to within one, and the CTAs in flight read all heads of the same tokens (adjacent in memory)
@@ -206,111 +175,129 @@ __global__ void __launch_bounds__(256, 2) zoo_prologue_linear_mma_kernel(Prologu
     }
     const bool use_g = a.g != nullptr;
     const float da = glast - gca, db = glast - gcb;
-    // ---------------------------------------------------------------- q then k: a warp owns an m-tile and one half
-    // of the output channels of both operands (equal work in every warp)
-#pragma unroll
-    for (int op = 0; op < 2; ++op) {
-      const bool is_q = op == 0;
-      const int half = warp >> 2;
-      // the channel half of the warp flips the sign of the steps whose input channels carry that bit: applied to the
-      // A fragments of those steps (an XOR on their way into the MMA's register quad)
-      const uint32_t sflip = half ? 0x80008000u : 0u;
+    // ---------------------------------------------------------------- warps 0 - 3: the rows of k; 4 - 7: of q
+    {
+      const bool is_q = warp >= 4;
       const uint8_t* src = s_qk + buf * 2 * RAW_Q + (is_q ? 0 : RAW_Q);
-      uint4 ra[K / 32], rb[K / 32];
+      F2 y[M][2][2][2];  // [m][eh][token a, b][channel pair]: channel 32 m + 8 j + 4 eh + 2 pair + (0, 1)
 #pragma unroll
-      for (int u = 0; u < K / 32; ++u) {
-        ra[u] = *reinterpret_cast<const uint4*>(src + ta * (K * 2) + (((4 * u + j) ^ swz) << 4));
-        rb[u] = *reinterpret_cast<const uint4*>(src + tb * (K * 2) + (((4 * u + j) ^ swz) << 4));
-      }
-      const float fka = use_g ? expf((1.0f - a.eta) * da) : 1.0f, fkb = use_g ? expf((1.0f - a.eta) * db) : 1.0f;
-      int8_t* rowmajor = (is_q ? a.qq : a.kl) + (tile * C) * K;
-#pragma unroll
-      for (int ngl = 0; ngl < K / 64; ++ngl) {
-        const int ng = half * (K / 64) + ngl;
-        float va[8], vb[8];
+      for (int m = 0; m < M; ++m) {
+        const uint4 ra = *reinterpret_cast<const uint4*>(src + ta * (K * 2) + (((4 * m + j) ^ swz) << 4));
+        const uint4 rb = *reinterpret_cast<const uint4*>(src + tb * (K * 2) + (((4 * m + j) ^ swz) << 4));
         if (rot) {
-          float acc[4][4];
 #pragma unroll
-          for (int s = 0; s < KS; ++s) {
-            const uint32_t* wa = reinterpret_cast<const uint32_t*>(&ra[s >> 1]);
-            const uint32_t* wb = reinterpret_cast<const uint32_t*>(&rb[s >> 1]);
-            const bool dep = K == 128 ? ((s >> 2) & 1) : ((s >> 1) & 1);
-            const uint32_t fl = dep ? sflip : 0u;
-            const uint32_t a0 = wa[2 * (s & 1)] ^ fl, a2 = wa[2 * (s & 1) + 1] ^ fl, a1 = wb[2 * (s & 1)] ^ fl, a3 = wb[2 * (s & 1) + 1] ^ fl;
+          for (int eh = 0; eh < 2; ++eh) {
+            const uint32_t a0 = eh ? ra.z : ra.x, a2 = eh ? ra.w : ra.y, a1 = eh ? rb.z : rb.x, a3 = eh ? rb.w : rb.y;
+            float d0[4] = {0.f, 0.f, 0.f, 0.f}, d1[4] = {0.f, 0.f, 0.f, 0.f};
+            if (std::is_same<T, __half>::value) {
+              mma_f16(d0, a0, a1, a2, a3, had, had);
+              mma_f16(d1, a0, a1, a2, a3, had, had ^ 0x80008000u);
+            } else {
+              mma_bf16(d0, a0, a1, a2, a3, had, had);
+              mma_bf16(d1, a0, a1, a2, a3, had, had ^ 0x80008000u);
+            }
 #pragma unroll
-            for (int n4 = 0; n4 < 4; ++n4) {
-              // output n-tile nt = 4*ng + n4; its bits above n4 are ngl (compile time) and the warp's channel half
-              const int Uc = ((s & 1) & ((n4 >> 1) & 1)) ^ (K == 128 ? (((s >> 1) & 1) & (ngl & 1)) : 0);
-              if (s == 0) mma_had<T, true>(acc[n4], a0, a1, a2, a3, hbp[2 * Uc + (Uc ^ (n4 & 1))]);
-              else mma_had<T, false>(acc[n4], a0, a1, a2, a3, hbp[2 * Uc + (Uc ^ (n4 & 1))]);
+            for (int r = 0; r < 2; ++r) {
+              y[m][eh][r][0] = F2(d0[2 * r], d0[2 * r + 1]);
+              y[m][eh][r][1] = F2(d1[2 * r], d1[2 * r + 1]);
             }
           }
-          const float4 s0 = *reinterpret_cast<const float4*>(s_sgn + 32 * ng + 8 * j);
-          const float4 s1 = *reinterpret_cast<const float4*>(s_sgn + 32 * ng + 8 * j + 4);
-          const float sg[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+        } else {
+          F2 xa[4], xb[4];
+          unpack_pairs<T>(ra, xa);
+          unpack_pairs<T>(rb, xb);
 #pragma unroll
-          for (int n4 = 0; n4 < 4; ++n4)
+          for (int i = 0; i < 4; ++i) {
+            y[m][i >> 1][0][i & 1] = xa[i];
+            y[m][i >> 1][1][i & 1] = xb[i];
+          }
+        }
+      }
+      if (rot) {  // the remaining channel bits: 2 (eh), 5 and 6 (m)
+        const F2 neg(-1.f, -1.f);
+        auto fly = [&](F2& p, F2& q) {
+          const F2 sum = add2(p, q);
+          q = fma2(q, neg, p);
+          p = sum;
+        };
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-              va[2 * n4 + e] = Act<T>::round(__fmul_rn(acc[n4][e], sg[2 * n4 + e]));
-              vb[2 * n4 + e] = Act<T>::round(__fmul_rn(acc[n4][2 + e], sg[2 * n4 + e]));
+        for (int r = 0; r < 2; ++r)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+#pragma unroll
+            for (int m = 0; m < M; ++m) fly(y[m][0][r][e], y[m][1][r][e]);
+#pragma unroll
+            for (int eh = 0; eh < 2; ++eh) {
+#pragma unroll
+              for (int m = 0; m < M; m += 2) fly(y[m][eh][r][e], y[m + 1][eh][r][e]);
+              if (M == 4) {
+                fly(y[0][eh][r][e], y[2 % M][eh][r][e]);
+                fly(y[1][eh][r][e], y[3 % M][eh][r][e]);
+              }
             }
-        } else {
-          Act<T>::unpack8(half ? ra[K / 64 + ngl] : ra[ngl], va);
-          Act<T>::unpack8(half ? rb[K / 64 + ngl] : rb[ngl], vb);
-        }
-        const int cb = 32 * ng + 8 * j;
-        int ca[8], cc[8];
-        if (is_q) {
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            ca[i] = code32<Q127>(__fmul_rn(va[i], a.scale), inv_sq, a.qmax);
-            cc[i] = code32<Q127>(__fmul_rn(vb[i], a.scale), inv_sq, a.qmax);
           }
-        } else {
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            ca[i] = code32<Q127>(va[i], inv_sk, a.qmax);
-            cc[i] = code32<Q127>(vb[i], inv_sk, a.qmax);
+        for (int m = 0; m < M; ++m)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float2 sg = *reinterpret_cast<const float2*>(s_sgn + 32 * m + 8 * j + 2 * i);
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+              float x0, x1;
+              mul2(y[m][i >> 1][r][i & 1], F2(sg.x, sg.y)).get(x0, x1);
+              const uint32_t w = Act<T>::pack2(x0, x1);
+              y[m][i >> 1][r][i & 1] = F2(Act<T>::get(w, 0), Act<T>::get(w, 1));
+            }
           }
-        }
-        const int pa_ = is_q ? ta : kl_row_of_token(ta), pb_ = is_q ? tb : kl_row_of_token(tb);
-        *reinterpret_cast<uint2*>(rowmajor + (size_t)pa_ * K + cb) = make_uint2(pack4s(ca, 0), pack4s(ca, 4));
-        *reinterpret_cast<uint2*>(rowmajor + (size_t)pb_ * K + cb) = make_uint2(pack4s(cc, 0), pack4s(cc, 4));
-        if (!is_q) {
-          const float4 i0 = *reinterpret_cast<const float4*>(s_ikw + cb);
-          const float4 i1 = *reinterpret_cast<const float4*>(s_ikw + cb + 4);
-          const float ik[8] = {i0.x, i0.y, i0.z, i0.w, i1.x, i1.y, i1.z, i1.w};
+      }
+      if (is_q) {
+        const F2 sc(a.scale, a.scale), inv(inv_sq, inv_sq);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int wa_ = code32<Q127>(__fmul_rn(va[i], fka), ik[i], a.qmax);
-            const int wb_ = code32<Q127>(__fmul_rn(vb[i], fkb), ik[i], a.qmax);
-            reinterpret_cast<uint16_t*>(&s_kw[cb + i][0])[ta >> 1] = (uint16_t)pack_sat2(wb_, wa_, 0u);
+        for (int m = 0; m < M; ++m)
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            uint32_t cd[2];
+#pragma unroll
+            for (int eh = 0; eh < 2; ++eh) cd[eh] = codes4<Q127>(mul2(y[m][eh][r][0], sc), mul2(y[m][eh][r][1], sc), inv, a.qmax);
+            *reinterpret_cast<uint2*>(a.qq + (tile * C + ta + r) * K + 32 * m + 8 * j) = make_uint2(cd[0], cd[1]);
+          }
+      } else {
+        const float fka = use_g ? expf((1.0f - a.eta) * da) : 1.0f, fkb = use_g ? expf((1.0f - a.eta) * db) : 1.0f;
+        const F2 inv(inv_sk, inv_sk), fa(fka, fka), fb(fkb, fkb);
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            uint32_t cd[2];
+#pragma unroll
+            for (int eh = 0; eh < 2; ++eh) cd[eh] = codes4<Q127>(y[m][eh][r][0], y[m][eh][r][1], inv, a.qmax);
+            *reinterpret_cast<uint2*>(a.kl + (tile * C + kl_row_of_token(ta + r)) * K + 32 * m + 8 * j) = make_uint2(cd[0], cd[1]);
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int cb = 32 * m + 8 * j + 2 * i;
+            const float2 ik = *reinterpret_cast<const float2*>(s_ikw + cb);
+            put_pair(&s_kw[cb][0], ta, codes4<Q127>(mul2(y[m][i >> 1][0][i & 1], fa), mul2(y[m][i >> 1][1][i & 1], fb), F2(ik.x, ik.y), a.qmax));
           }
         }
       }
     }
-    // ---------------------------------------------------------------- v: eight warps, m-tile x channel half
+    // ---------------------------------------------------------------- v: three quarters of the channels by the q warps, which
+    // have one code tensor to make where the k warps have two
     if (!a.skip_v) {
-      const int half = warp >> 2;
       const float fva = use_g ? expf(a.eta * da) : 1.0f, fvb = use_g ? expf(a.eta * db) : 1.0f;
+      const int u0 = warp >= 4 ? 0 : NVQ, u1 = warp >= 4 ? NVQ : V / 32;
+#pragma unroll 1
+      for (int uu = u0; uu < u1; ++uu) {
+        const int cb = 32 * uu + 8 * j;
+        F2 va[4], vb[4];
+        unpack_pairs<T>(*reinterpret_cast<const uint4*>(s_v + ta * (V * 2) + (((cb >> 3) ^ swz) << 4)), va);
+        unpack_pairs<T>(*reinterpret_cast<const uint4*>(s_v + tb * (V * 2) + (((cb >> 3) ^ swz) << 4)), vb);
 #pragma unroll
-      for (int uu = 0; uu < V / 64; ++uu) {
-        const int cb = 32 * (half * (V / 64) + uu) + 8 * j;
-        float va[8], vb[8];
-        Act<T>::unpack8(*reinterpret_cast<const uint4*>(s_v + ta * (V * 2) + (((cb >> 3) ^ swz) << 4)), va);
-        Act<T>::unpack8(*reinterpret_cast<const uint4*>(s_v + tb * (V * 2) + (((cb >> 3) ^ swz) << 4)), vb);
-        const float4 l0 = *reinterpret_cast<const float4*>(s_ivl + cb), l1 = *reinterpret_cast<const float4*>(s_ivl + cb + 4);
-        const float4 w0 = *reinterpret_cast<const float4*>(s_ivw + cb), w1 = *reinterpret_cast<const float4*>(s_ivw + cb + 4);
-        const float il[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
-        const float iw[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int la = code32<Q127>(va[i], il[i], a.qmax), lb = code32<Q127>(vb[i], il[i], a.qmax);
-          const int wa_ = code32<Q127>(__fmul_rn(va[i], fva), iw[i], a.qmax);
-          const int wb_ = code32<Q127>(__fmul_rn(vb[i], fvb), iw[i], a.qmax);
-          reinterpret_cast<uint16_t*>(&s_vl[cb + i][0])[ta >> 1] = (uint16_t)pack_sat2(lb, la, 0u);
-          reinterpret_cast<uint16_t*>(&s_vw[cb + i][0])[ta >> 1] = (uint16_t)pack_sat2(wb_, wa_, 0u);
+        for (int i = 0; i < 4; ++i) {
+          const float2 il = *reinterpret_cast<const float2*>(s_ivl + cb + 2 * i), iw = *reinterpret_cast<const float2*>(s_ivw + cb + 2 * i);
+          put_pair(&s_vl[cb + 2 * i][0], ta, codes4<Q127>(va[i], vb[i], F2(il.x, il.y), a.qmax));
+          put_pair(&s_vw[cb + 2 * i][0], ta, codes4<Q127>(mul2(va[i], F2(fva, fva)), mul2(vb[i], F2(fvb, fvb)), F2(iw.x, iw.y), a.qmax));
         }
       }
     }
