@@ -81,7 +81,7 @@ static size_t carve(const lq_zoo_problem* p, int delta, void* ws, lq_zoo_workspa
   return (cv.off + 255) & ~size_t(255);
 }
 
-int run_prologue_linear(const lq_zoo_problem* p, const lq_zoo_workspace* ws, int skip_v, cudaStream_t st);
+int run_prologue_linear(const lq_zoo_problem* p, const lq_zoo_workspace* ws, cudaStream_t st);
 int run_state_linear(const lq_zoo_problem* p, const lq_zoo_workspace* ws, cudaStream_t st);
 int run_output_scalar(const lq_zoo_problem* p, const lq_zoo_workspace* ws, const float* s_local_value, cudaStream_t st);
 int run_prologue_delta(const lq_zoo_problem* p, const lq_zoo_workspace* ws, cudaStream_t st);
@@ -129,7 +129,7 @@ extern "C" int lq_simple_gla_fwd(const lq_zoo_problem* p, void* workspace, size_
   if (int e = lq_zoo_carve_workspace(p, 0, workspace, workspace_bytes, &ws)) return e;
   cudaStream_t st = (cudaStream_t)stream;
   if (p->status == nullptr) cudaMemsetAsync(ws.status, 0, sizeof(int), st);
-  if (int e = lq::run_prologue_linear(p, &ws, 0, st)) return e;
+  if (int e = lq::run_prologue_linear(p, &ws, st)) return e;
   if (int e = lq::run_state_linear(p, &ws, st)) return e;
   return lq::run_output_scalar(p, &ws, p->svl, st);
 }

@@ -47,9 +47,9 @@ __global__ void __launch_bounds__(256) zoo_prologue_linear_kernel(PrologueArgs a
   }
   __syncthreads();
 
-  prologue_qk_rows<T, K>(a, b, c, h, tile, s_fk, nullptr, nullptr, 0, s_kw);
+  prologue_qk_rows<T, K>(a, b, c, h, tile, s_fk, s_kw);
   // ------------------------------------------------------------------ v rows (V channels)
-  if (!a.skip_v) {
+  {
     constexpr int LPR = V / 8, G = 32 / LPR;
     const int r = lane % LPR, grp = lane / LPR;
     float inv_vl[8], inv_vw[8];
@@ -87,13 +87,11 @@ __global__ void __launch_bounds__(256) zoo_prologue_linear_kernel(PrologueArgs a
   // ------------------------------------------------------------------ transposed tiles out, coalesced
   uint32_t* kw_out = reinterpret_cast<uint32_t*>(a.kwT + tile * (size_t)(K * C));
   for (int i = tid; i < K * 16; i += 256) kw_out[i] = s_kw[i >> 4][i & 15];
-  if (!a.skip_v) {
-    uint32_t* vl_out = reinterpret_cast<uint32_t*>(a.vlT + tile * (size_t)(V * C));
-    uint32_t* vw_out = reinterpret_cast<uint32_t*>(a.vwT + tile * (size_t)(V * C));
-    for (int i = tid; i < V * 16; i += 256) {
-      vl_out[i] = s_vl[i >> 4][i & 15];
-      vw_out[i] = s_vw[i >> 4][i & 15];
-    }
+  uint32_t* vl_out = reinterpret_cast<uint32_t*>(a.vlT + tile * (size_t)(V * C));
+  uint32_t* vw_out = reinterpret_cast<uint32_t*>(a.vwT + tile * (size_t)(V * C));
+  for (int i = tid; i < V * 16; i += 256) {
+    vl_out[i] = s_vl[i >> 4][i & 15];
+    vw_out[i] = s_vw[i >> 4][i & 15];
   }
 }
 
@@ -115,15 +113,14 @@ void fill_prologue_args(const lq_zoo_problem* p, const lq_zoo_workspace* ws, Pro
   a.sq = p->sq; a.sk = p->sk; a.skw = p->skw; a.svl = p->svl; a.svw = p->svw;
   a.qq = ws->qq; a.kl = ws->kl; a.kwT = ws->kwT; a.vlT = ws->vlT; a.vwT = ws->vwT; a.gc = ws->gc;
   a.T = p->T; a.H = p->H; a.NT = p->T / p->chunk;
-  a.scale = p->scale; a.eta = p->eta; a.qmax = p->qmax; a.skip_v = 0;
+  a.scale = p->scale; a.eta = p->eta; a.qmax = p->qmax;
 }
 
 int run_prologue_linear_mma(const lq_zoo_problem* p, const PrologueArgs& a, cudaStream_t st);
 
-int run_prologue_linear(const lq_zoo_problem* p, const lq_zoo_workspace* ws, int skip_v, cudaStream_t st) {
+int run_prologue_linear(const lq_zoo_problem* p, const lq_zoo_workspace* ws, cudaStream_t st) {
   PrologueArgs a;
   fill_prologue_args(p, ws, a);
-  a.skip_v = skip_v;
   // the tensor-core rotation needs operands that are exact in the activation dtype: with a D_QK rescale ahead of the
   // rotation the fp32 butterfly kernel below is used instead
   if (p->dqk == nullptr) return run_prologue_linear_mma(p, a, st);
@@ -138,5 +135,5 @@ extern "C" int lq_zoo_prologue_linear(const lq_zoo_problem* p, const lq_zoo_work
   if (int e = lq::validate_zoo_problem(p, false, false)) return e;
   if (!ws) return lq::fail(LQ_ERR_NULL, "prologue: workspace descriptor is null");
   if (p->decay == LQ_DECAY_DIAGONAL) return lq::fail(LQ_ERR_UNSUPPORTED, "prologue_linear: diagonal decay uses lq_zoo_prologue_diag");
-  return lq::run_prologue_linear(p, ws, 0, (cudaStream_t)stream);
+  return lq::run_prologue_linear(p, ws, (cudaStream_t)stream);
 }

@@ -90,7 +90,6 @@ __global__ void __launch_bounds__(256, 2) zoo_prologue_linear_mma_kernel(Prologu
     }
   };
   auto stage_v = [&](int h, int c, int b) {
-    if (a.skip_v) return;
     const T* sv = vp + (((size_t)b * a.T + (size_t)c * C + rv0) * a.H + h) * V + 8 * chv0;
     const size_t step = (size_t)RPIV * a.H * V;
 #pragma unroll
@@ -284,7 +283,7 @@ __global__ void __launch_bounds__(256, 2) zoo_prologue_linear_mma_kernel(Prologu
     }
     // ---------------------------------------------------------------- v: three quarters of the channels by the q warps, which
     // have one code tensor to make where the k warps have two
-    if (!a.skip_v) {
+    {
       const float fva = use_g ? expf(a.eta * da) : 1.0f, fvb = use_g ? expf(a.eta * db) : 1.0f;
       const int u0 = warp >= 4 ? 0 : NVQ, u1 = warp >= 4 ? NVQ : V / 32;
 #pragma unroll 1
@@ -308,13 +307,11 @@ __global__ void __launch_bounds__(256, 2) zoo_prologue_linear_mma_kernel(Prologu
     }
     uint32_t* kw_out = reinterpret_cast<uint32_t*>(a.kwT + tile * (size_t)(K * C));
     for (int i = tid; i < K * 16; i += 256) kw_out[i] = s_kw[i >> 4][i & 15];
-    if (!a.skip_v) {
-      uint32_t* vl_out = reinterpret_cast<uint32_t*>(a.vlT + tile * (size_t)(V * C));
-      uint32_t* vw_out = reinterpret_cast<uint32_t*>(a.vwT + tile * (size_t)(V * C));
-      for (int i = tid; i < V * 16; i += 256) {
-        vl_out[i] = s_vl[i >> 4][i & 15];
-        vw_out[i] = s_vw[i >> 4][i & 15];
-      }
+    uint32_t* vl_out = reinterpret_cast<uint32_t*>(a.vlT + tile * (size_t)(V * C));
+    uint32_t* vw_out = reinterpret_cast<uint32_t*>(a.vwT + tile * (size_t)(V * C));
+    for (int i = tid; i < V * 16; i += 256) {
+      vl_out[i] = s_vl[i >> 4][i & 15];
+      vw_out[i] = s_vw[i >> 4][i & 15];
     }
   }
 }

@@ -13,7 +13,6 @@ struct PrologueArgs {
   float* gc;
   int T, H, NT;
   float scale, eta, qmax;
-  int skip_v;  // delta family: the value operand is produced by the WY kernel instead
 };
 
 constexpr int kChunk = 64;
@@ -41,13 +40,9 @@ __device__ __forceinline__ void chunk_decay_scan(const float* g, int b, int c, i
 // q and k rows of one chunk. Lane-in-row r of LPR = K/8 lanes holds channels 8r..8r+7; a group of LPR lanes walks
 // four consecutive tokens so the transposed k_write tile can be packed four tokens to a word.
 //   s_fk   [C]    key-side write gate Omega^(1-eta)
-//   s_hw   [C]    optional per-token factor of the readout/write key (delta rule: beta^((1-sigma)tau)); the
-//                 product is rounded to the activation dtype (reference.py:211)
-//   s_kf   [C,LDK] optional fp32 copy of the rotated, rounded key (before s_hw) for the WY products
 template <typename T, int K>
 __device__ __forceinline__ void prologue_qk_rows(const PrologueArgs& a, int b, int c, int h, size_t tile,
-                                                 const float* s_fk, const float* s_hw, float* s_kf, int LDK,
-                                                 uint32_t (*s_kw)[17]) {
+                                                 const float* s_fk, uint32_t (*s_kw)[17]) {
   constexpr int C = kChunk;
   constexpr int LPR = K / 8, G = 32 / LPR;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -109,15 +104,6 @@ __device__ __forceinline__ void prologue_qk_rows(const PrologueArgs& a, int b, i
         fwht8<LPR>(x, r);
 #pragma unroll
         for (int j = 0; j < 8; ++j) x[j] = Act<T>::round(__fmul_rn(x[j], sgn[j]));
-      }
-      if (s_kf != nullptr) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) s_kf[t * LDK + 8 * r + j] = x[j];
-      }
-      if (s_hw != nullptr) {
-        const float hw = s_hw[t];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) x[j] = Act<T>::round(__fmul_rn(x[j], hw));
       }
 #pragma unroll
       for (int j = 0; j < 8; ++j) cd[j] = q8(x[j], inv_sk, a.qmax);
