@@ -325,22 +325,25 @@ __global__ void __launch_bounds__(256) zoo_diag_amat_kernel(DiagArgs a) {
           for (int p = 0; p < 4; ++p)
             split3_pair(mul2(code_pair(F2(x[2 * p], x[2 * p + 1]), fk, a.qmax), exp_pair(mul2(e1[p], F2(-1.f, -1.f)))), kh[r][p], km[r][p], kl[r][p]);
         }
+        // The tensor core cuts off what falls below the last bit of its accumulator: the products go small to big into a fresh
+        // one per 32 channels (only the two biggest meet a full sum), and the passes are added in fp32.
+        float d[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+        auto mma = [&](const uint32_t (&qa)[2][4], const uint32_t (&kb)[2][4]) {
 #pragma unroll
-        for (int eh = 0; eh < 2; ++eh) {
-          const int p = 2 * eh;
-          auto mma = [&](float (&d)[4], const uint32_t (&qa)[2][4], const uint32_t (&kb)[4]) {
-            mma_bf16(d, qa[0][p], qa[1][p], qa[0][p + 1], qa[1][p + 1], kb[p], kb[p + 1]);
-          };
+          for (int p = 0; p < 4; p += 2)
 #pragma unroll
-          for (int nt = 0; nt < 2; ++nt) {
-            mma(acc[nt], ql, kh[nt]);
-            mma(acc[nt], qh, kl[nt]);
-            mma(acc[nt], qm, km[nt]);
-            mma(acc[nt], qm, kh[nt]);
-            mma(acc[nt], qh, km[nt]);
-            mma(acc[nt], qh, kh[nt]);
-          }
-        }
+            for (int nt = 0; nt < 2; ++nt) mma_bf16(d[nt], qa[0][p], qa[1][p], qa[0][p + 1], qa[1][p + 1], kb[nt][p], kb[nt][p + 1]);
+        };
+        mma(ql, kh);
+        mma(qh, kl);
+        mma(qm, km);
+        mma(qm, kh);
+        mma(qh, km);
+        mma(qh, kh);
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) acc[nt][i] += d[nt][i];
       }
     } else {
       // one exp per (i, j, channel), a lane for each of its eight (i, j) of the accumulator layout
