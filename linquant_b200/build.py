@@ -42,6 +42,8 @@ def _compile(src):
     r = subprocess.run([NVCC, *FLAGS, "-c", os.path.join(CSRC, src), "-o", obj], capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"nvcc failed on {src}:\n{r.stdout}\n{r.stderr}")
+    with open(obj[:-2] + ".ptxas", "w") as f:  # registers, spills and shared memory of every kernel
+        f.write(r.stderr)
     return src, r.stderr
 
 
