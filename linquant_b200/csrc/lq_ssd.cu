@@ -79,7 +79,8 @@ __global__ void __launch_bounds__(256) ssd_cumsum_kernel(lq_ssd_problem p, int h
       const double o = __shfl_up_sync(0xffffffffu, off, d);
       if (lane >= d) off += o;
     }
-    off -= sum;  // lanes below this one
+    off = __shfl_up_sync(0xffffffffu, off, 1);  // the lanes below this one (not off - sum: an infinite step would make it NaN)
+    if (lane == 0) off = 0.0;
     float y[NPL];
 #pragma unroll
     for (int i = 0; i < NPL; ++i) y[i] = (float)(off + v[i]);
