@@ -215,6 +215,16 @@ __global__ void __launch_bounds__(256, 2) zoo_prologue_delta_kernel(DeltaPrepArg
           }
         }
     }
+    // The pieces of an infinity are inf and inf - inf. Every channel of a rotated row is a sum over the whole row, so any one of
+    // them shows it; such rows are made again below.
+    unsigned odd = 0u;  // bit 4 i: row i, bit 4 i + 1: row i + 8
+    if (!KF32 && rot && dqk) {
+      float y0, y1, z;
+      y[0][0][0][0].get(y0, z);
+      y[0][0][1][0].get(y1, z);
+      odd = (__ballot_sync(0xffffffffu, !(fabsf(y0) <= 3.402823466e38f)) & 0x11111111u) |
+            ((__ballot_sync(0xffffffffu, !(fabsf(y1) <= 3.402823466e38f)) & 0x11111111u) << 1);
+    }
     const float inv_sq = 1.0f / a.sq[h];
     const F2 inv(inv_sq, inv_sq), scale(a.scale, a.scale);
 #pragma unroll
@@ -252,6 +262,27 @@ __global__ void __launch_bounds__(256, 2) zoo_prologue_delta_kernel(DeltaPrepArg
           *reinterpret_cast<uint4*>(s_k + t * LDK + 32 * m + 8 * j) = make_uint4(w[0], w[1], w[2], w[3]);
         }
       }
+    if constexpr (!KF32) {
+      if (odd != 0u) {  // a lane per channel, the row summed in fp32
+        __syncwarp();
+#pragma unroll 1
+        for (int i = 0; i < 16; ++i) {
+          if (((odd >> (4 * (i & 7) + (i >> 3))) & 1u) == 0u) continue;
+          const T* row = src + (tok0 + (size_t)(t0 + i) * a.H) * K;
+          for (int n = lane; n < K; n += 32) {
+            float sum = 0.f;
+#pragma unroll 1
+            for (int e = 0; e < K; ++e) {
+              const float x = __fmul_rn(Act<T>::to(row[e]), dq[e]);
+              sum += (__popc(e & n) & 1) ? -x : x;
+            }
+            const T v = Act<T>::from(__fmul_rn(sum, s_sgn[n]));
+            if (isq) a.qq[(tile * C + t0 + i) * K + n] = (int8_t)q8(__fmul_rn(Act<T>::to(v), a.scale), inv_sq, a.qmax);
+            else s_k[(t0 + i) * LDK + n] = v;
+          }
+        }
+      }
+    }
   }
   __syncthreads();
 
