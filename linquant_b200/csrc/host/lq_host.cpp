@@ -133,7 +133,7 @@ PyObject* zoo_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
     c10::cuda::CUDAGuard guard(c.dev);
     const at::Tensor &q = c.dense(a[1]), &k = c.dense(a[2]), &v = c.dense(a[3]);
     const int64_t B = q.size(0), T = q.size(1), H = q.size(2), K = q.size(3);
-    if (v.dim() != 4 || k.sizes() != q.sizes()) throw NotPlain{};
+    if (v.dim() != 4 || k.sizes() != q.sizes() || k.scalar_type() != q.scalar_type() || v.scalar_type() != q.scalar_type()) throw NotPlain{};
     const int64_t V = v.size(3);
     if (v.size(0) != B || v.size(1) != T || v.size(2) != H) throw NotPlain{};
     const int chunk = integer(a[11]), bits = integer(a[14]);

@@ -34,9 +34,34 @@ def _sylvester(n):
     return Hm
 
 
+def _fits(t, shape):
+    """The extents of ``shape`` in order; extents of 1 may be missing or added."""
+    return [n for n in t.shape if n != 1] == [n for n in shape if n != 1]
+
+
+def check_inputs(q, k, v, g, beta, scales, *, decay, rot_signs=None, dqk=None, initial_state=None):
+    """The kernels get bare pointers and read them with q's extents and dtype: whatever does not fit raises here."""
+    assert q.dim() == 4 and k.shape == q.shape and v.dim() == 4 and v.shape[:3] == q.shape[:3], \
+        f"q, k [B,T,H,K] and v [B,T,H,V] do not fit: {tuple(q.shape)}, {tuple(k.shape)}, {tuple(v.shape)}"
+    if not (q.dtype == k.dtype == v.dtype):
+        raise NotImplementedError(f"q, k and v must have one dtype (got {q.dtype}, {k.dtype}, {v.dtype})")
+    if not (q.device == k.device == v.device):
+        raise _cabi.LinQuantError(f"q, k and v must be on one device (got {q.device}, {k.device}, {v.device})")
+    B, T, H, K = q.shape
+    V = v.shape[3]
+    want = {"g": (g, (B, T, H, K) if decay == _cabi.DECAY_DIAGONAL else (B, T, H)), "beta": (beta, (B, T, H)),
+            "rot": (rot_signs, (K,)), "dqk": (dqk, (H, K)), "initial_state": (initial_state, (B, H, K, V))}
+    keys = {"q": (H,), "k": (H,), "kw": (H, K), "state": (H, V)}
+    keys.update({"vl": (H, V), "vw": (H, V)} if beta is None else {"w": (H,), "el": (H, V), "ew": (H, V)})
+    want.update({f"scale {n!r}": (scales.get(n), shape) for n, shape in keys.items()})
+    for name, (t, shape) in want.items():
+        assert t is None or _fits(t, shape), f"{name} has shape {tuple(t.shape)}, {shape} expected"
+
+
 def make_problem(q, k, v, g, beta, scales, *, decay, eta, sigma, tau, scale, chunk_size, bits, out, final_state,
                  rot_signs, dqk, keep, initial_state=None, unrot=None):
     """Builds the C descriptor. ``keep`` collects every temporary tensor whose storage the descriptor points to."""
+    check_inputs(q, k, v, g, beta, scales, decay=decay, rot_signs=rot_signs, dqk=dqk, initial_state=initial_state)
     B, T, H, K = q.shape
     V = v.shape[-1]
     dev = q.device
@@ -51,8 +76,8 @@ def make_problem(q, k, v, g, beta, scales, *, decay, eta, sigma, tau, scale, chu
         setattr(P, name, None if t is None else t.data_ptr())
 
     put("q", q); put("k", k); put("v", v)
-    put("g", None if g is None else g.to(torch.float32).contiguous())
-    put("beta", None if beta is None else beta.to(torch.float32).contiguous())
+    put("g", _cabi.f32c(g, dev))
+    put("beta", _cabi.f32c(beta, dev))
     put("rot_signs", rot_signs)
     put("dqk", _cabi.f32c(dqk, dev))
     for name, key in (("sq", "q"), ("sk", "k"), ("skw", "kw"), ("svl", "vl"), ("svw", "vw"), ("sstate", "state"),
@@ -60,7 +85,7 @@ def make_problem(q, k, v, g, beta, scales, *, decay, eta, sigma, tau, scale, chu
         put(name, _cabi.f32c(scales.get(key), dev))
     put("o", out)
     put("final_state", final_state)
-    put("initial_state", None if initial_state is None else initial_state.to(device=dev, dtype=torch.float32).contiguous())
+    put("initial_state", _cabi.f32c(initial_state, dev))
     if unrot is not None:  # the kernels want the fp16 matrix with the input index contiguous: element [v'][v] = unrot[v][v']
         assert tuple(unrot.shape) == (V, V), f"unrot must be ({V},{V})"
         unrot = unrot.to(device=dev, dtype=torch.float16).t().contiguous()
