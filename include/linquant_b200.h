@@ -62,6 +62,7 @@ int lq_selftest_wait_timeout(int* status, int* trace, int hold_tmem, lq_stream s
  * Gated DeltaNet / KDA). Layouts follow the reference: q,k [B,T,H,K], v,o [B,T,H,V] dense, act dtype f16/bf16;
  * g [B,T,H] (scalar) or [B,T,H,K] (diagonal) fp32 log-decay or null; beta [B,T,H] fp32 or null.
  * Scales are fp32: sq,sk,sw [H]; skw [H,K]; svl,svw,sel,sew,sstate [H,V]  (invariances.py:102-112).
+ * q, k, v, o, unrot_t and a diagonal g start on 16-byte boundaries (else LQ_ERR_ALIGN).
  * ------------------------------------------------------------------------------------------------------------ */
 typedef struct {
   int B, T, H, K, V, chunk;

@@ -53,6 +53,11 @@ struct Call {
     if (!shaped) u = u.expand(shape);
     return hold(u.contiguous()).const_data_ptr<float>();
   }
+  // what f32 gave for `o`, moved to a 16-byte boundary where it is a view that starts elsewhere
+  const float* aligned16(const float* p, PyObject* o) {
+    if ((reinterpret_cast<uintptr_t>(p) & 15u) == 0) return p;
+    return hold(tensor(o).clone(at::MemoryFormat::Contiguous)).const_data_ptr<float>();
+  }
   // dense, as it is otherwise; must live on this device
   const at::Tensor& dense(PyObject* o) {
     const at::Tensor& t = tensor(o);
@@ -148,7 +153,7 @@ PyObject* zoo_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
     p.scale = (float)(a[10] == Py_None ? std::pow((double)K, -0.5) : number(a[10]));
     p.qmax = (float)((1 << (bits - 1)) - 1);
     p.q = q.const_data_ptr(); p.k = k.const_data_ptr(); p.v = v.const_data_ptr();
-    if (a[4] != Py_None) p.g = diag ? c.f32(a[4], {B, T, H, K}, true) : c.f32(a[4], {B, T, H}, true);
+    if (a[4] != Py_None) p.g = diag ? c.aligned16(c.f32(a[4], {B, T, H, K}, true), a[4]) : c.f32(a[4], {B, T, H}, true);
     if (a[5] != Py_None) p.beta = c.f32(a[5], {B, T, H}, true);
     if (a[16] != Py_None) p.rot_signs = c.f32(a[16], {K}, true);
     if (a[17] != Py_None) p.dqk = c.f32(a[17], {H, K}, true);

@@ -41,6 +41,7 @@ int validate_zoo_problem(const lq_zoo_problem* p, bool delta, bool diagonal) {
   if ((p->decay != LQ_DECAY_NONE) != (p->g != nullptr)) return fail(LQ_ERR_SHAPE, "g must be given exactly when decay != none");
   if (!aligned16(p->q) || !aligned16(p->k) || !aligned16(p->v) || !aligned16(p->o))
     return fail(LQ_ERR_ALIGN, "q, k, v, o must be 16-byte aligned");
+  if (diagonal && !aligned16(p->g)) return fail(LQ_ERR_ALIGN, "a per-channel g must be 16-byte aligned");
   if (p->act_dtype != LQ_F16 && p->act_dtype != LQ_BF16) return fail(LQ_ERR_UNSUPPORTED, "activation dtype must be f16 or bf16");
   if (p->unrot_t != nullptr && !aligned16(p->unrot_t)) return fail(LQ_ERR_ALIGN, "unrot_t must be 16-byte aligned");
   if (!(p->qmax >= 1.f && p->qmax <= 127.f)) return fail(LQ_ERR_SHAPE, "qmax=%f out of range", (double)p->qmax);

@@ -76,7 +76,10 @@ def make_problem(q, k, v, g, beta, scales, *, decay, eta, sigma, tau, scale, chu
         setattr(P, name, None if t is None else t.data_ptr())
 
     put("q", q); put("k", k); put("v", v)
-    put("g", _cabi.f32c(g, dev))
+    gd = _cabi.f32c(g, dev)
+    if gd is not None and decay == _cabi.DECAY_DIAGONAL and gd.data_ptr() % 16:  # read in 16-byte pieces
+        gd = gd.clone()
+    put("g", gd)
     put("beta", _cabi.f32c(beta, dev))
     put("rot_signs", rot_signs)
     put("dqk", _cabi.f32c(dqk, dev))

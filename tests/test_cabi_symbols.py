@@ -64,3 +64,26 @@ def test_ctypes_layouts_match_the_compiled_structs():
     assert L.lq_struct_bytes(0) == ctypes.sizeof(_cabi.ZooProblem)
     assert L.lq_struct_bytes(1) == ctypes.sizeof(_ssd.SsdProblem)
     assert L.lq_struct_bytes(2) == ctypes.sizeof(_cabi.ZooWorkspace)
+
+
+def test_misaligned_pointers_are_refused_on_the_host():
+    """Pointers only: nothing is launched and nothing is read. The per-channel log-decay is read in 16-byte pieces; a scalar one
+    element by element."""
+    from linquant_b200 import _cabi
+
+    L = _cabi.lib()
+    p = _cabi.ZooProblem()
+    p.B, p.T, p.H, p.K, p.V, p.chunk, p.act_dtype, p.out_dtype, p.qmax = 1, 128, 2, 64, 64, 64, _cabi.LQ_BF16, _cabi.LQ_BF16, 127.0
+    for name, t in _cabi.ZooProblem._fields_:
+        if t is ctypes.c_void_p and name not in ("unrot_t", "status"):
+            setattr(p, name, 4096)
+    for entry, decay, align in (("lq_gla_fwd", 2, True), ("lq_kda_fwd", 2, True), ("lq_simple_gla_fwd", 1, False), ("lq_delta_fwd", 1, False)):
+        fn = getattr(L, entry)
+        fn.argtypes = [ctypes.POINTER(_cabi.ZooProblem), ctypes.c_void_p, ctypes.c_size_t, ctypes.c_void_p]
+        p.decay = decay
+        for name in ("q", "k", "v", "o", "g"):
+            setattr(p, name, 4096 + 4)
+            want = 3 if name != "g" or align else 1  # LQ_ERR_ALIGN, else LQ_ERR_NULL: no workspace was given
+            assert fn(ctypes.byref(p), None, 0, None) == want, (entry, name)
+            setattr(p, name, 4096)
+        assert fn(ctypes.byref(p), None, 0, None) == 1

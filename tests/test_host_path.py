@@ -36,6 +36,28 @@ def test_zoo_cells(cell, K, V, dtype, form):
     assert torch.equal(o, o2) and torch.equal(s, s2) and o.dtype == dtype and float(o.float().abs().max()) > 0
 
 
+@pytest.mark.parametrize("cell", ["gla", "kda"])
+@pytest.mark.parametrize("offset", [1, 2])
+def test_per_channel_decay_at_an_odd_address(cell, offset):
+    """A dense slice of a flat gate buffer that starts off a 16-byte boundary gives what an aligned copy of it gives."""
+    from linquant_b200.kernels import zoo
+
+    B, T, H, K, V = 1, 128, 2, 64, 64
+    q, k, v, g, beta = (t.cuda() for t in zoo_inputs(B, T, H, K, V, decay="diagonal", delta=True, dtype=torch.bfloat16, seed=6))
+    flat = torch.empty(g.numel() + 4, device="cuda")
+    odd = flat[offset:offset + g.numel()].view(g.shape).copy_(g)
+    assert odd.is_contiguous() and odd.data_ptr() % 16
+    full = lambda *s: torch.full(s, 0.01, device="cuda")  # noqa: E731
+    sc = {"q": full(H), "k": full(H), "kw": full(H, K), "vw": full(H, V), "vl": full(H, V), "state": full(H, V),
+          "w": full(H), "el": full(H, V), "ew": full(H, V)}
+    extra = (beta,) if cell == "kda" else ()
+    fn = getattr(zoo, f"chunk_{cell}_int8")
+    want, _ = fn(q, k, v, g, *extra, sc)
+    for debug in (None, {}):
+        got, _ = fn(q, k, v, odd, *extra, sc, _debug=debug)
+        assert torch.equal(got, want)
+
+
 def test_zoo_errors():
     from linquant_b200 import _cabi
     from linquant_b200.kernels.zoo import chunk_simple_gla_int8
