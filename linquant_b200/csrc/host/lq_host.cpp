@@ -330,6 +330,9 @@ PyObject* ssd_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
       p.x_scale_hp = c.f32(a[21], {H, P});
       const at::Tensor& bg0 = Call::tensor(a[23]);
       if (bg0.dim() != 4 || bg0.device() != c.dev) throw NotPlain{};
+      const int64_t full[4] = {B, NC, H, N};
+      for (int i = 0; i < 4; ++i)
+        if (bg0.size(i) != 1 && bg0.size(i) != full[i]) throw NotPlain{};
       const at::Tensor& bg = bg0.scalar_type() == at::kFloat ? bg0 : c.hold(bg0.to(at::kFloat));
       p.b_gate_scale = bg.const_data_ptr<float>();
       for (int i = 0; i < 4; ++i) p.bgs_stride[i] = bg.size(i) > 1 ? bg.stride(i) : 0;

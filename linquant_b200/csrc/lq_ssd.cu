@@ -859,6 +859,7 @@ __global__ void __launch_bounds__(256) ssd_rotate_rows_kernel(const T* x, long l
 }
 
 // ------------------------------------------------------------------------------------------------ launchers
+static bool misaligned(const void* p, unsigned bytes) { return (reinterpret_cast<uintptr_t>(p) & (bytes - 1)) != 0; }
 static int ssd_check(const lq_ssd_problem* p, const char* what) {
   if (!p) return fail(LQ_ERR_NULL, "%s: problem descriptor is null", what);
   if (p->B <= 0 || p->L <= 0 || p->H <= 0 || p->G <= 0) return fail(LQ_ERR_SHAPE, "%s: non-positive extent", what);
@@ -922,6 +923,8 @@ extern "C" int lq_ssd_chunk_cumsum(const lq_ssd_problem* p, lq_stream stream) {
 extern "C" int lq_ssd_state_passing(const lq_ssd_problem* p, lq_stream stream) {
   if (int e = ssd_check(p, "state_passing")) return e;
   if (!p->states || !p->passed || !p->final_state || !p->dA) return fail(LQ_ERR_NULL, "state_passing: states, passed, final_state, dA required");
+  if (misaligned(p->states, 8) || misaligned(p->passed, 8) || misaligned(p->final_state, 8))
+    return fail(LQ_ERR_ALIGN, "state_passing: states, passed, final_state must be 8-byte aligned");
   const int D = p->P * p->N;
   if (D % 8 != 0) return fail(LQ_ERR_SHAPE, "state_passing: P*N must be a multiple of 8");
   if ((p->carry_in && (reinterpret_cast<uintptr_t>(p->carry_in) & 15u)) || (p->carry_out && (reinterpret_cast<uintptr_t>(p->carry_out) & 15u)))
@@ -956,6 +959,7 @@ static int ssd_chunk_state(const lq_ssd_problem* p, bool keyside, lq_stream stre
   dim3 grid(p->L / p->chunk, p->H, p->B);
   if (keyside) {
     if (!p->b_fp || !p->x_scale_hp || !p->b_gate_scale) return fail(LQ_ERR_NULL, "%s: b_fp, x_scale_hp, b_gate_scale required", what);
+    if (misaligned(p->b_fp, 4)) return fail(LQ_ERR_ALIGN, "%s: b_fp must be 4-byte aligned", what);
     // d_state 128 with chunks of 128 / 256 tokens: tcgen05, two heads per CTA; else the warp-level MMA kernel
     if (chunk_state_key_tc_applies(p)) return run_chunk_state_key_tc(p, p->status, st);
     launch_chunk_state<true>(p, grid, st);
@@ -963,6 +967,7 @@ static int ssd_chunk_state(const lq_ssd_problem* p, bool keyside, lq_stream stre
     if (!p->q_B || !p->alpha_hp || !p->bscale_g) return fail(LQ_ERR_NULL, "%s: q_B, alpha_hp, bscale_g required", what);
     // d_state 128 with chunks of 128 / 256 tokens: both tcgen05 operands in their natural layouts, no scratch at all
     if (!with_qbt && chunk_state_value_tc2_applies(p)) return run_chunk_state_value_tc2(p, p->status, st);
+    if (misaligned(p->q_B, 4)) return fail(LQ_ERR_ALIGN, "%s: q_B must be 4-byte aligned", what);
     if (!p->q_BT) return fail(LQ_ERR_NULL, "%s: q_BT (scratch for the transposed q_B) required for this shape", what);
     launch(ssd_transpose_b_kernel, dim3(p->L / 64, p->G, p->B), 256, 0, st, p->q_B, p->q_BT, p->L, p->G, p->N, p->chunk);
     if (int e = check_launch("ssd_transpose_b_kernel")) return e;
@@ -1025,6 +1030,9 @@ extern "C" int lq_ssd_bmm_chunk(const lq_ssd_problem* p, int b_is_fp, lq_stream 
   if (p->N != 64 && p->N != 128) return fail(LQ_ERR_UNSUPPORTED, "bmm_chunk: d_state %d (64 or 128 supported)", p->N);
   if (!p->q_C || !p->C_scale || !p->B_scale || !p->cb_scale || !p->cb) return fail(LQ_ERR_NULL, "bmm_chunk: q_C, scales, cb required");
   if (b_is_fp ? !p->b_fp : !p->q_B) return fail(LQ_ERR_NULL, "bmm_chunk: B operand missing");
+  if (b_is_fp && p->x_dtype != LQ_F16 && p->x_dtype != LQ_BF16) return fail(LQ_ERR_UNSUPPORTED, "bmm_chunk: a floating-point B must be f16 or bf16");
+  if (misaligned(p->q_C, 16) || misaligned(b_is_fp ? p->b_fp : static_cast<const void*>(p->q_B), 16) || misaligned(p->cb, 8))
+    return fail(LQ_ERR_ALIGN, "bmm_chunk: q_C and the B operand must be 16-byte aligned, cb 8-byte aligned");
   const int tiles = p->chunk / 64;
   dim3 grid(tiles * tiles, (p->L / p->chunk) * p->G, p->B);
   cudaStream_t st = (cudaStream_t)stream;
@@ -1055,6 +1063,8 @@ extern "C" int lq_ssd_chunk_scan(const lq_ssd_problem* p, lq_stream stream) {
   if (p->scan_kernel == 2 && !tc_ok) return fail(LQ_ERR_UNSUPPORTED, "chunk_scan: the tcgen05 kernel needs d_state 128 and chunk 128 or 256");
   if (p->scan_kernel < 0 || p->scan_kernel > 2) return fail(LQ_ERR_SHAPE, "chunk_scan: scan_kernel must be 0, 1 or 2");
   if (p->scan_kernel == 2 || (p->scan_kernel == 0 && tc_ok)) return run_chunk_scan_tc(p, p->status, st);
+  if (misaligned(p->q_C, 16) || misaligned(p->passed, 16) || misaligned(p->cb, 16) || misaligned(p->out, 4))
+    return fail(LQ_ERR_ALIGN, "chunk_scan: q_C, cb and the passed states must be 16-byte aligned");
   if (p->x_dtype == LQ_F16) return p->N == 128 ? launch_scan<__half, 128>(p, st) : launch_scan<__half, 64>(p, st);
   return p->N == 128 ? launch_scan<__nv_bfloat16, 128>(p, st) : launch_scan<__nv_bfloat16, 64>(p, st);
 }

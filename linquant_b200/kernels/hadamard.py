@@ -34,6 +34,7 @@ def kronecker_hadamard_fwd(x, signs, num_heads, n_chunks=2):
         return y
     B, T, H, D = x.shape
     assert D >= 64, f"Kronecker Hadamard needs D >= 64, got {D}"
+    assert tuple(signs.shape) == (H, D) or signs.numel() == H * D, f"signs has shape {tuple(signs.shape)}, {(H, D)} expected"
     if x.stride(-1) != 1 or x.stride(2) != D or x.stride(0) != T * x.stride(1):
         x = x.contiguous()
     y = torch.empty(B, T, H, D, device=x.device, dtype=x.dtype)

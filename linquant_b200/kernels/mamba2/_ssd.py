@@ -92,6 +92,21 @@ def require_cuda(t, what):
         raise _cabi.LinQuantError(f"{what} runs on CUDA tensors only (no CPU path)")
 
 
+def expect(name, t, shape, device=None, dtype=None):
+    """The kernels get bare pointers: extents, and the device and dtype of what is handed over as it is, raise here."""
+    assert tuple(t.shape) == tuple(shape), f"{name} has shape {tuple(t.shape)}, {tuple(shape)} expected"
+    if dtype is not None and t.dtype != dtype:
+        raise NotImplementedError(f"{name} must be {dtype} (got {t.dtype})")
+    if device is not None and t.device != device:
+        raise _cabi.LinQuantError(f"{name} must be on {device} (got {t.device})")
+    return t
+
+
+def expect_count(name, t, n):
+    """A tensor that is flattened and converted on its way: its number of elements."""
+    assert t is None or torch.as_tensor(t).numel() == n, f"{name} has {torch.as_tensor(t).numel()} elements, {n} expected"
+
+
 def scalar_or_dev(call, name, v):
     """A Python number goes into the descriptor; a tensor stays on the device (no host synchronisation)."""
     if torch.is_tensor(v):

@@ -12,6 +12,8 @@ def _quant_bmm_chunk_fwd(a, a_scale, b, b_scale, chunk_size, static_cb_scale, b_
     B, L, G, K = a.shape
     nc = _ssd.nchunks(L, chunk_size)
     dev = a.device
+    _ssd.expect("a", a, (B, L, G, K), dev, torch.int8)
+    _ssd.expect("b", b, (B, L, G, K), dev, None if b_is_fp else torch.int8)
     cb_scale = static_cb_scale.float().contiguous()
     assert cb_scale.shape == (G,), f"static_cb_scale must be (ngroups,), got {cb_scale.shape}"
     call = _ssd.Call(dev).dims(B=B, L=L, H=G, P=64, G=G, N=K, chunk=chunk_size)

@@ -21,6 +21,14 @@ def _quant_chunk_scan_fwd(cb_i8, x_fp, dt, dA_cumsum, q_C, C_scale, states, q_D,
     _, _, G, N = q_C.shape
     B, L, H, P = x_fp.shape
     dev = x_fp.device
+    _ssd.expect("cb_i8", cb_i8, (B, nc, G, chunk, chunk), dev, torch.int8)
+    _ssd.expect("q_C", q_C, (B, L, G, N), dev, torch.int8)
+    _ssd.expect("states", states, (B, nc, H, P, N), dev, torch.int8)
+    assert nc * chunk == L, f"dt covers {nc} chunks of {chunk} tokens, x {L} tokens"
+    for name, t in (("dt", dt), ("dA_cumsum", dA_cumsum)):
+        _ssd.expect(name, t, (B, H, nc, chunk))
+    if q_D is not None:
+        _ssd.expect("q_D", q_D, (H, P) if q_D.dim() == 2 else (H,), dev)
     if kernel is None:  # LQ_SCAN_KERNEL names one of the kernels for a whole process (measurements, bisecting)
         kernel = os.environ.get("LQ_SCAN_KERNEL") or None
         if kernel == "tcgen05" and not (N == 128 and chunk % 128 == 0):

@@ -13,6 +13,11 @@ def _quant_chunk_state_fwd_xfp_static_int8(x_fp, q_B, dt, dA_cumsum, alpha_hp, b
     _, _, G, N = q_B.shape
     B, L, H, P = x_fp.shape
     dev = x_fp.device
+    _ssd.expect("q_B", q_B, (B, L, G, N), dev, torch.int8)
+    assert nc * chunk == L, f"dt covers {nc} chunks of {chunk} tokens, x {L} tokens"
+    for name, t in (("dt", dt), ("dA_cumsum", dA_cumsum)):
+        _ssd.expect(name, t, (B, H, nc, chunk))
+    _ssd.expect_count("bscale_g", bscale_g, G)
     call = _ssd.Call(dev).dims(B=B, L=L, H=H, P=P, G=G, N=N, chunk=chunk)
     call.x(x_fp)
     call.put("q_B", q_B.contiguous())

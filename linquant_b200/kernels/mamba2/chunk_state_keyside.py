@@ -19,6 +19,14 @@ def _chunk_state_keyside_fwd(x_fp, x_scale_hp, b_fp, dt, dA_cumsum, out_qscale, 
     _, _, G, N = b_fp.shape
     B, L, H, P = x_fp.shape
     dev = x_fp.device
+    _ssd.expect("b_fp", b_fp, (B, L, G, N), dev)
+    assert nc * chunk == L, f"dt covers {nc} chunks of {chunk} tokens, x {L} tokens"
+    for name, t in (("dt", dt), ("dA_cumsum", dA_cumsum)):
+        _ssd.expect(name, t, (B, H, nc, chunk))
+    assert all(n in (1, m) for n, m in zip(b_gate_scale.shape, (B, nc, H, N))), \
+        f"b_gate_scale has shape {tuple(b_gate_scale.shape)}, not broadcastable to {(B, nc, H, N)}"
+    if b_gate_scale.device != dev:
+        raise _ssd._cabi.LinQuantError(f"b_gate_scale must be on {dev} (got {b_gate_scale.device})")
     call = _ssd.Call(dev).dims(B=B, L=L, H=H, P=P, G=G, N=N, chunk=chunk)
     call.x(x_fp)
     call.put("b_fp", b_fp.to(x_fp.dtype).contiguous())

@@ -5,6 +5,7 @@ import ctypes as C
 
 import torch
 
+from . import _ssd
 from ... import _cabi
 
 
@@ -28,6 +29,9 @@ def fused_split_rotate_quant_xBC(xBC, r_signs, nheads, ngroups, d_state, headdim
     batch, seq_len, xBC_dim = xBC.shape
     d_ssm, g_n = nheads * headdim, ngroups * d_state
     assert xBC_dim == d_ssm + 2 * g_n, f"xBC_dim={xBC_dim} != {d_ssm + 2 * g_n}"
+    for name, t, n in (("r_signs", r_signs, g_n), ("B_inv_scale", B_inv_scale, ngroups), ("C_inv_scale", C_inv_scale, ngroups),
+                       ("dqk_b", dqk_b, g_n), ("dqk_c", dqk_c, g_n)):
+        _ssd.expect_count(name, t, n)
     xBC = xBC.contiguous()
     dev = xBC.device
     f32 = lambda t: None if t is None else t.to(device=dev, dtype=torch.float32).reshape(-1).contiguous()  # noqa: E731

@@ -21,12 +21,14 @@ def _fixedpoint_state_passing_fwd(states_i8, dA_chunk_cumsum, gate_shift=7, init
         raise NotImplementedError("the fixed-point gate is Q0.7 (gate_shift=7)")
     B, nc, H, dim = states_i8.shape
     dev = states_i8.device
+    _ssd.expect("states_i8", states_i8, (B, nc, H, dim), dev, torch.int8)
+    _ssd.expect("dA_chunk_cumsum", dA_chunk_cumsum, (B, H, nc))
     states_i8 = states_i8.contiguous()
     a = dA_chunk_cumsum
     # The kernel reads dA[b, h, c, chunk-1] of a dense [B,H,NC,chunk] buffer. The usual argument is exactly that
     # column of the chunk cumsum (dA_cumsum[..., -1]): then the cumsum's own storage is handed over untouched.
     C_ = a.stride(2) if a.dim() == 3 and nc > 1 else 0
-    if (a.dtype == torch.float32 and a.shape == (B, H, nc) and C_ in (64, 128, 192, 256) and a.stride(1) == nc * C_
+    if (a.dtype == torch.float32 and a.device == dev and C_ in (64, 128, 192, 256) and a.stride(1) == nc * C_
             and a.stride(0) == H * nc * C_ and a.storage_offset() >= C_ - 1):
         call = _ssd.Call(dev).dims(B=B, L=nc * C_, H=H, P=1, G=1, N=dim, chunk=C_)
         call.keep.append(a)
