@@ -73,6 +73,11 @@ def host():
             from . import _host as mod
         except ImportError as e:
             raise LinQuantError(f"linquant_b200/_host.so cannot be loaded ({e}): build it with `python -m linquant_b200.build`") from e
+        from .build import host_key
+
+        if mod.built_for != host_key():  # it reads at::Tensor: another torch may import it and misread its arguments
+            raise LinQuantError(f"linquant_b200/_host.so was built for {mod.built_for}, this is {host_key()}: build it with "
+                                "`python -m linquant_b200.build`")
         _host = mod
     return _host
 

@@ -17,6 +17,7 @@ OBJ = os.path.join(HERE, "csrc", "build")
 LIB = os.path.join(HERE, "liblinquant_b200.so")
 HOST_SRC = os.path.join(CSRC, "host", "lq_host.cpp")
 HOST_LIB = os.path.join(HERE, "_host.so")
+HOST_KEY = os.path.join(OBJ, "lq_host.key")  # what the object of _host was compiled for
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 # no fast-math: precise division / sqrt / expf are required by the code rule
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-Xptxas", "-v"]
@@ -47,18 +48,34 @@ def _compile(src):
     return src, r.stderr
 
 
+def host_key():
+    """The ABI that ``_host`` is tied to; ``_cabi.host()`` compares it with the running one."""
+    import torch
+
+    return f"torch {torch.__version__}, {sysconfig.get_config_var('SOABI')}"
+
+
+def _host_stale(obj):
+    if _stale(os.path.join("host", "lq_host.cpp"), obj) or not os.path.exists(HOST_KEY):
+        return True
+    with open(HOST_KEY) as f:
+        return f.read() != host_key()
+
+
 def _compile_host(_=None):
     """The object file of ``_host``, and the torch library directories to link it against."""
     from torch.utils import cpp_extension as ext
 
     obj = os.path.join(OBJ, "lq_host.o")
-    if _stale(os.path.join("host", "lq_host.cpp"), obj):
+    if _host_stale(obj):
         inc = ext.include_paths() + [sysconfig.get_paths()["include"], "/usr/local/cuda/include"]
-        cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-w", *[a for i in inc for a in ("-isystem", i)],
+        cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-Wall", f'-DLQ_BUILT_FOR="{host_key()}"', *[a for i in inc for a in ("-isystem", i)],
                "-c", HOST_SRC, "-o", obj]
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"g++ failed on lq_host.cpp:\n{r.stdout}\n{r.stderr}")
+        with open(HOST_KEY, "w") as f:
+            f.write(host_key())
     return obj, ext.library_paths()
 
 

@@ -385,4 +385,8 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, null
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__host(void) { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__host(void) {
+  PyObject* m = PyModule_Create(&module);
+  if (m != nullptr && PyModule_AddStringConstant(m, "built_for", LQ_BUILT_FOR) != 0) Py_CLEAR(m);
+  return m;
+}

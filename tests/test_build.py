@@ -1,4 +1,5 @@
-"""What the compiler made of the kernels, from the resource lines it printed when the objects were built."""
+"""The build: what the compiler made of the kernels, from the resource lines it printed when the objects were built, and the ABI
+that the host module is tied to."""
 
 import os
 import re
@@ -26,3 +27,18 @@ def test_ctas_per_sm(src, kernel, threads, ctas):
     """The kernel's time rests on this many CTAs on an SM (65 536 registers, dealt to warps in units of 8 per thread)."""
     regs = registers(src, kernel)
     assert regs and all(ctas * threads * ((r + 7) // 8 * 8) <= 65536 for r in regs), regs
+
+
+def test_host_module_is_tied_to_its_torch(monkeypatch):
+    import torch
+
+    from linquant_b200 import _cabi
+
+    build.build()
+    obj = os.path.join(build.OBJ, "lq_host.o")
+    assert not build._host_stale(obj) and _cabi.host().built_for == build.host_key()
+    monkeypatch.setattr(torch, "__version__", torch.__version__ + ".post1")
+    assert build._host_stale(obj)  # the next build compiles it again, whatever the file times say
+    monkeypatch.setattr(_cabi, "_host", None)
+    with pytest.raises(_cabi.LinQuantError, match="build it with"):
+        _cabi.host()
