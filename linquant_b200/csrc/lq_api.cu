@@ -13,6 +13,7 @@ int fail(int status, const char* fmt, ...) {
   va_start(ap, fmt);
   vsnprintf(g_err, sizeof(g_err), fmt, ap);
   va_end(ap);
+  if (status == LQ_ERR_LAUNCH) (void)cudaGetLastError();  // reported here: not to be found by the thread's next CUDA call
   return status;
 }
 

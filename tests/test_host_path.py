@@ -58,6 +58,27 @@ def test_per_channel_decay_at_an_odd_address(cell, offset):
         assert torch.equal(got, want)
 
 
+@pytest.mark.parametrize("cell", ["simple_gla", "gla", "delta", "kda"])
+def test_a_refused_launch_is_reported_once(cell):
+    """More (batch, head) pairs than a grid has rows: the launch is refused on the host. The next call, and torch's own next launch,
+    must not find that error."""
+    from linquant_b200 import _cabi
+    from linquant_b200.kernels import zoo
+
+    delta, diag, K = cell in ("delta", "kda"), cell in ("gla", "kda"), 64
+
+    def call(B, H):
+        zero = lambda *s, dtype=torch.float32: torch.zeros(*s, dtype=dtype, device="cuda")  # noqa: E731
+        q, k, v = (zero(B, 64, H, K, dtype=torch.bfloat16) for _ in range(3))
+        sc = {n: zero(H) + 1 for n in ("q", "k", "w")} | {n: zero(H, K) + 1 for n in ("kw", "vl", "vw", "state", "el", "ew")}
+        g = zero(B, 64, H, K) if diag else zero(B, 64, H)
+        return getattr(zoo, f"chunk_{cell}_int8")(q, k, v, g, *((zero(B, 64, H),) if delta else ()), sc)[0]
+
+    with pytest.raises(_cabi.LinQuantError, match="invalid configuration"):
+        call(4100, 16)
+    assert float((call(1, 2) + 1).abs().max()) == 1.0
+
+
 def test_zoo_errors():
     from linquant_b200 import _cabi
     from linquant_b200.kernels.zoo import chunk_simple_gla_int8
