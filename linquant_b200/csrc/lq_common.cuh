@@ -38,7 +38,8 @@ static inline cudaError_t launch(void (*kern)(KArgs...), dim3 grid, dim3 block, 
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
-}// More than 48 KB of dynamic shared memory: the opt-in is set on every launch (it is per kernel and device and costs a
+}
+// More than 48 KB of dynamic shared memory: the opt-in is set on every launch (it is per kernel and device and costs a
 // fraction of a microsecond).
 template <typename... KArgs, typename... Args>
 static inline cudaError_t launch_opt_in(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {

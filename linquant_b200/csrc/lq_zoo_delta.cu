@@ -429,7 +429,7 @@ struct DeltaStage {
 };
 template <int K, int KS, int GV, int NS>
 constexpr size_t delta_state_smem() {
-  return (size_t)NS * DeltaStage<K, GV>::kBytes + GV * 2048 + (KS > 1 ? GV * KS * 8 * 512 : 0) + 16 * NS + 4 * K;
+  return (size_t)NS * DeltaStage<K, GV>::kBytes + GV * 2048 + GV * KS * 8 * 512 + 16 * NS + 4 * K;
 }
 
 // A group of KS warps owns 16 value rows of the state; a warp keeps K / KS key channels of the fp32 carry in registers (rows
@@ -451,13 +451,14 @@ template <typename T, int K, int KS, int GV, int NS, int MINB, bool DIAG, bool Q
 __global__ void __launch_bounds__(32 * (KS * GV + 1), MINB) zoo_state_delta_kernel(DeltaStateArgs a) {
   pdl_enter();
   constexpr int C = 64, NB = K / 32 / KS, NTE = 8 / KS, TE = 2 * NTE;
+  static_assert(KS == 2 || KS == 4, "a group is two or four warps");
   typedef DeltaStage<K, GV> S;
   extern __shared__ __align__(128) uint8_t smem_raw[];
   uint8_t* s_stage = smem_raw;                                  // [NS][S::kBytes]
   uint8_t* s_codes = s_stage + NS * S::kBytes;                  // [GV][e_write | e_local][16][C]
   int4* s_part = reinterpret_cast<int4*>(s_codes + GV * 2048);  // [GV][from][n-tile][lane]
-  const uint32_t bars = smem_u32(s_codes + GV * 2048 + (KS > 1 ? GV * KS * 8 * 512 : 0));  // full[NS], empty[NS]
-  float* s_skw = reinterpret_cast<float*>(s_codes + GV * 2048 + (KS > 1 ? GV * KS * 8 * 512 : 0) + 16 * NS);  // [K]
+  const uint32_t bars = smem_u32(s_codes + GV * 2048 + GV * KS * 8 * 512);  // full[NS], empty[NS]
+  float* s_skw = reinterpret_cast<float*>(s_codes + GV * 2048 + GV * KS * 8 * 512 + 16 * NS);  // [K]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int bh = blockIdx.y, h = bh % a.H;
@@ -507,10 +508,7 @@ __global__ void __launch_bounds__(32 * (KS * GV + 1), MINB) zoo_state_delta_kern
   const int va = v0 + 16 * gv + g, vb = va + 8;
   const int kc0 = 32 * NB * ks + 8 * j;  // first of the lane's eight key channels in its first block
   const int t0 = 16 * j + TE * ks;       // first of the lane's TE tokens
-  auto group_sync = [&]() {
-    if (KS == 1) __syncwarp();
-    else asm volatile("bar.sync %0, %1;\n" ::"r"(1 + gv), "n"(32 * KS) : "memory");
-  };
+  auto group_sync = [&]() { asm volatile("bar.sync %0, %1;\n" ::"r"(1 + gv), "n"(32 * KS) : "memory"); };
   F2 nsws[2], ihq[2], isel[2], isew[2], sew[2];  // per value row: -s_w s_state, 1 / s_state, 1 / s_el, 1 / s_ew, s_ew
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
@@ -588,30 +586,22 @@ __global__ void __launch_bounds__(32 * (KS * GV + 1), MINB) zoo_state_delta_kern
 #pragma unroll
       for (int b = 0; b < NB; ++b) {
         const uint2 w = EARLY ? wf[EARLY ? nt : 0] : *reinterpret_cast<const uint2*>(wrow + b * 2048 + nt * 256);
-        if (b == 0 && KS == 1) mma_s8_biased(acc, hq[b][0][0], hq[b][1][0], hq[b][0][1], hq[b][1][1], w.x, w.y);
-        else if (b == 0) mma_s8_first(acc, hq[b][0][0], hq[b][1][0], hq[b][0][1], hq[b][1][1], w.x, w.y);
+        if (b == 0) mma_s8_first(acc, hq[b][0][0], hq[b][1][0], hq[b][0][1], hq[b][1][1], w.x, w.y);
         else mma_s8(acc, hq[b][0][0], hq[b][1][0], hq[b][0][1], hq[b][1][1], w.x, w.y);
       }
-      if (KS > 1) {
-        s_part[((gv * KS + ks) * 8 + nt) * 32 + lane] = make_int4(acc[0], acc[1], acc[2], acc[3]);
-      } else {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) ws[nt % NTE][e] = acc[e];
-      }
+      s_part[((gv * KS + ks) * 8 + nt) * 32 + lane] = make_int4(acc[0], acc[1], acc[2], acc[3]);
     }
-    if (KS > 1) {
-      group_sync();
+    group_sync();
 #pragma unroll
-      for (int i = 0; i < NTE; ++i) {
-        const int4* p = s_part + (gv * KS * 8 + NTE * ks + i) * 32 + lane;
-        int4 s = p[0];
+    for (int i = 0; i < NTE; ++i) {
+      const int4* p = s_part + (gv * KS * 8 + NTE * ks + i) * 32 + lane;
+      int4 s = p[0];
 #pragma unroll
-        for (int q = 1; q < KS; ++q) {
-          const int4 x = p[q * 256];
-          s.x += x.x; s.y += x.y; s.z += x.z; s.w += x.w;
-        }
-        ws[i][0] = s.x + 0x4B400000; ws[i][1] = s.y + 0x4B400000; ws[i][2] = s.z + 0x4B400000; ws[i][3] = s.w + 0x4B400000;
+      for (int q = 1; q < KS; ++q) {
+        const int4 x = p[q * 256];
+        s.x += x.x; s.y += x.y; s.z += x.z; s.w += x.w;
       }
+      ws[i][0] = s.x + 0x4B400000; ws[i][1] = s.y + 0x4B400000; ws[i][2] = s.z + 0x4B400000; ws[i][3] = s.w + 0x4B400000;
     }
 
     // ---- 3. E = (U - ws) fw and its codes for TE tokens of two value rows

@@ -29,7 +29,7 @@ struct DiagArgs {
   float scale, eta, sigma, tau, qmax;
 };
 
-template <int K, int BATCH = 64 * K / 4 / 256>
+template <int K, int BATCH>
 __device__ __forceinline__ void load_gc_tile(const float* gc_tile, float* s_gc) {  // 256 threads
   // BATCH 16-byte loads of the thread are requested before the first of them is stored (one or two trips to memory
   // instead of one per load)
@@ -741,10 +741,9 @@ static void fill_diag_args(const lq_zoo_problem* p, const lq_zoo_workspace* ws, 
 }
 
 template <typename KernelT>
-static int launch_big_smem(KernelT kern, const char* name, dim3 grid, size_t smem, const DiagArgs& a, cudaStream_t st) {
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return fail(LQ_ERR_LAUNCH, "%s: cannot opt in to %zu bytes of shared memory: %s", name, smem, cudaGetErrorString(e));
-  launch(kern, grid, 256, smem, st, a);
+static int launch_diag(KernelT kern, const char* name, dim3 grid, size_t smem, const DiagArgs& a, cudaStream_t st) {
+  const cudaError_t e = launch_opt_in(kern, grid, 256, smem, st, a);
+  if (e != cudaSuccess) return fail(LQ_ERR_LAUNCH, "%s (%zu bytes of shared memory): %s", name, smem, cudaGetErrorString(e));
   return check_launch(name);
 }
 
@@ -753,14 +752,14 @@ static int run_diag_T(const lq_zoo_problem* p, const DiagArgs& a, bool delta, in
   dim3 grid(a.NT, p->B * p->H);
   if (stage == 0) {
     constexpr size_t smem = diag_rows_smem<K, V>();
-    if (delta) return launch_big_smem(zoo_diag_rows_kernel<T, K, V, true>, "zoo_diag_rows_kernel", grid, smem, a, st);
-    return launch_big_smem(zoo_diag_rows_kernel<T, K, V, false>, "zoo_diag_rows_kernel", grid, smem, a, st);
+    if (delta) return launch_diag(zoo_diag_rows_kernel<T, K, V, true>, "zoo_diag_rows_kernel", grid, smem, a, st);
+    return launch_diag(zoo_diag_rows_kernel<T, K, V, false>, "zoo_diag_rows_kernel", grid, smem, a, st);
   }
   if (stage == 1) {
     const size_t smem = sizeof(float) * (64 * (K + 4) + K + 64) + (size_t)9 * (K / 32) * 512;
-    return launch_big_smem(zoo_diag_amat_kernel<T, K>, "zoo_diag_amat_kernel", grid, smem, a, st);
+    return launch_diag(zoo_diag_amat_kernel<T, K>, "zoo_diag_amat_kernel", grid, smem, a, st);
   }
-  return launch_big_smem(zoo_kda_wy_kernel<T, K, V>, "zoo_kda_wy_kernel", grid, kda_wy_smem<K, V>(), a, st);
+  return launch_diag(zoo_kda_wy_kernel<T, K, V>, "zoo_kda_wy_kernel", grid, kda_wy_smem<K, V>(), a, st);
 }
 
 template <typename T>

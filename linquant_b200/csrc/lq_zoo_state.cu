@@ -32,9 +32,8 @@ template <int NC>
 __device__ __forceinline__ void store_codes(int8_t* dst, const float (&x)[NC], float inv) {
   if constexpr (NC == 8) {
     *reinterpret_cast<uint2*>(dst) = make_uint2(q8x4_127(x[0], x[1], x[2], x[3], inv), q8x4_127(x[4], x[5], x[6], x[7], inv));
-  } else if constexpr (NC == 4) {
-    *reinterpret_cast<uint32_t*>(dst) = q8x4_127(x[0], x[1], x[2], x[3], inv);
   } else {
+    static_assert(NC == 2, "key channels per thread");
     *reinterpret_cast<uint16_t*>(dst) = (uint16_t)pack_sat_s8x2(q8_lower127(x[1], inv), q8_lower127(x[0], inv), 0u);
   }
 }
