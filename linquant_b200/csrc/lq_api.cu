@@ -23,6 +23,13 @@ int check_launch(const char* what) {
   return LQ_OK;
 }
 
+int sm_count() {
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // Mirrors the reference's asserts (zoo/gla.py:246, zoo/gated_delta_rule.py:170, zoo/kda.py:165): T % chunk == 0,

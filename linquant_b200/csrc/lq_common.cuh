@@ -13,6 +13,7 @@ namespace lq {
 // ---- host-side error plumbing (defined in lq_api.cu)
 int fail(int status, const char* fmt, ...);
 int check_launch(const char* what);
+int sm_count();  // of the current device
 
 // ---- programmatic dependent launch
 // The kernels of a call form a chain in which each reads what the one before wrote. They are launched with the

@@ -912,7 +912,7 @@ extern "C" int lq_ssd_chunk_cumsum(const lq_ssd_problem* p, lq_stream stream) {
   if (int e = ssd_check(p, "chunk_cumsum")) return e;
   if (!p->dt_in || !p->A_log || !p->dt || !p->dA) return fail(LQ_ERR_NULL, "chunk_cumsum: dt_in, A_log, dt, dA required");
   // sixteen heads per CTA (64-byte pieces of a token's row); eight where that would leave the GPU underfilled
-  const int hs = (long long)(p->L / p->chunk) * p->B * ((p->H + 15) / 16) < 296 ? 8 : 16;
+  const int hs = (long long)(p->L / p->chunk) * p->B * ((p->H + 15) / 16) < 2 * sm_count() ? 8 : 16;
   const dim3 grid(p->L / p->chunk, p->B, (p->H + hs - 1) / hs);
   const size_t smem = (size_t)hs * (p->chunk + 33) * sizeof(float);
   auto kern = p->chunk == 256 ? ssd_cumsum_kernel<256> : p->chunk == 192 ? ssd_cumsum_kernel<192> : p->chunk == 128 ? ssd_cumsum_kernel<128> : ssd_cumsum_kernel<64>;
@@ -1114,8 +1114,9 @@ static int launch_rotate(const T* x, long long sb, long long stt, long long ob, 
                          int gy, const float* signs, const float* ib, const float* ic, const float* db, const float* dc,
                          int8_t* qb, int8_t* qc, T* y, cudaStream_t st) {
   // 256 rows per CTA amortise the per-thread constants; a problem too small to fill the GPU that way takes 128 or 64
+  const int fill = 4 * sm_count();
   int rows_per_cta = 256;
-  while (rows_per_cta > 64 && (long long)((T_len + rows_per_cta - 1) / rows_per_cta) * gy * B < 592) rows_per_cta >>= 1;
+  while (rows_per_cta > 64 && (long long)((T_len + rows_per_cta - 1) / rows_per_cta) * gy * B < fill) rows_per_cta >>= 1;
   dim3 grid((T_len + rows_per_cta - 1) / rows_per_cta, gy, B);
   if (N == 128) launch(ssd_rotate_rows_kernel<T, 128, QUANT>, grid, 256, 0, st, x, sb, stt, ob, oc, T_len, G, signs, ib, ic, db, dc, qb, qc, y, rows_per_cta);
   else if (N == 64) launch(ssd_rotate_rows_kernel<T, 64, QUANT>, grid, 256, 0, st, x, sb, stt, ob, oc, T_len, G, signs, ib, ic, db, dc, qb, qc, y, rows_per_cta);

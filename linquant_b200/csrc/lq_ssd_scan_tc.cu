@@ -590,9 +590,7 @@ int run_chunk_scan_tc(const lq_ssd_problem* p, int* status, cudaStream_t st) {
     const cuuint32_t box[4] = {64, 1, (cuuint32_t)C, 1};
     if (int e = encode_map4(&to, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, p->out, gdim, gstr, box, "chunk_scan (out)")) return e;
   }
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = sm_count();
   const size_t smem = 2 * (size_t)scantc::kStageBytes + scantc::kRing * 16384 + 2 * 8192 + 1024 + 64 + 64 + 512 + 512 + 512 + 96 + 16 + 1024;
   const int grid = (int)(items < sms ? items : sms);
   cudaError_t e;

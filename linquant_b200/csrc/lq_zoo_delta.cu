@@ -1000,7 +1000,7 @@ template <typename T, int K, bool Q127>
 static cudaError_t launch_delta_state(const lq_zoo_problem* p, const DeltaStateArgs& a, cudaStream_t st) {
   // Up to two groups of 16 value rows per SM: one group per CTA, a warp per 32 key channels (the shortest step). More: two
   // warps per group and two groups per CTA (fewer instructions per group; three CTAs per SM).
-  if ((long long)p->B * p->H * (p->V / 16) <= 296) return launch_delta_state_v<T, K, Q127, 4, 1, 2, 1>(p, a, st);
+  if ((long long)p->B * p->H * (p->V / 16) <= 2 * sm_count()) return launch_delta_state_v<T, K, Q127, 4, 1, 2, 1>(p, a, st);
   return launch_delta_state_v<T, K, Q127, 2, 2, 2, 3>(p, a, st);
 }
 

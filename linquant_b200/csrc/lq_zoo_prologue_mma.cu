@@ -319,11 +319,8 @@ __global__ void __launch_bounds__(256, 2) zoo_prologue_linear_mma_kernel(Prologu
 template <typename T, int K, int V>
 static int launch_mma(const lq_zoo_problem* p, const PrologueArgs& a, cudaStream_t st) {
   const int tiles = a.NT * p->B * p->H;
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   // a grid that is a multiple of the head count keeps every CTA on one head (its scales are staged once)
-  int ctas = 2 * sms;
+  int ctas = 2 * sm_count();
   if (p->H <= ctas) ctas = (ctas / p->H) * p->H;
   dim3 grid(tiles < ctas ? tiles : ctas), block(256);
   const size_t smem = sizeof(uint32_t) * 17 * (K + 2 * V) + sizeof(float) * (2 * K + 2 * V) + (size_t)(4 * 64 * K * 2 + 64 * V * 2);

@@ -180,7 +180,8 @@ int run_state_linear(const lq_zoo_problem* p, const lq_zoo_workspace* ws, cudaSt
   // four chunks in flight; up to two per SM, three chunks in flight (up to 219 registers); beyond that one in flight, which
   // keeps five CTAs per SM (at 512 CTAs two in flight in 128 registers took 59 us instead of 52).
   const long long n64 = (long long)(p->V / 32) * (p->K / 64) * p->B * p->H;
-  const bool quarter = n64 <= 148, deep = n64 <= 296;
+  const int sms = sm_count();
+  const bool quarter = n64 <= sms, deep = n64 <= 2 * sms;
   dim3 grid((p->V / 32) * (p->K / (quarter ? 16 : 64)), p->B * p->H), block(128);
 #define LQ_LAUNCH_STATE_N(KK_, VV_, DD_)                                                                \
   if (quarter) launch(zoo_state_linear_kernel<KK_, VV_, DD_, 1, 4>, grid, block, 0, st, a);             \
