@@ -19,7 +19,7 @@ int sm_count();  // of the current device
 // The kernels of a call form a chain in which each reads what the one before wrote. They are launched with the
 // stream-serialisation attribute and open with pdl_enter(), which waits until everything before has completed and is
 // visible: the launch itself (block scheduling, instruction and parameter fetch) then overlaps the end of the kernel before,
-// 1 to 3 us per kernel, which is a third of a short prompt's time (six Mamba-2 kernels on one chunk: 55 -> 30 us). All
+// 1 to 3 us per kernel, which is a third of a short prompt's time (a Mamba-2 layer on one chunk: 55 -> 38 us). All
 // memory traffic, barrier set-up and tensor-memory allocation stay behind the wait. No kernel triggers its successor
 // early: CTAs that are placed while a kernel is still running fill whatever SMs have room, several to an SM, and the serial
 // state passes then keep that uneven placement to their end (DeltaNet, 1 x 1024 tokens: 75 us instead of 60).

@@ -1,5 +1,6 @@
-// WY-representation helpers shared by the delta-rule prologues: TF32 MMA wrappers, the unit-lower-triangular
-// inverse by forward substitution and the T . diag(cw) . B product with the left factor split into three TF32 pieces.
+// WY-representation helpers shared by the delta-rule prologues: the blocked unit-lower-triangular inverse (forward substitution
+// inside 16 x 16 blocks, the blocks below by doubling as 3xTF32 products) and the T . diag(cw) . B product with the left
+// factor split into three bf16 pieces.
 #pragma once
 #include <type_traits>
 

@@ -3,12 +3,12 @@
 // Prologue (one CTA per (batch*head, chunk), parallel over chunks):
 //   q, k rows as in the linear prologue (rescale, Walsh-Hadamard rotation, rounding, codes); the readout/write
 //   key is Hw = round(beta^((1-sigma)tau) * k). Then the WY representation of the chunk in fp32-grade arithmetic:
-//     G = tril( (beta^sigma k)(beta^(1-sigma) k)^T * exp(gc_i - gc_j), -1 )      TF32 MMA on exact operands
-//     T = (I + G)^-1                                                             forward substitution in smem
-//     W = T diag(beta^sigma exp(gc)) k ,  U = T diag(beta^sigma) v              3xTF32 split MMA (A split in three)
+//     G = tril( (beta^sigma k)(beta^(1-sigma) k)^T * exp(gc_i - gc_j), -1 )      fp16 / bf16 MMA on the keys as they are
+//     T = (I + G)^-1                                                             blocked inverse (lq_wy.cuh)
+//     W = T diag(beta^sigma exp(gc)) k ,  U = T diag(beta^sigma) v              bf16 MMA, the left factor in three pieces
 //   W is rounded to the activation dtype and quantised per head (w_read codes); U is stored in the activation dtype.
-//   Operands k, v are fp16/bf16 values, exactly representable in TF32, and the fp32 left factor is split into three
-//   TF32 pieces, so every product is exact and only the fp32 accumulation rounds.
+//   k and v are one bf16 piece (bf16) or two (fp16), the fp32 left factor T diag(.) three (8 + 8 + 8 bits): every product is
+//   exact and only the fp32 accumulation rounds.
 //
 // State pass (groups of warps own 16 value channels of a (batch, head), serial over chunks, fp32 carry [v,k] in registers):
 //   hq = q8(carry)  -> stored state and MMA operand;  ws = wq . hq (INT8 MMA);  E = (U - deq(ws)) * fw
@@ -445,7 +445,7 @@ constexpr size_t delta_state_smem() {
 // the GV groups of the CTA. The step is serial over the chunks: bound by its latency with few (b, h), by instruction issue
 // with many (about 400 instructions per warp and step; shared memory 40 %, ALU pipe 26 % busy). Measured at K = V = 128
 // against one CTA per 32 value rows with E codes stored bytewise and two block barriers per step: 25.6 -> 15.5 us at 16
-// (b, h) x 16 chunks, 280 -> 237 us at 64 x 128; diagonal decay 54 -> 38 us at 32 x 31, 994 -> 720 us at 256 x 128.
+// (b, h) x 16 chunks, 280 -> 240 us at 64 x 128; diagonal decay 54 -> 38 us at 32 x 31, 994 -> 720 us at 256 x 128.
 // Every wait is bounded; on expiry the CTA raises the status word, stores nothing more and waits no more.
 template <typename T, int K, int KS, int GV, int NS, int MINB, bool DIAG, bool Q127>
 __global__ void __launch_bounds__(32 * (KS * GV + 1), MINB) zoo_state_delta_kernel(DeltaStateArgs a) {

@@ -5,7 +5,8 @@
 //          gated k_write codes (Omega * s^-eta), and for the linear family the v_local / v_write codes
 //   amat   the intra-chunk matrix A in 16-token secondary chunks: off-diagonal blocks as INT8 MMAs on operands
 //          re-scaled around the block's anchor row (optionally rotated by a signed Hadamard on fp16-rounded values),
-//          diagonal blocks as an fp32 reduction with the exact per-channel weights on the dequantised codes
+//          diagonal blocks as tensor-core products of the dequantised codes times their weights around the block's first
+//          row, three bf16 pieces each (an fp32 reduction with one exp per (i, j, channel) where the decay is too strong)
 //   kda_wy KDA only: unquantised Gram matrix with per-channel weights, (I+G)^-1, W codes, U
 // The state pass and the output kernel are the scalar-decay kernels instantiated with per-channel carry decay
 // and a precomputed A.
@@ -50,7 +51,7 @@ __device__ __forceinline__ void load_gc_tile(const float* gc_tile, float* s_gc) 
 // ------------------------------------------------------------------------------------------------ rows
 // Work items of a warp: 32 tokens x 32 channels of q and k, or of v; a thread takes four tokens x eight channels, so that the
 // transposed codes are whole words and go straight to global memory (32 contiguous bytes per channel). The q / k rows travel
-// during the decay scan. Bound by instruction issue and the scan's latency. The kernel before it (codes one at a time,
+// during the decay scan. Bound by HBM at the KDA configuration, by the scan's latency where few CTAs run. The kernel before it (codes one at a time,
 // transposed through shared memory, rows requested after the scan) took 892 us for 256 (b, h) x 128 chunks at K = 128 (KDA)
 // and 88 us for 32 x 64 with K = V = 128 (GLA); this one 584
 // (0.98 of the time its 3.8 GB take at 6.55 TB/s) and 56.
@@ -229,7 +230,8 @@ __global__ void __launch_bounds__(256, 3) zoo_diag_rows_kernel(DiagArgs a) {
 // Bound by instruction issue. The kernel before it (operands through shared memory, shuffle butterflies, 3xTF32 with the
 // split in the product loop: 42 k warp instructions and 27 block barriers per chunk) took 2070 us for 256 (b, h) x 128 chunks at
 // K = 128, this one 1637; with pairwise exponentials, the channel loop of the diagonal blocks rolled (unrolled, waiting for instructions
-// was the first stall) and one form of the code rule 1236.
+// was the first stall) and one form of the code rule 1228; 1233 since a diagonal block is summed from one fresh accumulator per 32
+// channels (sums in one accumulator throughout cut off bits: up to 1.5 times as many fp16 results beside the right one).
 template <typename T, int K>
 __global__ void __launch_bounds__(256) zoo_diag_amat_kernel(DiagArgs a) {
   pdl_enter();

