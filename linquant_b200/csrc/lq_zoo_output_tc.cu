@@ -10,6 +10,9 @@
 //     reads them with tcgen05.ld.16x256b, which hands each thread the (row g / g+8, column 2j / 2j+1) fragment of a
 //     warp-level MMA. The decay-masked P therefore feeds the fp16 A.v product (mma.sync on the value codes, staged by
 //     cp.async) directly from registers, exactly as in the mma.sync version of this kernel.
+// Bound by latency (a CTA is one pass through load, product, mask, product, store; four share an SM) and, with many, by instruction
+// issue. Every warp waits for the accumulators on its own (block barriers with one polling thread: 65 us at 64 (b, h) x 64 chunks,
+// V = 128, and 7.1 at 16 x 2), and the scales of the state read are multiplied once, two channels to an instruction: 59 and 6.4.
 // Every wait on an mbarrier is bounded; on expiry the CTA raises the status word, skips its stores and still frees TMEM.
 // Arithmetic and references: see lq_zoo_output.cu.
 #include "lq_tc.cuh"
@@ -63,6 +66,7 @@ __global__ void __launch_bounds__(128) zoo_output_tc_kernel(const __grid_constan
   float* s_svl = s_ss + V;
   uint64_t* bars = reinterpret_cast<uint64_t*>(s_svl + V);  // [0] operands landed, [1] S2, [2] S1 first half, [3] second half
   uint32_t* s_tbase = reinterpret_cast<uint32_t*>(bars + 4);
+  volatile uint32_t* s_failed = s_tbase + 1;  // written by the issuing thread ahead of its arrivals, read after the waits
 
   const int c = blockIdx.x, bh = blockIdx.y;
   const int b = bh / a.H, h = bh % a.H;
@@ -72,6 +76,7 @@ __global__ void __launch_bounds__(128) zoo_output_tc_kernel(const __grid_constan
   const uint32_t bar_ld = smem_u32(&bars[0]), bar_s2 = smem_u32(&bars[1]), bar_s1 = smem_u32(&bars[2]), bar_s1b = smem_u32(&bars[3]);
 
   if (tid == 0) {
+    *s_failed = 0u;
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(bar_ld));
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(bar_s2));
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(bar_s1));
@@ -92,7 +97,7 @@ __global__ void __launch_bounds__(128) zoo_output_tc_kernel(const __grid_constan
     cp_async_commit();
     if (tid < C) s_gc[tid] = a.gc[tile * C + tid];
     for (int i = tid; i < V; i += 128) {
-      s_ss[i] = a.ss[h * V + i];
+      s_ss[i] = __fmul_rn(a.sq[h], a.ss[h * V + i]);
       s_svl[i] = a.svl[h * V + i];
     }
   }
@@ -117,16 +122,13 @@ __global__ void __launch_bounds__(128) zoo_output_tc_kernel(const __grid_constan
       umma_commit(bar_s1);
     } else {
       atomicExch(a.status, 1);
+      *s_failed = 1u;
       // release the waiters: nothing was issued, so arrive on both accumulator barriers by hand
       asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar_s2) : "memory");
       asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar_s1) : "memory");
       asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar_s1b) : "memory");
     }
   }
-  cp_async_wait<0>();
-  __syncthreads();
-  ok = __syncthreads_and(ok ? 1 : 0) != 0;
-
   const float sq = a.sq[h], sk = a.sk[h];
   const float sqk = __fmul_rn(sq, sk);
   const int ia = warp * 16 + g, ib = ia + 8;
@@ -136,8 +138,7 @@ __global__ void __launch_bounds__(128) zoo_output_tc_kernel(const __grid_constan
   // ---- S2 -> P (fp16 A fragments). S2 column n is row n of the k_local tile = token 16*(n/16) + 4j + 2*half + e
   // for n = 16ks + 8*half + 2j + e.
   uint32_t P[4][4];
-  if (tid == 0 && ok) ok = mbar_wait_bounded(bar_s2, 0);  // one poller per barrier; the block barrier releases the rest
-  ok = __syncthreads_and(ok ? 1 : 0) != 0;
+  ok = __all_sync(0xffffffffu, mbar_wait_bounded(bar_s2, 0) && *s_failed == 0u);  // every warp on its own: no block barrier
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
 #pragma unroll
   for (int ks = 0; ks < 4; ++ks) {
@@ -162,9 +163,11 @@ __global__ void __launch_bounds__(128) zoo_output_tc_kernel(const __grid_constan
     }
   }
 
-  if (V == 128) {  // S2 has been read by every warp: its columns now take the second half of the state product
-    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();
+  // S2 has been read by every warp: its columns now take the second half of the state product; the value codes have landed
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+  cp_async_wait<0>();
+  __syncthreads();
+  if (V == 128) {
     if (tid == 0) {
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
       if (ok) {
@@ -198,8 +201,7 @@ __global__ void __launch_bounds__(128) zoo_output_tc_kernel(const __grid_constan
   }
 
   // ---- S1 from TMEM, combine, store. S1 column n is row n of the state tile = channel 32*(n/32) + 8j + 2*n4 + e.
-  if (tid == 0 && ok) ok = mbar_wait_bounded(bar_s1, 0);
-  ok = __syncthreads_and(ok ? 1 : 0) != 0;
+  ok = __all_sync(0xffffffffu, mbar_wait_bounded(bar_s1, 0) && ok);
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
   if (ok) {
     const float ega = __expf(gia), egb = __expf(gib);
@@ -221,20 +223,18 @@ __global__ void __launch_bounds__(128) zoo_output_tc_kernel(const __grid_constan
       float outa[8], outb[8];
 #pragma unroll
       for (int n4 = 0; n4 < 4; ++n4) {
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int vc = 32 * ng + 8 * j + 2 * n4 + e;
-          const float ss = s_ss[vc], svl = s_svl[vc];
-          const float ra = __fmul_rn(__fmul_rn(__fmul_rn((float)(int)r[4 * n4 + e], sq), ss), ega);
-          const float rb = __fmul_rn(__fmul_rn(__fmul_rn((float)(int)r[4 * n4 + 2 + e], sq), ss), egb);
-          outa[2 * n4 + e] = fmaf(acco[4 * ng + n4][e], svl, ra);
-          outb[2 * n4 + e] = fmaf(acco[4 * ng + n4][2 + e], svl, rb);
-        }
+        const int vc = 32 * ng + 8 * j + 2 * n4;
+        const float2 ss = *reinterpret_cast<const float2*>(s_ss + vc), svl = *reinterpret_cast<const float2*>(s_svl + vc);
+        const F2 s2(ss.x, ss.y), l2(svl.x, svl.y);
+        const F2 ra = mul2(mul2(F2((float)(int)r[4 * n4], (float)(int)r[4 * n4 + 1]), s2), F2(ega, ega));
+        const F2 rb = mul2(mul2(F2((float)(int)r[4 * n4 + 2], (float)(int)r[4 * n4 + 3]), s2), F2(egb, egb));
+        fma2(F2(acco[4 * ng + n4][0], acco[4 * ng + n4][1]), l2, ra).get(outa[2 * n4], outa[2 * n4 + 1]);
+        fma2(F2(acco[4 * ng + n4][2], acco[4 * ng + n4][3]), l2, rb).get(outb[2 * n4], outb[2 * n4 + 1]);
       }
       store8_tc<OT>(op + rowa + 32 * ng + 8 * j, outa);
       store8_tc<OT>(op + rowb + 32 * ng + 8 * j, outb);
     }
-  } else if (tid == 0) {
+  } else if (lane == 0) {
     atomicExch(a.status, 1);
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
