@@ -51,8 +51,13 @@ __device__ __forceinline__ void store8<__nv_bfloat16>(__nv_bfloat16* dst, const 
                  Act<__nv_bfloat16>::pack2(x[4], x[5]), Act<__nv_bfloat16>::pack2(x[6], x[7]));
 }
 
+// Bound by how many CTAs share an SM (each is one pass through load, product, store) and by HBM with the precomputed A: the
+// launch bounds keep the count that shared memory allows. With A requested after the tiles had landed, three CTAs an SM (142 to 150
+// registers) and the scales of the state read multiplied one by one, 256 (b, h) x 128 chunks at K = V = 128, diagonal decay, took
+// 439 us; now 337 (285 at the copy bandwidth). GLA, 64 (b, h) x 64 chunks: K = V = 64 26.6 -> 22.8, K = 128, V = 64 35.5 -> 27.7; scalar
+// decay, K = V = 64: 34.3 -> 33.1; un-rotated, K = V = 128: 145 -> 137.
 template <int K, int V, typename OT, bool DIAG, bool UNROT>
-__global__ void __launch_bounds__(128) zoo_output_scalar_kernel(OutputArgs a) {
+__global__ void __launch_bounds__(128, V == 64 ? 5 : UNROT ? 3 : 4) zoo_output_scalar_kernel(OutputArgs a) {
   pdl_enter();
   constexpr int C = 64, LDR = V + 8;
   constexpr int KK = K / 64;  // 64-byte reduction blocks per row
@@ -99,9 +104,26 @@ __global__ void __launch_bounds__(128) zoo_output_scalar_kernel(OutputArgs a) {
       }
     }
     cp_async_commit();
+  }
+  const int ia = warp * 16 + g, ib = ia + 8;
+  uint32_t P[4][4];
+  if (DIAG) {
+    // A operand straight from the precomputed matrix, on its way with the tiles: slots (2j,2j+1 | 8+2j,8+2j+1) of k-step ks
+    // are the tokens 16ks + 4j + {0,1 | 2,3}
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks) {
+      uint2 ra = make_uint2(0u, 0u), rb = ra;
+      if (ks <= warp) {
+        ra = *reinterpret_cast<const uint2*>(a.amat + (tile * C + ia) * C + 16 * ks + 4 * j);
+        rb = *reinterpret_cast<const uint2*>(a.amat + (tile * C + ib) * C + 16 * ks + 4 * j);
+      }
+      P[ks][0] = ra.x; P[ks][1] = rb.x; P[ks][2] = ra.y; P[ks][3] = rb.y;
+    }
+  }
+  {
     if (tid < C) s_gc[tid] = DIAG ? 0.f : a.gc[tile * C + tid];
     for (int i = tid; i < V; i += 128) {
-      s_ss[i] = a.ss[h * V + i];
+      s_ss[i] = __fmul_rn(a.sq[h], a.ss[h * V + i]);  // of the state read: query and state scale
       s_svl[i] = a.svl[h * V + i];
     }
     cp_async_wait<0>();
@@ -110,7 +132,6 @@ __global__ void __launch_bounds__(128) zoo_output_scalar_kernel(OutputArgs a) {
 
   const float sq = a.sq[h], sk = a.sk[h];
   const float sqk = __fmul_rn(sq, sk);
-  const int ia = warp * 16 + g, ib = ia + 8;
   const float gia = s_gc[ia], gib = s_gc[ib];
 
   uint4 qa[KK], qb[KK];
@@ -121,19 +142,10 @@ __global__ void __launch_bounds__(128) zoo_output_scalar_kernel(OutputArgs a) {
   }
 
   // ---- S2 and P. MMA column (nt, cn) of S2 is token 16*(nt/2) + 4*(cn/2) + 2*(nt%2) + (cn%2).
-  uint32_t P[4][4];
 #pragma unroll
   for (int ks = 0; ks < 4; ++ks) {
     if (DIAG) {
-      // A operand straight from the precomputed matrix: slots (2j,2j+1 | 8+2j,8+2j+1) of k-step ks are the
-      // tokens 16ks + 4j + {0,1 | 2,3}
-      if (ks <= warp) {
-        const uint2 ra = *reinterpret_cast<const uint2*>(a.amat + (tile * C + ia) * C + 16 * ks + 4 * j);
-        const uint2 rb = *reinterpret_cast<const uint2*>(a.amat + (tile * C + ib) * C + 16 * ks + 4 * j);
-        P[ks][0] = ra.x; P[ks][1] = rb.x; P[ks][2] = ra.y; P[ks][3] = rb.y;
-      } else {
-        P[ks][0] = P[ks][1] = P[ks][2] = P[ks][3] = 0u;
-      }
+      // from above
     } else if (ks <= warp) {
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
@@ -224,22 +236,24 @@ __global__ void __launch_bounds__(128) zoo_output_scalar_kernel(OutputArgs a) {
     for (int n4 = 0; n4 < 4; ++n4) {
       const int nt = 4 * ng + n4;
       const int vr = 8 * nt + g;  // row n of the stored-state tile is MMA column n
-      int acc[4] = {0, 0, 0, 0};
+      int acc[4];
 #pragma unroll
       for (int kk = 0; kk < KK; ++kk) {
         const uint4 bs = *reinterpret_cast<const uint4*>(s_h + swz_k<K>(vr, 4 * kk + j));
-        mma_s8(acc, qa[kk].x, qb[kk].x, qa[kk].y, qb[kk].y, bs.x, bs.y);
+        if (kk == 0) mma_s8_first(acc, qa[kk].x, qb[kk].x, qa[kk].y, qb[kk].y, bs.x, bs.y);
+        else mma_s8(acc, qa[kk].x, qb[kk].x, qa[kk].y, qb[kk].y, bs.x, bs.y);
         mma_s8(acc, qa[kk].z, qb[kk].z, qa[kk].w, qb[kk].w, bs.z, bs.w);
       }
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int vc = 32 * ng + 8 * j + 2 * n4 + e;
-        const float ss = s_ss[vc], svl = s_svl[vc];
-        const float ra = __fmul_rn(__fmul_rn(__fmul_rn((float)acc[e], sq), ss), ega);
-        const float rb = __fmul_rn(__fmul_rn(__fmul_rn((float)acc[2 + e], sq), ss), egb);
-        outa[2 * n4 + e] = UNROT ? __fadd_rn(acco[nt][e], ra) : fmaf(acco[nt][e], svl, ra);
-        outb[2 * n4 + e] = UNROT ? __fadd_rn(acco[nt][2 + e], rb) : fmaf(acco[nt][2 + e], svl, rb);
+      const int vc = 32 * ng + 8 * j + 2 * n4;
+      const float2 ss = *reinterpret_cast<const float2*>(s_ss + vc), sl = *reinterpret_cast<const float2*>(s_svl + vc);
+      F2 ra = mul2(F2((float)acc[0], (float)acc[1]), F2(ss.x, ss.y)), rb = mul2(F2((float)acc[2], (float)acc[3]), F2(ss.x, ss.y));
+      if (!DIAG) {
+        ra = mul2(ra, F2(ega, ega));
+        rb = mul2(rb, F2(egb, egb));
       }
+      const F2 oa(acco[nt][0], acco[nt][1]), ob(acco[nt][2], acco[nt][3]), l2(sl.x, sl.y);
+      (UNROT ? add2(oa, ra) : fma2(oa, l2, ra)).get(outa[2 * n4], outa[2 * n4 + 1]);
+      (UNROT ? add2(ob, rb) : fma2(ob, l2, rb)).get(outb[2 * n4], outb[2 * n4 + 1]);
     }
     store8<OT>(op + rowa + 32 * ng + 8 * j, outa);
     store8<OT>(op + rowb + 32 * ng + 8 * j, outb);
