@@ -944,8 +944,6 @@ int run_chunk_state_value_tc(const lq_ssd_problem* p, int* status, cudaStream_t 
 bool chunk_state_value_tc2_applies(const lq_ssd_problem* p);
 int run_chunk_state_value_tc2(const lq_ssd_problem* p, int* status, cudaStream_t st);
 int run_chunk_scan_tc(const lq_ssd_problem* p, int* status, cudaStream_t st);
-int run_chunk_scan_codes(const lq_ssd_problem* p, int* status, cudaStream_t st);
-bool chunk_scan_codes_applies(const lq_ssd_problem* p);
 bool chunk_state_key_tc_applies(const lq_ssd_problem* p);
 int run_chunk_state_key_tc(const lq_ssd_problem* p, int* status, cudaStream_t st);
 bool bmm_tc_applies(const lq_ssd_problem* p, bool b_is_fp);
@@ -1059,17 +1057,11 @@ extern "C" int lq_ssd_chunk_scan(const lq_ssd_problem* p, lq_stream stream) {
   if (!p->cb || !p->dt || !p->dA || !p->q_C || !p->C_scale || !p->passed || !p->state_scale || !p->cb_scale || !p->out)
     return fail(LQ_ERR_NULL, "chunk_scan: cb, dt, dA, q_C, C_scale, passed, state_scale, cb_scale, out required");
   cudaStream_t st = (cudaStream_t)stream;
-  // Three kernels. The persistent tcgen05 kernel that keeps a chunk's CB codes in tensor memory and scales x takes about 10 us to
-  // get going (codes, first tiles) and then the least time per item: it is the library's choice from 4096 head-tokens per SM on
-  // (measured against the next one at chunk 256, d_state 128: 4 items per SM 32 : 29 us, 17 per SM 81 : 93, 277 per SM 950 : 1303;
-  // at chunk 128 55 per SM 128 : 141; against the warp-level kernel at chunk 64 16 per SM 36 : 32, 443 per SM 746 : 1020, chunk 192
-  // 55 per SM 193 : 309). Below, the tcgen05 kernel that builds the weights (d_state 128, chunks of 128 or 256 tokens), and the
-  // warp-level MMA kernel for every other shape.
+  // Two kernels: a persistent, software-pipelined tcgen05 + TMA kernel (d_state 128, chunks of 128 or 256 tokens: the
+  // Mamba-2 shapes), which is the library's choice where it applies, and the warp-level MMA kernel (every supported shape).
   const bool tc_ok = p->N == 128 && p->chunk % 128 == 0;
   if (p->scan_kernel == 2 && !tc_ok) return fail(LQ_ERR_UNSUPPORTED, "chunk_scan: the tcgen05 kernel needs d_state 128 and chunk 128 or 256");
   if (p->scan_kernel < 0 || p->scan_kernel > 2) return fail(LQ_ERR_SHAPE, "chunk_scan: scan_kernel must be 0, 1 or 2");
-  const long long head_tokens = (long long)p->B * p->L * p->H;
-  if (p->scan_kernel == 0 && head_tokens >= 4096LL * sm_count() && chunk_scan_codes_applies(p)) return run_chunk_scan_codes(p, p->status, st);
   if (p->scan_kernel == 2 || (p->scan_kernel == 0 && tc_ok)) return run_chunk_scan_tc(p, p->status, st);
   if (misaligned(p->q_C, 16) || misaligned(p->passed, 16) || misaligned(p->cb, 16) || misaligned(p->out, 4))
     return fail(LQ_ERR_ALIGN, "chunk_scan: q_C, cb and the passed states must be 16-byte aligned");

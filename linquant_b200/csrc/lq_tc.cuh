@@ -32,13 +32,6 @@ __device__ __forceinline__ uint64_t desc_kmajor_sw128(uint32_t saddr) {
   return (uint64_t)((saddr >> 4) & 0x3FFF) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) |
          ((uint64_t)2 << 61);
 }
-// K-major operand with rows of 128 or 64 bytes, swizzled over the row (8-row groups are dense)
-template <int ROW>
-__device__ __forceinline__ uint64_t desc_kmajor(uint32_t saddr) {
-  static_assert(ROW == 128 || ROW == 64, "row bytes");
-  return (uint64_t)((saddr >> 4) & 0x3FFF) | ((uint64_t)1 << 16) | ((uint64_t)((8 * ROW) >> 4) << 32) | ((uint64_t)1 << 46) |
-         ((uint64_t)(ROW == 128 ? 2 : 4) << 61);
-}
 __device__ __forceinline__ void umma_i8(uint32_t d_tmem, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
