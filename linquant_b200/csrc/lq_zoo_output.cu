@@ -51,16 +51,24 @@ __device__ __forceinline__ void store8<__nv_bfloat16>(__nv_bfloat16* dst, const 
                  Act<__nv_bfloat16>::pack2(x[4], x[5]), Act<__nv_bfloat16>::pack2(x[6], x[7]));
 }
 
-// Bound by how many CTAs share an SM (each is one pass through load, product, store) and by HBM with the precomputed A: the
-// launch bounds keep the count that shared memory allows. With A requested after the tiles had landed, three CTAs an SM (142 to 150
-// registers) and the scales of the state read multiplied one by one, 256 (b, h) x 128 chunks at K = V = 128, diagonal decay, took
-// 439 us; now 337 (285 at the copy bandwidth). GLA, 64 (b, h) x 64 chunks: K = V = 64 26.6 -> 22.8, K = 128, V = 64 35.5 -> 27.7; scalar
-// decay, K = V = 64: 34.3 -> 33.1; un-rotated, K = V = 128: 145 -> 137.
+// Bound by how many CTAs share an SM (each is one pass through load, product, store) and by HBM with the precomputed A. The launch
+// bounds are register caps found by measuring: 96 registers at V = 64 (five CTAs; shared memory would hold seven or more, un-rotated
+// five or more), 128 at V = 128 (four; shared memory holds five at K = 128, eight at K = 64). Un-rotated at V = 128 shared memory holds
+// three CTAs at K = 64 and two at K = 128: the cap of 168 registers is out of the way there. With A requested after the tiles had
+// landed, 142 to 150 registers at K = V = 128 and the scales of the state read multiplied one by one, 256 (b, h) x 128 chunks at
+// K = V = 128, diagonal decay, took 439 us; now 337 (285 at the copy bandwidth). 64 (b, h) x 64 chunks, bf16, before and now:
+//   diagonal      K,V = 64,64 26.4 22.6    64,128 43.0 35.4    128,64 35.2 28.6    128,128 63.1 47.9
+//   scalar        K,V = 64,64 31.9 30.9    64,128 49.1 48.1
+//   un-rotated    K,V = 64,64 42.2 41.7    64,128 120.6 119.1    128,64 55.1 50.6    128,128 142.0 134.1
+// (scalar at K = 128: not taken by the library but where no status word is given.) The state read goes two channels to an instruction
+// but for the scalar form at 64,128: pairs spill there under the cap of 128 (2 chunks x 16 (b, h) 4.40 -> 4.57 us, float output 55.0 ->
+// 55.5); one by one 4.41 and 52.9.
 template <int K, int V, typename OT, bool DIAG, bool UNROT>
 __global__ void __launch_bounds__(128, V == 64 ? 5 : UNROT ? 3 : 4) zoo_output_scalar_kernel(OutputArgs a) {
   pdl_enter();
   constexpr int C = 64, LDR = V + 8;
   constexpr int KK = K / 64;  // 64-byte reduction blocks per row
+  constexpr bool PAIRS = !(K == 64 && V == 128 && !DIAG && !UNROT);
   extern __shared__ __align__(128) uint8_t smem[];
   uint8_t* s_q = smem;
   uint8_t* s_k = s_q + C * K;
@@ -246,14 +254,23 @@ __global__ void __launch_bounds__(128, V == 64 ? 5 : UNROT ? 3 : 4) zoo_output_s
       }
       const int vc = 32 * ng + 8 * j + 2 * n4;
       const float2 ss = *reinterpret_cast<const float2*>(s_ss + vc), sl = *reinterpret_cast<const float2*>(s_svl + vc);
-      F2 ra = mul2(F2((float)acc[0], (float)acc[1]), F2(ss.x, ss.y)), rb = mul2(F2((float)acc[2], (float)acc[3]), F2(ss.x, ss.y));
-      if (!DIAG) {
-        ra = mul2(ra, F2(ega, ega));
-        rb = mul2(rb, F2(egb, egb));
+      if (PAIRS) {
+        F2 ra = mul2(F2((float)acc[0], (float)acc[1]), F2(ss.x, ss.y)), rb = mul2(F2((float)acc[2], (float)acc[3]), F2(ss.x, ss.y));
+        if (!DIAG) {
+          ra = mul2(ra, F2(ega, ega));
+          rb = mul2(rb, F2(egb, egb));
+        }
+        const F2 oa(acco[nt][0], acco[nt][1]), ob(acco[nt][2], acco[nt][3]), l2(sl.x, sl.y);
+        (UNROT ? add2(oa, ra) : fma2(oa, l2, ra)).get(outa[2 * n4], outa[2 * n4 + 1]);
+        (UNROT ? add2(ob, rb) : fma2(ob, l2, rb)).get(outb[2 * n4], outb[2 * n4 + 1]);
+      } else {
+        const float s2[2] = {ss.x, ss.y}, l2[2] = {sl.x, sl.y};
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          outa[2 * n4 + e] = fmaf(acco[nt][e], l2[e], __fmul_rn(__fmul_rn((float)acc[e], s2[e]), ega));
+          outb[2 * n4 + e] = fmaf(acco[nt][2 + e], l2[e], __fmul_rn(__fmul_rn((float)acc[2 + e], s2[e]), egb));
+        }
       }
-      const F2 oa(acco[nt][0], acco[nt][1]), ob(acco[nt][2], acco[nt][3]), l2(sl.x, sl.y);
-      (UNROT ? add2(oa, ra) : fma2(oa, l2, ra)).get(outa[2 * n4], outa[2 * n4 + 1]);
-      (UNROT ? add2(ob, rb) : fma2(ob, l2, rb)).get(outb[2 * n4], outb[2 * n4 + 1]);
     }
     store8<OT>(op + rowa + 32 * ng + 8 * j, outa);
     store8<OT>(op + rowb + 32 * ng + 8 * j, outb);

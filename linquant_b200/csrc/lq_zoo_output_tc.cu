@@ -13,7 +13,8 @@
 // Bound by latency (a CTA is one pass through load, product, mask, product, store; four share an SM) and, with many, by instruction
 // issue. Every warp waits for the accumulators on its own (block barriers with one polling thread: 65 us at 64 (b, h) x 64 chunks,
 // V = 128, and 7.1 at 16 x 2), and the scales of the state read are multiplied once, two channels to an instruction: 59 and 6.4.
-// Every wait on an mbarrier is bounded; on expiry the CTA raises the status word, skips its stores and still frees TMEM.
+// Every wait on an mbarrier is bounded; on expiry the status word is raised, the warp concerned (every warp where the operands never
+// landed) stores nothing from there on, and the CTA still frees TMEM.
 // Arithmetic and references: see lq_zoo_output.cu.
 #include "lq_tc.cuh"
 
