@@ -52,9 +52,9 @@ __device__ __forceinline__ void store8<__nv_bfloat16>(__nv_bfloat16* dst, const 
 }
 
 // Bound by how many CTAs share an SM (each is one pass through load, product, store) and by HBM with the precomputed A. The launch
-// bounds are register caps found by measuring: 96 registers at V = 64 (five CTAs; shared memory would hold seven or more, un-rotated
-// five or more), 128 at V = 128 (four; shared memory holds five at K = 128, eight at K = 64). Un-rotated at V = 128 shared memory holds
-// three CTAs at K = 64 and two at K = 128: the cap of 168 registers is out of the way there. With A requested after the tiles had
+// bounds are register caps found by measuring: 96 registers at V = 64 (five CTAs; by the bytes 228 KB of shared memory would hold seven
+// or more, un-rotated five or more), 128 at V = 128 (four; five at K = 128 and eight at K = 64 by the bytes). Un-rotated at V = 128 the
+// bytes allow three CTAs at K = 64 and two at K = 128: the cap of 168 registers is out of the way there. With A requested after the tiles had
 // landed, 142 to 150 registers at K = V = 128 and the scales of the state read multiplied one by one, 256 (b, h) x 128 chunks at
 // K = V = 128, diagonal decay, took 439 us; now 337 (285 at the copy bandwidth). 64 (b, h) x 64 chunks, bf16, before and now:
 //   diagonal      K,V = 64,64 26.4 22.6    64,128 43.0 35.4    128,64 35.2 28.6    128,128 63.1 47.9
