@@ -19,14 +19,16 @@ def make(B, NC, H, G, N, C, dtype, decay, seed, D_dims=1):
     randn = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
     L = NC * C
     dt = torch.nn.functional.softplus(randn(B, H, NC, C) * 0.5 - 2.0)
-    lo, hi = {"slow": (0.1, 3.0), "mixed": (1.0, 16.0), "fast": (40.0, 80.0), "reset": (0.5, 4.0)}[decay]
+    lo, hi = {"slow": (0.1, 3.0), "mixed": (1.0, 16.0), "fast": (40.0, 80.0), "reset": (0.5, 4.0), "wander": (0.1, 0.4)}[decay]
     if decay == "reset":  # a token in a hundred forgets everything before it
         dt = torch.where(rand(*dt.shape) < 0.01, torch.full_like(dt, 200.0), dt)
+    if decay == "wander":  # log-decays that rise and fall
+        dt = dt * randn(*dt.shape)
     dA = (-torch.linspace(lo, hi, H, device="cuda", dtype=torch.float64).view(1, H, 1, 1) * dt).cumsum(-1).float()
     i8 = lambda *s: torch.randint(-127, 128, s, generator=g, device="cuda", dtype=torch.int32).to(torch.int8)  # noqa: E731
     sc = lambda *s: rand(*s) * 0.01 + 0.01  # noqa: E731
     return dict(cb=i8(B, NC, G, C, C), x=randn(B, L, H, 64).to(dtype), dt=dt, dA=dA, qC=i8(B, L, G, N), sC=sc(G), passed=i8(B, NC, H, 64, N),
-                D=randn(H) if D_dims == 1 else randn(H, 64), sS=sc(H, 64), sCB=sc(G))
+                D=(None, randn(H), randn(H, 64))[D_dims], sS=sc(H, 64), sCB=sc(G))
 
 
 def scan(k):
@@ -49,7 +51,9 @@ def exact(k):
         M = k["cb"][:, :, gr].double() * (dA.unsqueeze(-1) - dA.unsqueeze(-2)).exp().tril() * (k["sCB"][gr].double() * k["dt"][:, h].double()).unsqueeze(-2)
         read = k["qC"][:, :, gr].double().view(B, NC, C, -1) @ k["passed"][:, :, h].double().transpose(-1, -2)
         y = M @ X + read * (k["sC"][gr].double() * k["sS"][h].double()) * dA.exp().unsqueeze(-1)
-        out[:, :, h] = (y + X * k["D"][h].double()).reshape(B, L, P)
+        if k["D"] is not None:
+            y = y + X * k["D"][h].double()
+        out[:, :, h] = y.reshape(B, L, P)
     return out
 
 
@@ -113,15 +117,37 @@ def test_opposite_infinities_reach_every_later_row(C, N, dtype):
     assert not torch.isfinite(scan(k)[0, 30:C, 0, 5]).any()
 
 
-@pytest.mark.parametrize("decay", ["slow", "mixed", "fast", "reset"])
-@pytest.mark.parametrize("B,NC,H,G,N,C,dtype,D_dims", [(2, 80, 16, 1, 128, 256, torch.bfloat16, 1), (2, 80, 16, 2, 64, 256, torch.float16, 2),
-                                                       (1, 291, 33, 1, 64, 64, torch.bfloat16, 1), (1, 101, 7, 7, 128, 128, torch.float16, 1),
-                                                       (1, 1, 1, 1, 128, 256, torch.bfloat16, 2), (1, 5, 3, 1, 64, 192, torch.bfloat16, 1)])
-def test_every_chunk_against_64_bits(B, NC, H, G, N, C, dtype, D_dims, decay):
+def check(o, k, e):
     """Relative error of each (batch, chunk, head) by itself, so that rows with large steps do not outweigh the rest. A weight is rounded
     to fp16 up to three times (relative 2^-11 each, once more for D on the diagonal) and the output once: 5 * 2^-11 = 2.4e-3 if every
     rounding were at its bound with the same sign."""
-    k = make(B, NC, H, G, N, C, dtype, decay, 3, D_dims)
-    o, e = scan(k).double().view(B, NC, C, H, 64), exact(k).view(B, NC, C, H, 64)
+    B, L, H, P = o.shape
+    NC, C = k["dt"].shape[2:]
+    o, e = o.double().view(B, NC, C, H, P), e.view(B, NC, C, H, P)
     err = (o - e).pow(2).sum((2, 4)).sqrt() / e.pow(2).sum((2, 4)).sqrt()
     assert float(err.max()) < 2.4e-3, f"worst chunk {float(err.max()):.2e}, mean {float(err.mean()):.2e}"
+
+
+@pytest.mark.parametrize("decay", ["slow", "mixed", "fast", "reset", "wander"])
+@pytest.mark.parametrize("B,NC,H,G,N,C,dtype,D_dims", [(2, 80, 16, 1, 128, 256, torch.bfloat16, 1), (2, 80, 16, 2, 64, 256, torch.float16, 2),
+                                                       (2, 106, 16, 2, 128, 192, torch.bfloat16, 0), (1, 291, 33, 1, 64, 64, torch.bfloat16, 2),
+                                                       (1, 101, 7, 7, 128, 128, torch.float16, 1), (1, 1, 1, 1, 128, 256, torch.bfloat16, 2),
+                                                       (1, 5, 3, 1, 64, 192, torch.bfloat16, 1)])
+def test_every_chunk_against_64_bits(B, NC, H, G, N, C, dtype, D_dims, decay):
+    k = make(B, NC, H, G, N, C, dtype, decay, 3, D_dims)
+    check(scan(k), k, exact(k))
+
+
+@pytest.mark.parametrize("H,NC,C,N", [(1, 2399, 256, 128), (149, 33, 128, 128), (37, 65, 256, 64), (33, 291, 64, 128), (7, 500, 192, 64)])
+def test_item_counts_that_do_not_divide_among_the_sms(H, NC, C, N):
+    k = make(1, NC, H, 1, N, C, torch.bfloat16, "mixed", 5)
+    check(scan(k), k, exact(k))
+
+
+def test_x_as_a_view_into_wider_rows():
+    k = make(2, 40, 32, 1, 128, 256, torch.bfloat16, "mixed", 6)
+    wide = torch.full((2, k["x"].shape[1], 32 * 64 + 256), 7.0, device="cuda", dtype=torch.bfloat16)
+    wide[..., :2048] = k["x"].flatten(-2)
+    e = exact(k)
+    k["x"] = wide[..., :2048].unflatten(-1, (32, 64))
+    check(scan(k), k, e)
